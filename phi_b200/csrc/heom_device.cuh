@@ -78,9 +78,12 @@ struct HeomConsts {
   long long first_wait_polls;
   // Tile-kernel schedule (host side only, chosen by the autotuner):
   // block-size variant (0 the default of the shape, 1 the alternative) and
-  // persistent CTAs per SM (0: as many as fit).
+  // persistent CTAs per SM (0: as many as fit), for the apply and RK4 stages
+  // and for the RKF45 stages (other kernels with more operands).
   int tile_variant;
   int tile_cps;
+  int tile_variant_rkf;
+  int tile_cps_rkf;
   // Adaptive hierarchy filtering (PHI's FilterTolerance, independent baths):
   // a node whose largest |element| drops below filter_tol stops feeding its
   // neighbours until it rises above it again.

@@ -24,7 +24,7 @@ struct TileSchedule {
   float ms_default = 0.f;
 };
 int tile_block_threads(const HeomConsts &c, bool mixed, int variant);
-// Times one Liouvillian apply (L's x -> out, apply mode) for every block-size
+// Times stage launch L (its outputs are overwritten) for every block-size
 // variant and CTAs-per-SM cap and returns the fastest (about 30 launches).
 cudaError_t tile_autotune(const StageLaunch &L, cudaStream_t stream, TileSchedule *out);
 

@@ -16,25 +16,29 @@
 //          elements so each node range is 16-byte aligned.
 //
 // A CTA of BT threads (kTileThreads = 256, or what the single-instance
-// launch picks per (N, arithmetic)) owns a tile of NT consecutive nodes (one
-// or two upper-triangle pairs of one node per thread).  Everything the tile reads of
-// its own nodes is contiguous in HBM and arrives by TMA bulk copies issued at
-// CTA start:
+// launch picks) owns a tile of NT consecutive nodes.  Everything the tile
+// reads of its own nodes is contiguous in HBM and arrives by TMA bulk copies:
+// its stage input X_s, its neighbour records and every epilogue operand
+// (state y, RK4 accumulator, RKF45 k_r).  Per tile:
 //
-//   t = 0   one thread issues cp.async.bulk copies of the tile's stage input
-//           X_s (barrier 0) and of every epilogue operand -- state y, RK4
-//           accumulator, RKF45 k_r -- (barrier 1) into shared memory; all
-//           threads load the tile's next/prev ids and occupations.
-//   phase 2 (after barrier 0) work item = (node, upper-triangle pair i <= j):
-//           A_ij, A_ji from shared memory (A = H X, [H, X] = A - A^+),
-//           dephasing + Matsubara factor, and the neighbour terms: for each
-//           term on site j (column part) or site i (row part), the one
-//           element of the linked ADO this pair needs, loaded from L2 with
-//           independent predicated loads (a Hermitian ADO's row m is the
-//           conjugate of its column m).  dX_ij and dX_ji = conj(dX_ij) go to
-//           shared memory.
-//   phase 3 (after barrier 1) epilogue per tile element: plain store, RK4 or
-//           RKF45 stage combine, RKF45 error max; operands from shared memory.
+//   phase 1  neighbour records: element offsets and coefficients per (node,
+//            term).
+//   phase 2  (tile_derivative) A = H X from shared memory ([H, X] = A - A^+),
+//            dephasing + Matsubara factor, and the neighbour terms from the
+//            linked ADOs, gathered from L2 with independent predicated loads.
+//            Only column m of an ADO linked by a bath on site m is read: the
+//            row m of a Hermitian ADO is its conjugate.
+//   phase 3  (tile_epilogue) plain store, RK4 or RKF45 stage combine, RKF45
+//            error max; operands from shared memory.
+//
+// What bounds it (B200): latency -- shared-memory and L2 round trips and the
+// tile's barriers at 20 to 32 warps per SM, issue slots 40-45 % used -- and
+// the shared-memory pipe (60-69 % of peak in the 7-site kernel), not DRAM.
+// Mapping the products and, outside the RKF45 stages of few sites, the
+// neighbour terms by element instead of by upper-triangle pair measured:
+// 16-site FP64 RK4 stage 37 -> 20 us, 24-site FP64 61 -> 45 us, 8-site mixed
+// 9.1 -> 6.5 us, 4-site K = 2 FP64 apply 49 -> 36 us, 48 uneven instances in
+// mixed precision 2.55 -> 1.76 ms per RK4 step.
 //
 // Stores of the next stage input use the default cache policy (its neighbour
 // gathers in the next stage should hit L2); k and accumulator stores stream.
@@ -160,32 +164,37 @@ __device__ __forceinline__ double2 cfma(double2 acc, double2 b, double s) {
 }
 template <class TX> __device__ __forceinline__ void st_stream(TX *p, TX v) { __stcs(p, v); }
 
-template <int N, bool MIXED, int KT, int BT = kTileThreads>
+template <int N, bool MIXED, int KT, int BT = kTileThreads, bool RKF = false>
 struct TileShape {
   static constexpr int E = N * N;
   static constexpr int EP = E + (E & 1);  // complex64 node stride (16-byte aligned nodes)
+  static constexpr int ES = MIXED ? EP : E;  // node stride of X / k buffers
   static constexpr int P = N * (N + 1) / 2;
-  // (node, pair) items per thread: two for N >= 12, whose nodes would
-  // otherwise leave a tile of one node and idle threads, two in mixed
-  // precision from N = 4 (timed on B200: the 7-site RKF45 step 0.245 ->
-  // 0.238 ms, the batched workload +16 % throughput; from N = 2 it gains
-  // less, three are slower in both arithmetics), and two in FP64 for
-  // K+1 = 3 up to N = 6 (the 4-site steady solve -4.5 %; with K+1 <= 2 FP64
-  // is slower with two: 9 % on the 7-site step, 5 % on the batched one);
-  // one otherwise.
-  static constexpr bool kTwo = N >= 12 || (MIXED && N >= 4) || (!MIXED && KT == 3 && N <= 6);
-  static constexpr int NT0 = (kTwo ? 2 : 1) * BT / P;
+  // How the neighbour terms are mapped (tile_derivative): by upper-triangle
+  // pair, or by element.
+  static constexpr bool kPairs = RKF && N < 10;
+  // Thread t < CS * N works on row t % N of the tile's columns t / N, t / N +
+  // CS, ...: one H_ik serves all of a thread's elements, and a warp's
+  // gathers and stores run along whole columns.
+  static constexpr int CS = BT / N;
+  // Nodes per tile: one pair per thread, or 32 bytes of elements per thread
+  // and operand; FP64 halves tiles of more than 40 nodes (sites <= 3), which
+  // would leave a small hierarchy too few CTAs (84-node trimer, 256 RK4
+  // steps: 4.35 -> 3.80 ms).
+  static constexpr int NT0 = kPairs ? BT / P : (MIXED ? 4 : (2 * CS / N > 40 ? 1 : 2)) * CS / N;
   static constexpr int NT = NT0 < 1 ? 1 : (NT0 > 64 ? 64 : NT0);
-  // Column stride of the derivative tile in shared memory: odd, so the
-  // transposed (j, i) writes of one warp fall in distinct banks.
+  static constexpr int RR = (NT * N + CS - 1) / CS;  // elements per thread
+  static constexpr int PR = (NT * P + BT - 1) / BT;  // pairs per thread
+  // The exchange tile's column stride is odd, so the transposed (j, i) reads
+  // of one warp fall in distinct banks; an odd N shares X's offsets.
   static constexpr int NP = (N & 1) ? N : N + 1;
-  static constexpr int EU = N * NP;
+  static constexpr int EU = (N & 1) ? ES : N * NP;
 };
 
-template <int N, bool MIXED, int KT, int BT = kTileThreads>
+template <int N, bool MIXED, int KT, int BT = kTileThreads, bool RKF = false>
 struct TileLayout {
-  using S = TileShape<N, MIXED, KT, BT>;
-  static constexpr int ES = MIXED ? S::EP : S::E;  // node stride of X / k buffers
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  static constexpr int ES = S::ES;
   static constexpr int XB = MIXED ? 8 : 16;        // bytes per element of X / k
   // byte offsets in dynamic shared memory
   static constexpr size_t kBars = 0;
@@ -196,25 +205,21 @@ struct TileLayout {
   static constexpr size_t kPre = kU + kUBytes;
 };
 
-// Resident warps per SM the register budget is fitted to (timed on B200).
-// K+1 = 2 (7 sites): FP64 6 % faster at 4 CTAs than at 5 without spills;
-// mixed, with its two items per thread, 1 % faster at 4 (64 registers) than
-// at 5 and 4 % faster than at 3.  K+1 = 1 (24 sites): FP64 1.6 % faster at
-// 4 CTAs than at 5; the 320-thread mixed kernel fastest at 4 CTAs (40
-// warps).  More neighbour terms per site keep more gathered values live.
-template <int KT, bool MIXED, int BT = kTileThreads>
+// Resident warps per SM the register budget is fitted to.
+template <int KT, bool MIXED, int BT, bool PAIRS>
 struct TileMinBlocks {
-  static constexpr int warps = KT == 1 ? (MIXED ? 40 : 32) : (KT == 2 ? 32 : 24);
+  static constexpr int warps = MIXED ? (PAIRS ? 32 : 24) : (KT == 1 ? 32 : 24);
   static constexpr int value = warps / (BT / 32);
 };
 
 // New filter flags of a tile's nodes from |y_new|^2 staged in the first 8
-// bytes of each derivative-tile slot (slot bytes apart, column stride NP):
+// bytes of each exchange-tile slot (slot bytes apart, column stride NP, node
+// stride EU):
 // one warp per node; below the tolerance -> inactive, above -> active, equal
 // -> unchanged (hierarchy_integrator.cc:2827-2850, :2359-2384).  A NaN never
 // wins the `>`, as in PHI's scan.  Kept out of line so its registers do not
 // add to the tile body's.
-static __device__ __noinline__ void tile_filter_flags(const unsigned char *us, int slot, int N, int NP, int nt_here,
+static __device__ __noinline__ void tile_filter_flags(const unsigned char *us, int slot, int N, int NP, int EU, int nt_here,
                                                const uint8_t *act_in, uint8_t *act_out, double tol,
                                                int warps) {
   const int E = N * N, lane = threadIdx.x & 31;
@@ -222,7 +227,7 @@ static __device__ __noinline__ void tile_filter_flags(const unsigned char *us, i
     double m = 0.0;
     for (int w = lane; w < E; w += 32) {
       const int col = w / N;
-      const double v = *reinterpret_cast<const double *>(us + (size_t)(nd * N * NP + (w - col * N) + col * NP) * slot);
+      const double v = *reinterpret_cast<const double *>(us + (size_t)(nd * EU + (w - col * N) + col * NP) * slot);
       m = v > m ? v : m;
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -243,245 +248,424 @@ struct TileArith {
 };
 
 // ---- the parts of one tile shared by the kernels ----
-// Phase 2: the derivative of every (node, upper-triangle pair) of a tile into
-// the derivative tile Us, from shared memory (the tile's stage input Xs, H,
-// per-element Matsubara factors, pair lists, per-(node, term) neighbour
-// offsets and prefactor magnitudes, dephasing rates) and, for the neighbour
-// terms, from the stage input in HBM (xin).  HX_US: the products A = H X of
-// the tile are already in Us (computed on the tensor cores); each item reads
-// its two entries A_ij, A_ji there before it overwrites them with the
-// derivative (no other item touches those two slots).
-template <int N, int KT, bool MIXED, int BT, bool HX_US = false>
-__device__ __forceinline__ void tile_pairs(const HeomConsts &c, const typename TileArith<MIXED>::TX *Xs,
-                                           typename TileArith<MIXED>::TX *Us,
-                                           const typename TileArith<MIXED>::TX *Hs,
-                                           const typename TileArith<MIXED>::R *mats, const unsigned char *pi,
-                                           const unsigned char *pj, const int *ids,
-                                           const typename TileArith<MIXED>::R *cn,
-                                           const typename TileArith<MIXED>::R *cp,
-                                           const typename TileArith<MIXED>::R *ccr, const double *deph,
-                                           const int *nts, const typename TileArith<MIXED>::TX *xin, int nt_here) {
-  using S = TileShape<N, MIXED, KT, BT>;
-  using Lay = TileLayout<N, MIXED, KT, BT>;
-  using TX = typename TileArith<MIXED>::TX;
-  using R = typename TileArith<MIXED>::R;
-  constexpr int P = S::P, ES = Lay::ES, NP = S::NP, EU = S::EU;
-  constexpr int T = N * KT;
-  const int tid = threadIdx.x;
-  const bool hreal = c.h_real;
-  const R *Hr = reinterpret_cast<const R *>(Hs);
-  const R ih = (R)c.inv_hbar;
-  const int items = nt_here * P;
-  for (int it = tid; it < items; it += BT) {
-    const int nd = it / P, u = it - nd * P;
-    const int i = pi[u], j = pj[u];
-    const TX *X = Xs + nd * ES;
-    // Every neighbour value this pair needs, as independent predicated loads.
-    // In mixed precision they are issued before the products, whose work
-    // then hides their latency (timed on B200: 7-site RKF45 step -1.5 %,
-    // 24-site -1 %, batched RK4 -2.6 %); the FP64 kernels issue them after
-    // the products, where the extra live registers do not spill (hoisted:
-    // 7-site FP64 unchanged, 4-site steady solve 0.7 % slower).
-    constexpr bool kHoist = MIXED;
-    TX gn_c[KT], gp_c[KT], gn_r[KT], gp_r[KT];
-    auto gather = [&]() {
-      const int *nid = ids + nd * 2 * T;
-      const int oij = i + j * N, oji = j + i * N;
-      const TX zero = mk<TX>(0.0, 0.0);
-      const bool on = !c.vacuum;
+// One (node, term): prefactor magnitude s of the next ADO; the previous
+// one's scale sp and c_t (pairs), or a = sp * c_t (elements).
+template <class R, bool PAIRS>
+struct TileCoef;
+template <class R>
+struct alignas(16) TileCoef<R, true> {
+  R s, sp, cx, cy;
+};
+template <class R>
+struct alignas(16) TileCoef<R, false> {
+  R s, pad, ax, ay;
+};
+template <class C, class R>
+__device__ __forceinline__ C tile_coef(R s, R sp, double2 c) {
+  C f;
+  f.s = s;
+  if constexpr (std::is_same<C, TileCoef<R, true>>::value) {
+    f.sp = sp;
+    f.cx = (R)c.x;
+    f.cy = (R)c.y;
+  } else {
+    f.pad = 0;
+    f.ax = sp * (R)c.x;
+    f.ay = sp * (R)c.y;
+  }
+  return f;
+}
+// Reserved per-warp words (even, so what follows stays 16-byte aligned).
+__host__ __device__ constexpr int tile_warp_slots(int threads) { return (threads / 32 + 1) & ~1; }
+
+// This thread's share of a tile, the same in every tile: element r is row i
+// of column j of node nd.  Offsets of elements past the tile repeat its last
+// column, so every read stays inside the tile's buffers.
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+struct TileMap {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  int i;
+  int xo[S::RR];   // element in X (and k buffers): nd * ES + i + j * N
+  int ut[S::RR];   // its transpose in the exchange tile
+  int rec[S::RR];  // nd * T + j * KT, the first record of site j
+  unsigned live;   // bit r: the element is in the (full) tile
+  // kPairs: upper-triangle pairs i | j << 8 | node << 16 (node NT: none).
+  int ij[S::kPairs ? S::PR : 1];
+  __device__ __forceinline__ explicit TileMap(const HeomConsts &c) {
+    if constexpr (S::kPairs) {
 #pragma unroll
-      for (int q = 0; q < KT; ++q) {
-        const int tj = j * KT + q, ti = i * KT + q;
-        const int nxj = nid[tj], pvj = nid[T + tj], nxi = nid[ti], pvi = nid[T + ti];
-        gn_c[q] = (on && nxj >= 0 && i != j) ? __ldg(xin + nxj + oij) : zero;
-        gp_c[q] = (on && pvj >= 0 && i != j) ? __ldg(xin + pvj + oij) : zero;
-        gn_r[q] = (on && nxi >= 0 && i != j) ? __ldg(xin + nxi + oji) : zero;
-        gp_r[q] = (on && pvi >= 0) ? __ldg(xin + pvi + oji) : zero;
-      }
-    };
-    if constexpr (kHoist) gather();
-    R ar = 0, ai = 0, br = 0, bi = 0;  // A_ij, A_ji
-    if (HX_US) {
-      const TX aij = Us[nd * EU + i + j * NP], aji = Us[nd * EU + j + i * NP];
-      ar = aij.x;
-      ai = aij.y;
-      br = aji.x;
-      bi = aji.y;
-    } else if (hreal) {
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        // X_ki = conj(X_ik) (Hermitian ADO): lanes with consecutive i read
-        // consecutive words instead of a stride of N.
-        const R hik = Hr[i + k * N], hjk = Hr[j + k * N];
-        const TX xkj = X[k + j * N], xik = X[i + k * N];
-        ar = fma(hik, xkj.x, ar);
-        ai = fma(hik, xkj.y, ai);
-        br = fma(hjk, xik.x, br);
-        bi = fma(-hjk, xik.y, bi);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const TX hik = Hs[i + k * N], xkj = X[k + j * N];
-        const TX hjk = Hs[j + k * N], xik = X[i + k * N];  // X_ki = conj(X_ik)
-        ar = fma(hik.x, xkj.x, ar);
-        ar = fma(-hik.y, xkj.y, ar);
-        ai = fma(hik.x, xkj.y, ai);
-        ai = fma(hik.y, xkj.x, ai);
-        br = fma(hjk.x, xik.x, br);
-        br = fma(hjk.y, xik.y, br);
-        bi = fma(-hjk.x, xik.y, bi);
-        bi = fma(hjk.y, xik.x, bi);
+      for (int r = 0; r < S::PR; ++r) {
+        const int it = (int)threadIdx.x + r * BT;
+        const int nd = it / S::P, u = it - nd * S::P;
+        ij[r] = nd < S::NT ? (int)__ldg(c.pair_i + u) | (int)__ldg(c.pair_j + u) << 8 | nd << 16 : S::NT << 16;
       }
     }
-    // -i/hbar (A_ij - conj(A_ji))
-    R vx = (ai + bi) * ih, vy = -(ar - br) * ih;
-    const TX xij = X[i + j * N];
-    if (!c.vacuum) {
-      const R fac = (R)deph[nd] + mats[i + j * N];
-      vx = fma(-fac, xij.x, vx);
-      vy = fma(-fac, xij.y, vy);
-      const R *ncn = cn + nd * T, *ncp = cp + nd * T;
-      if constexpr (!kHoist) gather();
-      if (i != j) {
+    i = (int)threadIdx.x % N;
+    const int c0 = (int)threadIdx.x / N;
+    live = 0;
 #pragma unroll
-        for (int q = 0; q < KT; ++q) {
-          const int tj = j * KT + q, ti = i * KT + q;
-          // column part: + p X+_ij (p = i s), + i conj(c) sp X-_ij
-          const R sj = ncn[tj];
-          vx = fma(-sj, gn_c[q].y, vx);
-          vy = fma(sj, gn_c[q].x, vy);
-          const R spj = ncp[tj];
-          const R cjx = ccr[2 * tj], cjy = ccr[2 * tj + 1];
-          const TX g = gp_c[q];
-          const R re = cjx * g.x + cjy * g.y, im = cjx * g.y - cjy * g.x;
-          vx = fma(-spj, im, vx);
-          vy = fma(spj, re, vy);
-          // row part: - p conj(X+_ji), - i c sp conj(X-_ji)
-          const R si = ncn[ti];
-          vx = fma(-si, gn_r[q].y, vx);
-          vy = fma(-si, gn_r[q].x, vy);
-          const R spi = ncp[ti];
-          const R cix = ccr[2 * ti], ciy = ccr[2 * ti + 1];
-          const TX h = gp_r[q];
-          const R re2 = cix * h.x + ciy * h.y, im2 = ciy * h.x - cix * h.y;
-          vx = fma(spi, im2, vx);
-          vy = fma(-spi, re2, vy);
-        }
-      } else {
-        // diagonal: next terms cancel; prev gives 2 sp Im(c) X-_mm
-#pragma unroll
-        for (int q = 0; q < KT; ++q) {
-          const int ti = i * KT + q;
-          const R spi = ncp[ti];
-          const R ciy = ccr[2 * ti + 1];
-          vx = fma((R)2 * spi * ciy, gp_r[q].x, vx);
-        }
-      }
-    }
-    TX v;
-    v.x = vx;
-    v.y = vy;
-    if (i == j) {
-      v.y = 0;
-      Us[nd * EU + i + j * NP] = v;
-    } else {
-      Us[nd * EU + i + j * NP] = v;
-      v.y = -v.y;
-      Us[nd * EU + j + i * NP] = v;
+    for (int r = 0; r < S::RR; ++r) {
+      int col = c0 + r * S::CS;
+      if (c0 < S::CS && col < S::NT * N) live |= 1u << r;
+      col = col < S::NT * N ? col : S::NT * N - 1;
+      const int nd = col / N, j = col - nd * N;
+      xo[r] = nd * S::ES + i + j * N;
+      ut[r] = nd * S::EU + j + i * S::NP;
+      rec[r] = col * KT;
     }
   }
-  // Time-local truncation: the deepest tier's term, a pass of its own so the
-  // pair loop above keeps its registers.  Item `it` maps to the thread that
-  // wrote its two slots in the pair loop, so no barrier is needed before it.
-  if (c.time_local) {
-    for (int it = tid; it < items; it += BT) {
-      const int nd = it / P, u = it - nd * P;
-      const int i = pi[u], j = pj[u];
-      if (i == j) continue;
-      int tier = 0;  // deepest tier only (is_timelocal_truncated)
-      for (int t = 0; t < T; ++t) tier += nts[nd * T + t];
-      if (tier != c.L) continue;
-      const TX tv = tl_pair_term<TX>(Xs + nd * ES, c.tl_q, N, i, j);
-      TX a = Us[nd * EU + i + j * NP];
-      a.x += tv.x;
-      a.y += tv.y;
-      Us[nd * EU + i + j * NP] = a;
-      TX b = Us[nd * EU + j + i * NP];  // the Hermitian partner takes conj(tv)
-      b.x += tv.x;
-      b.y -= tv.y;
-      Us[nd * EU + j + i * NP] = b;
+  __device__ __forceinline__ bool on(int r, int nt_here) const {
+    return ((live >> r) & 1u) && xo[r] < nt_here * S::ES;
+  }
+  __device__ __forceinline__ int j(int r) const { return rec[r] / KT % N; }
+  __device__ __forceinline__ int nd(int r) const { return rec[r] / KT / N; }
+  // its own offset in the exchange tile
+  __device__ __forceinline__ int uo(int r) const { return (N & 1) ? xo[r] : rec[r] / KT * S::NP + i; }
+  // its offset in complex128 buffers
+  __device__ __forceinline__ int eo(int r) const { return S::ES == S::E ? xo[r] : xo[r] - nd(r); }
+};
+// A = H X of this thread's elements, from shared memory: k runs outside, so
+// one H_ik serves all of the thread's elements and a warp's reads of X are
+// broadcasts along its columns.
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+__device__ __forceinline__ void tile_products(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, RKF> &m,
+                                              const typename TileArith<MIXED>::TX *Xs,
+                                              const typename TileArith<MIXED>::TX *Hs,
+                                              typename TileArith<MIXED>::TX (&a)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using TX = typename TileArith<MIXED>::TX;
+  using R = typename TileArith<MIXED>::R;
+#pragma unroll
+  for (int r = 0; r < S::RR; ++r) a[r] = mk<TX>(0.0, 0.0);
+  const TX *Xc = Xs - m.i;
+  if (c.h_real) {
+    const R *Hr = reinterpret_cast<const R *>(Hs) + m.i;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const R h = Hr[k * N];
+#pragma unroll
+      for (int r = 0; r < S::RR; ++r) {
+        const TX x = Xc[m.xo[r] + k];
+        a[r].x = fma(h, x.x, a[r].x);
+        a[r].y = fma(h, x.y, a[r].y);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const TX h = Hs[m.i + k * N];
+#pragma unroll
+      for (int r = 0; r < S::RR; ++r) {
+        const TX x = Xc[m.xo[r] + k];
+        a[r].x = fma(h.x, x.x, a[r].x);
+        a[r].x = fma(-h.y, x.y, a[r].x);
+        a[r].y = fma(h.x, x.y, a[r].y);
+        a[r].y = fma(h.y, x.x, a[r].y);
+      }
     }
   }
 }
 
-// Phase 3: the epilogue over a tile's elements (plain store, RK4 or RKF45
-// stage combine) from the derivative tile Us and the prefetched operands at
-// PreBase + pre_off[b]; the RKF45 stage-5 error of this thread's elements is
-// folded into emax (max of |y4 - y5|, or of its square in mixed precision).
-// coef holds the 24 RKF45 coefficients in FP64 followed by the same 24 in
-// FP32.
-template <int N, int KT, bool MIXED, int BT>
-__device__ __forceinline__ void tile_epilogue(const TileParams &p, const typename TileArith<MIXED>::TX *Xs,
-                                              typename TileArith<MIXED>::TX *Us, const unsigned char *PreBase,
-                                              const uint32_t (&pre_off)[kMaxPre], const double *coef,
-                                              unsigned long long *wmax, long long tile, long long n0, int nt_here,
-                                              int ycur, double &emax) {
-  using S = TileShape<N, MIXED, KT, BT>;
-  using Lay = TileLayout<N, MIXED, KT, BT>;
+// What a tile's derivative is computed from (shared memory, except xin).
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+struct TileIn {
   using TX = typename TileArith<MIXED>::TX;
-  constexpr int E = S::E, ES = Lay::ES, NP = S::NP, EU = S::EU;
-  const HeomConsts &c = p.c;
+  using R = typename TileArith<MIXED>::R;
+  using C = TileCoef<R, TileShape<N, MIXED, KT, BT, RKF>::kPairs>;
+  const TX *Xs;         // the tile's stage input
+  TX *Us;               // exchange tile
+  const TX *Hs;         // H
+  const R *mats;        // Matsubara factor per element
+  const int2 *ids;      // neighbour element offsets (next, prev), -1 absent
+  const C *cfs;         // neighbour coefficients
+  const double *deph;   // dephasing rates
+  const uint8_t *mi;    // occupations (time-local truncation)
+  const TX *xin;        // the stage input of every node (HBM)
+  int nt_here;
+};
+
+// The deepest tier's time-local term of element (i, j), i < j, of node nd.
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+__device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileIn<N, KT, MIXED, BT, RKF> &in, int nd, int i,
+                                                int j, typename TileArith<MIXED>::TX &tv) {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  int tier = 0;  // deepest tier only (is_timelocal_truncated)
+  for (int t = 0; t < N * KT; ++t) tier += in.mi[nd * N * KT + t];
+  if (tier != c.L) return false;
+  tv = tl_pair_term<typename TileArith<MIXED>::TX>(in.Xs + nd * S::ES, c.tl_q, N, i, j);
+  return true;
+}
+
+// Phase 2: the derivative dx of this thread's elements of a tile.
+//
+// By element (kPairs off).  With
+//   B_ij = -i/hbar (H X)_ij + sum_q (i s X+_ij + i conj(c) sp X-_ij)
+// over the terms q of site j (column j of the linked ADOs), the derivative of
+// a Hermitian ADO is dX_ij = B_ij + conj(B_ji) - (dephasing + Matsubara_ij)
+// X_ij: the row parts of PHI's DoNext / DoPrevious are the conjugates of the
+// transposed element's column parts.  Each thread forms B of its elements --
+// a warp's gathers run along whole columns of the neighbours -- and the tile
+// exchanges B through Us.
+//
+// By pair (RKF45 stages below N = 10).  The products go through Us, then a
+// thread evaluates pair (i, j), both neighbour parts included, with the
+// operations and in the order of the first such kernel: the error estimate
+// of a stiff hierarchy (7 sites, K = 1, depth 6) is rounding amplified in the
+// deep tiers, so another order of this sum accepts and rejects other steps,
+// and a run can then end past t_end instead of at it (PHI's clamp does not
+// see a grown step).
+//
+// A_US: the products are already in Us (computed on the tensor cores).
+// Barriers: every thread of the CTA calls; Us must be free (or hold the
+// products, visible) on entry, and is free again after the CTA's next barrier.
+template <int N, int KT, bool MIXED, int BT, bool RKF, bool A_US = false>
+__device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, RKF> &m,
+                                                const TileIn<N, KT, MIXED, BT, RKF> &in,
+                                                typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using TX = typename TileArith<MIXED>::TX;
+  using R = typename TileArith<MIXED>::R;
+  constexpr int ES = S::ES, NP = S::NP, EU = S::EU, RR = S::RR, T = N * KT;
+  const R ih = (R)c.inv_hbar;
+  const bool nb = !c.vacuum;
+  const TX zero = mk<TX>(0.0, 0.0);
+  TX *Us = in.Us;
+  if constexpr (S::kPairs) {
+    static_assert(!A_US, "the tensor-core kernel maps by element");
+    // Every neighbour value the pairs need, as independent predicated loads,
+    // issued before the products, whose work hides their latency, where the
+    // registers hold them.
+    constexpr bool kHoist = MIXED || KT <= 2;
+    TX gn_c[S::PR][KT], gp_c[S::PR][KT], gn_r[S::PR][KT], gp_r[S::PR][KT];
+    auto gather = [&](int r) {
+      const int i = m.ij[r] & 255, j = m.ij[r] >> 8 & 255, nd = m.ij[r] >> 16;
+      const bool on = nb && nd < in.nt_here;
+      const int oij = i + j * N, oji = j + i * N, ndr = nd < S::NT ? nd : 0;
+#pragma unroll
+      for (int q = 0; q < KT; ++q) {
+        const int2 idj = in.ids[ndr * T + j * KT + q], idi = in.ids[ndr * T + i * KT + q];
+        gn_c[r][q] = (on && idj.x >= 0 && i != j) ? __ldg(in.xin + idj.x + oij) : zero;
+        gp_c[r][q] = (on && idj.y >= 0 && i != j) ? __ldg(in.xin + idj.y + oij) : zero;
+        gn_r[r][q] = (on && idi.x >= 0 && i != j) ? __ldg(in.xin + idi.x + oji) : zero;
+        gp_r[r][q] = (on && idi.y >= 0) ? __ldg(in.xin + idi.y + oji) : zero;
+      }
+    };
+    if constexpr (kHoist) {
+#pragma unroll
+      for (int r = 0; r < S::PR; ++r) gather(r);
+    }
+    tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < S::PR; ++r) {
+      if constexpr (!kHoist) gather(r);
+      const int i = m.ij[r] & 255, j = m.ij[r] >> 8 & 255, nd = m.ij[r] >> 16;
+      if (nd >= in.nt_here) continue;
+      const int uij = nd * EU + i + j * NP, uji = nd * EU + j + i * NP;
+      const TX a = Us[uij], b = Us[uji];
+      // -i/hbar (A_ij - conj(A_ji))
+      R vx = (a.y + b.y) * ih, vy = -(a.x - b.x) * ih;
+      if (nb) {
+        const TX xij = in.Xs[nd * ES + i + j * N];
+        const R fac = (R)in.deph[nd] + in.mats[i + j * N];
+        vx = fma(-fac, xij.x, vx);
+        vy = fma(-fac, xij.y, vy);
+        if (i != j) {
+#pragma unroll
+          for (int q = 0; q < KT; ++q) {
+            const auto fj = in.cfs[nd * T + j * KT + q], fi = in.cfs[nd * T + i * KT + q];
+            // column part: + p X+_ij (p = i s), + i conj(c) sp X-_ij
+            vx = fma(-fj.s, gn_c[r][q].y, vx);
+            vy = fma(fj.s, gn_c[r][q].x, vy);
+            const TX g = gp_c[r][q];
+            const R re = fj.cx * g.x + fj.cy * g.y, im = fj.cx * g.y - fj.cy * g.x;
+            vx = fma(-fj.sp, im, vx);
+            vy = fma(fj.sp, re, vy);
+            // row part: - p conj(X+_ji), - i c sp conj(X-_ji)
+            vx = fma(-fi.s, gn_r[r][q].y, vx);
+            vy = fma(-fi.s, gn_r[r][q].x, vy);
+            const TX h = gp_r[r][q];
+            const R re2 = fi.cx * h.x + fi.cy * h.y, im2 = fi.cy * h.x - fi.cx * h.y;
+            vx = fma(fi.sp, im2, vx);
+            vy = fma(-fi.sp, re2, vy);
+          }
+        } else {
+          // diagonal: next terms cancel; prev gives 2 sp Im(c) X-_mm
+#pragma unroll
+          for (int q = 0; q < KT; ++q) {
+            const auto fi = in.cfs[nd * T + i * KT + q];
+            vx = fma((R)2 * fi.sp * fi.cy, gp_r[r][q].x, vx);
+          }
+        }
+      }
+      TX v = mk<TX>(vx, vy);
+      if (c.time_local && i != j) {
+        TX tv;
+        if (tile_time_local<N, KT, MIXED, BT, RKF>(c, in, nd, i, j, tv)) {
+          v.x += tv.x;
+          v.y += tv.y;
+        }
+      }
+      if (i == j) v.y = 0;
+      Us[uij] = v;
+      if (i != j) Us[uji] = mk<TX>(v.x, -v.y);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RR; ++r) dx[r] = Us[m.uo(r)];
+  } else {
+    const int i = m.i;
+    // FP64 issues the gathers after the products (registers).
+    constexpr bool kHoist = MIXED || KT == 1 || (KT == 2 && RKF);
+    TX gn[RR][KT], gp[RR][KT];
+    auto gather = [&](int r) {
+      const bool on = nb && m.on(r, in.nt_here);
+      const int off = m.xo[r] - m.nd(r) * ES;
+      const bool diag = m.j(r) == i;
+#pragma unroll
+      for (int q = 0; q < KT; ++q) {
+        const int2 id = in.ids[m.rec[r] + q];
+        gn[r][q] = (on && id.x >= 0 && !diag) ? __ldg(in.xin + id.x + off) : zero;
+        gp[r][q] = (on && id.y >= 0) ? __ldg(in.xin + id.y + off) : zero;
+      }
+    };
+    if constexpr (kHoist) {
+#pragma unroll
+      for (int r = 0; r < RR; ++r) gather(r);
+    }
+    if constexpr (A_US) {
+#pragma unroll
+      for (int r = 0; r < RR; ++r) dx[r] = Us[m.uo(r)];
+    } else {
+      tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
+    }
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      if constexpr (!kHoist) gather(r);
+      R bx = dx[r].y * ih, by = -dx[r].x * ih;  // -i/hbar A
+      if (nb) {
+#pragma unroll
+        for (int q = 0; q < KT; ++q) {
+          const auto f = in.cfs[m.rec[r] + q];
+          bx = fma(-f.s, gn[r][q].y, bx);
+          by = fma(f.s, gn[r][q].x, by);
+          bx = fma(f.ay, gp[r][q].x, bx);
+          bx = fma(-f.ax, gp[r][q].y, bx);
+          by = fma(f.ax, gp[r][q].x, by);
+          by = fma(f.ay, gp[r][q].y, by);
+        }
+      }
+      dx[r] = mk<TX>(bx, by);
+      if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const TX bt = Us[m.ut[r]];
+      const int j = m.j(r);
+      R vx = dx[r].x + bt.x, vy = i == j ? (R)0 : dx[r].y - bt.y;
+      if (nb) {
+        // The upper triangle's X (a lower element is its conjugate).
+        const int nd = m.nd(r);
+        const TX x = in.Xs[i <= j ? m.xo[r] : nd * ES + j + i * N];
+        const R fac = (R)in.deph[nd] + in.mats[i + j * N];
+        vx = fma(-fac, x.x, vx);
+        vy = fma(i == j ? (R)0 : (i < j ? -fac : fac), x.y, vy);
+      }
+      dx[r] = mk<TX>(vx, vy);
+    }
+    if (c.time_local) {
+#pragma unroll 1
+      for (int r = 0; r < RR; ++r) {
+        int j = 0, nd = 0;
+#pragma unroll
+        for (int q = 0; q < RR; ++q)
+          if (q == r) {
+            j = m.j(q);
+            nd = m.nd(q);
+          }
+        TX tv;
+        if (i == j || !tile_time_local<N, KT, MIXED, BT, RKF>(c, in, nd, i < j ? i : j, i < j ? j : i, tv)) continue;
+#pragma unroll
+        for (int q = 0; q < RR; ++q)
+          if (q == r) {
+            dx[q].x += tv.x;
+            dx[q].y += i < j ? tv.y : -tv.y;
+          }
+      }
+    }
+  }
+}
+
+// Byte offset of prefetched epilogue operand b: operand 0, then the others,
+// one size apart (each padded to 128 bytes).
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+__host__ __device__ __forceinline__ uint32_t tile_pre_size(int bytes) {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  return ((uint32_t)S::NT * (bytes == 16 ? S::E : S::ES) * bytes + 127) / 128 * 128;
+}
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+__host__ __device__ __forceinline__ uint32_t tile_pre_off(const TileParams &p, int b) {
+  return b == 0 ? 0
+                : tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[0]) + (b - 1) * tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[1]);
+}
+
+// Phase 3: the epilogue of this thread's elements (plain store, RK4 or RKF45
+// stage combine) from its derivatives dx and the prefetched operands at
+// Pre; the RKF45 stage-5 error is folded into emax (max of |y4 - y5|, or of
+// its square in mixed precision).  coef holds the 24 RKF45 coefficients in
+// FP64 followed by the same 24 in FP32.
+template <int N, int KT, bool MIXED, int BT, bool RKF>
+__device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap<N, KT, MIXED, BT, RKF> &m,
+                                              const TileIn<N, KT, MIXED, BT, RKF> &in, const unsigned char *Pre,
+                                              const double *coef, unsigned long long *wmax, long long tile,
+                                              long long n0, int ycur, double &emax,
+                                              const typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using TX = typename TileArith<MIXED>::TX;
+  using R = typename TileArith<MIXED>::R;
+  constexpr int E = S::E, ES = S::ES, RR = S::RR;
   const int tid = threadIdx.x;
-  const int tile_elems = nt_here * E;
-  auto uix = [](int e) {
-    if (NP == N) return e;
-    const int nd = e / E, w = e - nd * E, cc = w / N;
-    return nd * EU + (w - cc * N) + cc * NP;
+  // Element r of this thread: m.xo[r] in the tile's X / k ranges, m.eo(r) in
+  // its complex128 ranges (and in the operands staged from either).
+  const long long gx0 = n0 * ES, gd0 = n0 * E;
+  const uint32_t off1 = tile_pre_off<N, KT, MIXED, BT, RKF>(p, 1);
+  const uint32_t offs = tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[1]);
+  const double2 *pre0d = reinterpret_cast<const double2 *>(Pre);
+  const TX *pre0x = reinterpret_cast<const TX *>(Pre);
+  // New filter flags follow: |y_new|^2 of every element goes to its slot of
+  // the exchange tile once every thread has read its transposed elements.
+  const bool flags = p.c.filtered && p.stage == (RKF ? 5 : 3) && (RKF || p.mode == kModeRk4);
+  if (flags) __syncthreads();
+  auto fl_put = [&](int r, double2 v) {
+    *reinterpret_cast<double *>(&in.Us[m.uo(r)]) = fma(v.x, v.x, v.y * v.y);
   };
-  auto flag_stage = [&]() {
-    return c.filtered && ((p.mode == kModeRk4 && p.stage == 3) || (p.mode == kModeRkf45 && p.stage == 5));
-  };
-  // element e of the tile: node nd = e / E, offset w = e % E; complex128
-  // buffers are indexed (n0 + nd) * E + w, X / k buffers (n0 + nd) * ES + w.
-  auto preD = [&](int b) { return reinterpret_cast<const double2 *>(PreBase + pre_off[b]); };
-  // RKF45 operand slot 0 is the state y: 16 bytes -> y staged in complex128;
-  // 8 bytes (mixed stages 1-4) -> its complex64 copy y32, which is all the
-  // complex64 stage input X_{s+1} = y + sum b k needs; 0 bytes -> y read from
-  // global memory in the epilogue (mixed stage 5, and the 24-site FP64
-  // kernels' stages 3-5: less shared memory per tile, more CTAs per SM).
-  const int ybytes = p.npre > 0 ? p.pre_bytes[0] : 16;
-  auto preX = [&](int b) { return reinterpret_cast<const TX *>(PreBase + pre_off[b]); };
-  // Filtering: |y_new|^2 of element e goes to the first 8 bytes of its own
-  // slot Us[uix(e)], which only this thread reads, and only before; the
-  // per-node maxima are taken from there after the loop.
-  auto fl_put = [&](int e, double2 v) {
-    *reinterpret_cast<double *>(&Us[uix(e)]) = fma(v.x, v.x, v.y * v.y);
-  };
-  if (p.mode == kModeApply) {
-    TX *out = static_cast<TX *>(p.out);
+  if (!RKF && p.mode == kModeApply) {
+    TX *out = static_cast<TX *>(p.out) + gx0;
     bool dot = false;
     if constexpr (!MIXED) dot = p.dot_w != nullptr;
     if (!dot) {
-      for (int e = tid; e < tile_elems; e += BT) {
-        const int nd = e / E, w = e - nd * E;
-        st_stream(out + (n0 + nd) * ES + w, Us[uix(e)]);
-      }
+#pragma unroll
+      for (int r = 0; r < RR; ++r)
+        if (m.on(r, in.nt_here)) st_stream(out + m.xo[r], dx[r]);
     } else if constexpr (!MIXED) {
       // Steady-state solve: the output's element (0,0) of node 0 is the
       // eliminated unknown (zero), and the tile's share of <dot_w, out> (the
       // real inner product of Hermitian states) goes to dot_part[tile] --
       // the inner product the solver would otherwise read the vector for.
       double dsum = 0.0;
-      for (int e = tid; e < tile_elems; e += BT) {
-        const int nd = e / E, w = e - nd * E;
-        const long long gx = (n0 + nd) * ES + w;
-        TX v = Us[uix(e)];
-        if (gx == 0) v = mk<TX>(0.0, 0.0);
-        st_stream(out + gx, v);
-        const double2 r = __ldg(p.dot_w + gx);
-        dsum = fma(r.x, v.x, fma(r.y, v.y, dsum));
-      }
+#pragma unroll
+      for (int r = 0; r < RR; ++r)
+        if (m.on(r, in.nt_here)) {
+          TX v = dx[r];
+          if (gx0 + m.xo[r] == 0) v = mk<TX>(0.0, 0.0);
+          st_stream(out + m.xo[r], v);
+          const double2 w = __ldg(p.dot_w + gx0 + m.xo[r]);
+          dsum = fma(w.x, v.x, fma(w.y, v.y, dsum));
+        }
       for (int off = 16; off > 0; off >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
       double *wsum = reinterpret_cast<double *>(wmax);
       if ((tid & 31) == 0) wsum[tid >> 5] = dsum;
@@ -492,40 +676,41 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const typenam
         p.dot_part[tile] = t;
       }
     }
-  } else if (p.mode == kModeRk4) {
+  } else if (!RKF) {  // RK4
     const int s = p.stage;
-    TX *out = static_cast<TX *>(p.out);
+    TX *out = static_cast<TX *>(p.out) + gx0;
     long long row = -1;
     if (s == 3 && n0 == 0 && p.traj) {
       const Rk4Ctl *rc = p.rk4;
       if (rc->out_factor > 0 && rc->step % rc->out_factor == 0 && rc->nout < rc->capacity) row = rc->nout;
     }
-    for (int e = tid; e < tile_elems; e += BT) {
-      const int nd = e / E, w = e - nd * E;
-      const long long gd = (n0 + nd) * E + w, gx = (n0 + nd) * ES + w;
-      const double2 kv = to_d2(Us[uix(e)]);
+    const double2 *pre1d = reinterpret_cast<const double2 *>(Pre + off1);
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      if (!m.on(r, in.nt_here)) continue;
+      const int x = m.xo[r], e = m.eo(r);
+      const TX kx = dx[r];
       if (MIXED && s < 3) {
         // Mixed: the complex64 stage input y32 + a k in FP32 (stage 0: y32
         // is the input; stages 1-2: pre = {y32, acc}); the accumulator in
         // FP64 (stage 0: pre = {y}).
         const float af = (float)p.a_next;
-        const TX kx = Us[uix(e)];
-        const TX ys = s == 0 ? Xs[nd * ES + w] : preX(0)[nd * ES + w];
-        out[gx] = mk<TX>(fmaf((float)kx.x, af, (float)ys.x), fmaf((float)kx.y, af, (float)ys.y));
-        st_stream(p.acc + gd, cfma((s == 0 ? preD(0) : preD(1))[e], kv, p.w_acc));
+        const TX ys = s == 0 ? in.Xs[x] : pre0x[x];
+        out[x] = mk<TX>(fmaf((float)kx.x, af, (float)ys.x), fmaf((float)kx.y, af, (float)ys.y));
+        st_stream(p.acc + gd0 + e, cfma((s == 0 ? pre0d : pre1d)[e], to_d2(kx), p.w_acc));
       } else if (s == 0) {  // FP64: pre = {} (y is the input)
-        const double2 ys = to_d2(Xs[nd * ES + w]);
-        out[gx] = from_d2<TX>(cfma(ys, kv, p.a_next));
-        st_stream(p.acc + gd, cfma(ys, kv, p.w_acc));
+        const double2 ys = to_d2(in.Xs[x]);
+        out[x] = from_d2<TX>(cfma(ys, to_d2(kx), p.a_next));
+        st_stream(p.acc + gd0 + e, cfma(ys, to_d2(kx), p.w_acc));
       } else if (s < 3) {  // pre = {y, acc}
-        out[gx] = from_d2<TX>(cfma(preD(0)[e], kv, p.a_next));
-        st_stream(p.acc + gd, cfma(preD(1)[e], kv, p.w_acc));
+        out[x] = from_d2<TX>(cfma(pre0d[e], to_d2(kx), p.a_next));
+        st_stream(p.acc + gd0 + e, cfma(pre1d[e], to_d2(kx), p.w_acc));
       } else {             // pre = {acc}
-        const double2 yn = cfma(preD(0)[e], kv, p.w_acc);
-        p.y[gd] = yn;
-        if (MIXED) static_cast<TX *>(p.y32)[gx] = from_d2<TX>(yn);
+        const double2 yn = cfma(pre0d[e], to_d2(kx), p.w_acc);
+        p.y[gd0 + e] = yn;
+        if (MIXED) static_cast<TX *>(p.y32)[gx0 + x] = from_d2<TX>(yn);
         if (row >= 0 && e < E) p.traj[row * E + e] = yn;
-        if (flag_stage()) fl_put(e, yn);
+        if (flags) fl_put(r, yn);
       }
     }
     if (s == 3 && n0 == 0 && p.traj) {
@@ -536,73 +721,82 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const typenam
         rc->step = rc->step + 1;
       }
     }
-  } else {
+  } else if (p.stage < 5) {
+    // RKF45 stages 0-4: k_s and X_{s+1} = y + sum b k, in the storage type's
+    // arithmetic (a complex64 stage input combined in FP32 differs from an
+    // FP64 combine rounded to it by an ulp of complex64).  pre = {y, k_0 ..
+    // k_{s-1}} (stage 0: y is the input); y is staged as y32 (mixed), staged
+    // in complex128, or read from global memory (0 bytes).
     const int s = p.stage;
+    TX *out = static_cast<TX *>(p.out) + gx0, *ks = static_cast<TX *>(p.k[s]) + gx0;
+    const R *cf = MIXED ? reinterpret_cast<const R *>(coef + 24) : reinterpret_cast<const R *>(coef);
+    cf += s * (s + 1) / 2;
+    TX xv[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const int x = m.xo[r];
+      if (s == 0) {
+        xv[r] = in.Xs[x];
+      } else if (MIXED || p.pre_bytes[0] != 0) {
+        xv[r] = pre0x[x];
+      } else {
+        xv[r] = m.on(r, in.nt_here) ? from_d2<TX>(__ldg(p.ybuf[ycur] + gd0 + x)) : mk<TX>(0.0, 0.0);
+      }
+    }
+    const TX *kb = reinterpret_cast<const TX *>(Pre + off1);
+#pragma unroll 1
+    for (int b = 0; b < s; ++b) {
+      const R cb = cf[b];
+#pragma unroll
+      for (int r = 0; r < RR; ++r) {
+        const TX kr = kb[m.xo[r]];
+        xv[r].x = fma(kr.x, cb, xv[r].x);
+        xv[r].y = fma(kr.y, cb, xv[r].y);
+      }
+      kb = reinterpret_cast<const TX *>(reinterpret_cast<const unsigned char *>(kb) + offs);
+    }
+    const R cs = cf[s];
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (m.on(r, in.nt_here)) {
+        const int x = m.xo[r];
+        st_stream(ks + x, dx[r]);
+        out[x] = mk<TX>(fma(dx[r].x, cs, xv[r].x), fma(dx[r].y, cs, xv[r].y));
+      }
+  } else {
+    // RKF45 stage 5: pre = {y (or read from global), k0, k2, k3, k4}.
     const double *cf = coef;
-    TX *out = static_cast<TX *>(p.out);
-    for (int e = tid; e < tile_elems; e += BT) {
-      const int nd = e / E, w = e - nd * E;
-      const long long gd = (n0 + nd) * E + w, gx = (n0 + nd) * ES + w;
-      const TX kx = Us[uix(e)];
-      const double2 kv = to_d2(kx);
-      if (MIXED && s < 5) {
-        // Mixed stages 0-4: the complex64 stage input X_{s+1} = y32 + sum b k
-        // in FP32 throughout (it is stored in complex64; an FP64 combine
-        // rounded to it differs by an ulp of complex64).  pre = {y32, k_0 ..
-        // k_{s-1}}; stage 0: y32 is the input.
-        const float *cff = reinterpret_cast<const float *>(coef + 24);
-        const TX ys = s == 0 ? Xs[nd * ES + w] : preX(0)[nd * ES + w];
-        st_stream(static_cast<TX *>(p.k[s]) + gx, kx);
-        const int row = s * (s + 1) / 2;
-        float xr = ys.x, xi = ys.y;
+    const TX *kb = reinterpret_cast<const TX *>(Pre + off1);
+    const uint32_t ksz = offs / sizeof(TX);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-          if (r < s) {
-            const TX kr = preX(1 + r)[nd * ES + w];
-            xr = fmaf((float)kr.x, cff[row + r], xr);
-            xi = fmaf((float)kr.y, cff[row + r], xi);
-          }
-        xr = fmaf((float)kx.x, cff[row + s], xr);
-        xi = fmaf((float)kx.y, cff[row + s], xi);
-        out[gx] = mk<TX>(xr, xi);
-      } else if (s < 5) {  // pre = {y, k_0 .. k_{s-1}}; stage 0: y is the input
-        const double2 ys = s == 0 ? to_d2(Xs[nd * ES + w])
-                           : (ybytes == 0 ? __ldg(p.ybuf[ycur] + gd)
-                                          : (ybytes == 8 ? to_d2(preX(0)[nd * ES + w]) : preD(0)[e]));
-        st_stream(static_cast<TX *>(p.k[s]) + gx, kx);
-        const int row = s * (s + 1) / 2;
-        double2 xv = ys;
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-          if (r < s) xv = cfma(xv, to_d2(preX(1 + r)[nd * ES + w]), cf[row + r]);
-        xv = cfma(xv, kv, cf[row + s]);
-        out[gx] = from_d2<TX>(xv);
-      } else {      // pre = {y, k0, k2, k3, k4}
-        const double2 ys = ybytes == 0 ? __ldg(p.ybuf[ycur] + gd) : preD(0)[e];
-        const double2 k0 = to_d2(preX(1)[nd * ES + w]), k2 = to_d2(preX(2)[nd * ES + w]);
-        const double2 k3 = to_d2(preX(3)[nd * ES + w]), k4 = to_d2(preX(4)[nd * ES + w]);
-        double2 y4 = cfma(ys, k0, cf[15]);
-        y4 = cfma(y4, k2, cf[16]);
-        y4 = cfma(y4, k3, cf[17]);
-        y4 = cfma(y4, k4, cf[18]);
-        double2 y5 = cfma(ys, k0, cf[19]);
-        y5 = cfma(y5, k2, cf[20]);
-        y5 = cfma(y5, k3, cf[21]);
-        y5 = cfma(y5, k4, cf[22]);
-        y5 = cfma(y5, kv, cf[23]);
-        st_stream(p.ybuf[ycur ^ 1] + gd, y5);
-        if (MIXED) st_stream(static_cast<TX *>(p.y32buf[ycur ^ 1]) + gx, from_d2<TX>(y5));
-        if (flag_stage()) fl_put(e, y5);
-        const double dx = y4.x - y5.x, dy = y4.y - y5.y;
-        if (MIXED) {
-          // max of |y4 - y5|^2; one square root per thread below
-          const double e2 = fma(dx, dx, dy * dy);
-          emax = (e2 > emax || e2 != e2) ? e2 : emax;
-        } else {
-          // |z| as PHI computes it (std::abs of the complex difference)
-          const double err = hypot(dx, dy);
-          emax = (err > emax || err != err) ? err : emax;
-        }
+    for (int r = 0; r < RR; ++r) {
+      if (!m.on(r, in.nt_here)) continue;
+      const int x = m.xo[r], e = m.eo(r);
+      const double2 kv = to_d2(dx[r]);
+      const double2 ys = p.pre_bytes[0] == 0 ? __ldg(p.ybuf[ycur] + gd0 + e) : pre0d[e];
+      const double2 k0 = to_d2(kb[x]), k2 = to_d2(kb[ksz + x]);
+      const double2 k3 = to_d2(kb[2 * ksz + x]), k4 = to_d2(kb[3 * ksz + x]);
+      double2 y4 = cfma(ys, k0, cf[15]);
+      y4 = cfma(y4, k2, cf[16]);
+      y4 = cfma(y4, k3, cf[17]);
+      y4 = cfma(y4, k4, cf[18]);
+      double2 y5 = cfma(ys, k0, cf[19]);
+      y5 = cfma(y5, k2, cf[20]);
+      y5 = cfma(y5, k3, cf[21]);
+      y5 = cfma(y5, k4, cf[22]);
+      y5 = cfma(y5, kv, cf[23]);
+      st_stream(p.ybuf[ycur ^ 1] + gd0 + e, y5);
+      if (MIXED) st_stream(static_cast<TX *>(p.y32buf[ycur ^ 1]) + gx0 + x, from_d2<TX>(y5));
+      if (flags) fl_put(r, y5);
+      const double ex = y4.x - y5.x, ey = y4.y - y5.y;
+      if (MIXED) {
+        // max of |y4 - y5|^2; one square root per thread below
+        const double e2 = fma(ex, ex, ey * ey);
+        emax = (e2 > emax || e2 != e2) ? e2 : emax;
+      } else {
+        // |z| as PHI computes it (std::abs of the complex difference)
+        const double err = hypot(ex, ey);
+        emax = (err > emax || err != err) ? err : emax;
       }
     }
   }
@@ -633,18 +827,18 @@ __device__ __forceinline__ void tile_error_max(const TileParams &p, double emax,
 
 // New filter flags of a tile's nodes after the stage that writes the new
 // state (RK4 stage 3, RKF45 stage 5).
-template <int N, int KT, bool MIXED, int BT>
+template <int N, int KT, bool MIXED, int BT, bool RKF>
 __device__ __forceinline__ void tile_flags(const TileParams &p, const typename TileArith<MIXED>::TX *Us, long long n0,
                                            int nt_here, int ycur) {
-  using S = TileShape<N, MIXED, KT, BT>;
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
   using TX = typename TileArith<MIXED>::TX;
   const HeomConsts &c = p.c;
-  if (!(c.filtered && ((p.mode == kModeRk4 && p.stage == 3) || (p.mode == kModeRkf45 && p.stage == 5)))) return;
+  if (!(c.filtered && p.stage == (RKF ? 5 : 3) && (RKF || p.mode == kModeRk4))) return;
   // Below the tolerance -> inactive, above -> active, equal -> unchanged
   // (hierarchy_integrator.cc:2827-2850, :2359-2384).
   __syncthreads();
-  const int ap = p.mode == kModeRkf45 ? ycur : p.act_par;
-  tile_filter_flags(reinterpret_cast<const unsigned char *>(Us), (int)sizeof(TX), N, S::NP, nt_here,
+  const int ap = RKF ? ycur : p.act_par;
+  tile_filter_flags(reinterpret_cast<const unsigned char *>(Us), (int)sizeof(TX), N, S::NP, S::EU, nt_here,
                     p.act[ap] + n0, p.act[ap ^ 1] + n0, c.filter_tol, BT / 32);
 }
 
@@ -653,74 +847,38 @@ __device__ __forceinline__ void tile_flags(const TileParams &p, const typename T
 // One tile (NT consecutive nodes of one hierarchy) of one stage.  The caller
 // has initialised the two mbarriers at the start of shared memory and passes
 // the phase parity each is at.  Returns 1 when the tile was skipped before
-// any copy was issued (RKF45 run finished), 0 when both barriers completed a
+// any copy was issued, 0 when both barriers completed a
 // phase (barrier 1 with 0 bytes when p.npre == 0), -1 after a bounded wait gave up
 // (err_flag set; the caller must stop).
 template <int N, int KT, bool MIXED, int BT = kTileThreads>
 __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, unsigned char *smem_raw,
                                          uint32_t par0, uint32_t par1) {
-  using S = TileShape<N, MIXED, KT, BT>;
-  using Lay = TileLayout<N, MIXED, KT, BT>;
+  constexpr bool RKF = false;  // apply and RK4 stages
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using Lay = TileLayout<N, MIXED, KT, BT, RKF>;
   using TX = typename std::conditional<MIXED, float2, double2>::type;
   using R = typename std::conditional<MIXED, float, double>::type;
-  constexpr int E = S::E, P = S::P, NT = S::NT, ES = Lay::ES;
+  constexpr int E = S::E, NT = S::NT, ES = Lay::ES;
+  using In = TileIn<N, KT, MIXED, BT, RKF>;
   const HeomConsts &c = p.c;
   constexpr int T = N * KT;  // PHI's identity site map: K+1 terms per site
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + Lay::kBars);
   TX *Xs = reinterpret_cast<TX *>(smem_raw + Lay::kX);   // NT*ES
   TX *Us = reinterpret_cast<TX *>(smem_raw + Lay::kU);   // NT*EU (column stride NP)
   unsigned char *PreBase = smem_raw + Lay::kPre;
-  // Byte offsets of the prefetched epilogue operands.  Every loop over them
-  // is unrolled so the offsets stay in registers.
-  uint32_t pre_off[kMaxPre];
-  size_t tail = Lay::kPre;
-  {
-    uint32_t acc_off = 0;
-#pragma unroll
-    for (int b = 0; b < kMaxPre; ++b) {
-      pre_off[b] = acc_off;
-      if (b < p.npre) acc_off += ((uint32_t)NT * (p.pre_bytes[b] == 16 ? E : ES) * p.pre_bytes[b] + 127) / 128 * 128;
-    }
-    tail += acc_off;
-  }
+  const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, RKF>(p, p.npre) : 0);
   TX *Hs = reinterpret_cast<TX *>(smem_raw + tail);                 // E
-  double *deph = reinterpret_cast<double *>(Hs + E);                // NT (8-aligned: E*8 or E*16)
-  double *coef = deph + NT;                                         // 24, then 24 floats
-  unsigned long long *wmax = reinterpret_cast<unsigned long long *>(coef + 36);  // per-warp maxima
-  R *cn = reinterpret_cast<R *>(wmax + (BT / 32));                          // NT*T |next prefactor|
-  R *cp = cn + NT * T;                                              // NT*T prev scale
-  R *ccr = cp + NT * T;                                             // 2T   c_t (re, im)
-  R *mats = ccr + 2 * T;                                            // E    Matsubara factor per element
-  int *ids = reinterpret_cast<int *>(mats + E);                     // NT*2T element offsets
-  int *nts = ids + NT * 2 * T;                                      // NT*T
-  unsigned char *pi = reinterpret_cast<unsigned char *>(nts + NT * T);
-  unsigned char *pj = pi + P;
+  double *deph = reinterpret_cast<double *>(Hs + E + (E & 1));       // NT (16-aligned)
+  unsigned long long *wmax = reinterpret_cast<unsigned long long *>(deph + NT + (NT & 1));  // per-warp sums
+  typename In::C *cfs = reinterpret_cast<typename In::C *>(wmax + tile_warp_slots(BT));  // NT*T neighbour coefficients
+  R *mats = reinterpret_cast<R *>(cfs + NT * T);                    // E    Matsubara factor per element
+  int2 *ids = reinterpret_cast<int2 *>(mats + E + (E & 1));         // NT*T element offsets (next, prev)
 
   const int tid = threadIdx.x;
-  int ycur = 0;
-  if (p.mode == kModeRkf45) {
-    if (*(volatile int *)&p.ctl->done) return 1;  // uniform across the grid
-    ycur = p.ctl->ycur;
-    if (tid < 24) {
-      const double v = p.ctl->coef[tid];
-      coef[tid] = v;
-      reinterpret_cast<float *>(coef + 24)[tid] = (float)v;
-    }
-  }
   const long long n0 = tile * NT;
   if (n0 >= c.M) return 1;
-  // Filtering: the flags of the current state are p.act[ap], ap = ycur
-  // (RKF45) or p.act_par; the launch that writes the new state (RK4 stage 3,
-  // RKF45 stage 5 -- the candidate, kept on accept) writes its flags to
-  // p.act[ap ^ 1].  Both are recomputed from the parameters where used, so
-  // nothing of it stays live across the tile.
-  auto act_idx = [&]() { return p.mode == kModeRkf45 ? ycur : p.act_par; };
   const int nt_here = (int)((c.M - n0) < NT ? (c.M - n0) : NT);
-  const TX *xin;
-  if (p.mode == kModeRkf45 && p.stage == 0)
-    xin = MIXED ? static_cast<const TX *>(p.y32buf[ycur]) : reinterpret_cast<const TX *>(p.ybuf[ycur]);
-  else
-    xin = static_cast<const TX *>(p.x);
+  const TX *xin = static_cast<const TX *>(p.x);
 
   // ---- t = 0: bulk prefetch of the tile's contiguous ranges ----
   if (tid == 0) {
@@ -737,13 +895,10 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
 #pragma unroll
     for (int b = 0; b < kMaxPre; ++b) {
       if (b >= p.npre) break;
-      if (p.pre_bytes[b] == 0) continue;  // read from global in the epilogue
       const unsigned char *src = static_cast<const unsigned char *>(p.pre[b]);
-      if (b == 0 && p.mode == kModeRkf45)
-        src = static_cast<const unsigned char *>(p.pre_bytes[0] == 8 ? p.y32buf[ycur] : (const void *)p.ybuf[ycur]);
       const int stride = p.pre_bytes[b] == 16 ? E : ES;
       const uint32_t bytes = (uint32_t)(nt_here * stride * p.pre_bytes[b]);
-      bulk_g2s(PreBase + pre_off[b], src + (size_t)n0 * stride * p.pre_bytes[b], bytes, &bars[1]);
+      bulk_g2s(PreBase + tile_pre_off<N, KT, MIXED, BT, RKF>(p, b), src + (size_t)n0 * stride * p.pre_bytes[b], bytes, &bars[1]);
     }
   }
   // A real Hamiltonian (every in-scope workload) is kept as E reals in the
@@ -756,45 +911,28 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
     for (int i = tid; i < E; i += BT) Hs[i] = from_d2<TX>(__ldg(c.H + i));
   }
   for (int i = tid; i < E; i += BT) mats[i] = (R)__ldg(c.mats_elem + i);
-  for (int i = tid; i < P; i += BT) {
-    pi[i] = __ldg(c.pair_i + i);
-    pj[i] = __ldg(c.pair_j + i);
-  }
   const int W = c.L + 2;
   const int tile_terms = nt_here * T;
   // Per (node, term): neighbour ids scaled to element offsets of the stage
   // input (-1 when absent), occupation, and the prefactor magnitudes for that
   // occupation, so the pair loop reads shared memory only.
-  const uint8_t *act_in = c.filtered ? p.act[act_idx()] : nullptr;
+  const uint8_t *act_in = c.filtered ? p.act[p.act_par] : nullptr;
   for (int q = tid; q < tile_terms; q += BT) {
-    const int nd = q / T, t = q - nd * T;
+    const int t = q % T;
     const int nx = __ldg(c.next + n0 * T + q), pv = __ldg(c.prev + n0 * T + q);
     const int nt = __ldg(c.mi + n0 * T + q);
     // An inactive neighbour contributes nothing (the DoNext / DoPrevious
     // overrides of IndependentBathAdaptiveTruncation, hierarchy_updater.cc:256-303).
     const bool nx_on = nx >= 0 && (!act_in || __ldg(act_in + nx));
     const bool pv_on = pv >= 0 && (!act_in || __ldg(act_in + pv));
-    ids[nd * 2 * T + t] = nx_on ? nx * ES : -1;
-    ids[nd * 2 * T + T + t] = pv_on ? pv * ES : -1;
-    nts[q] = nt;
-    cn[q] = (R)__ldg(c.sq_next + t * W + nt);
-    cp[q] = (R)__ldg(c.sq_prev + t * W + nt);
+    ids[q] = make_int2(nx_on ? nx * ES : -1, pv_on ? pv * ES : -1);
+    cfs[q] = tile_coef<typename In::C, R>((R)__ldg(c.sq_next + t * W + nt), (R)__ldg(c.sq_prev + t * W + nt),
+                                          __ldg(c.corr + t));
   }
-  for (int t = tid; t < T; t += BT) {
-    const double2 ct = __ldg(c.corr + t);
-    ccr[2 * t] = (R)ct.x;
-    ccr[2 * t + 1] = (R)ct.y;
-  }
-  __syncthreads();  // barrier init and metadata visible
-  if (tid < nt_here) {
-    double d = 0.0;
-    for (int t = 0; t < T; ++t) d = fma((double)nts[tid * T + t], __ldg(c.nu + t), d);
-    deph[tid] = d;
-  }
+  if (tid < nt_here) deph[tid] = __ldg(c.deph_node + n0 + tid);
   const long long polls0 = c.first_wait_polls == 0 ? kMaxPolls : (c.first_wait_polls < 0 ? 0 : c.first_wait_polls);
   bool ok = mbar_wait_bounded(&bars[0], par0, polls0);
-  __syncthreads();  // deph visible
-  if (!__syncthreads_and(ok)) {
+  if (!__syncthreads_and(ok)) {  // metadata visible as well
     if (tid == 0) atomicOr(c.err_flag, 1);
     // Drain this tile's own copies with the built-in limit, so no copy is
     // still writing into shared memory when the CTA stops.
@@ -803,36 +941,57 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
     return -1;
   }
 
-  tile_pairs<N, KT, MIXED, BT>(c, Xs, Us, Hs, mats, pi, pj, ids, cn, cp, ccr, deph, nts, xin, nt_here);
+  const TileMap<N, KT, MIXED, BT, RKF> m(c);
+  const In in{Xs, Us, Hs, mats, ids, cfs, deph, c.mi + n0 * T, xin, nt_here};
+  TX dx[S::RR];
+  tile_derivative<N, KT, MIXED, BT, RKF>(c, m, in, dx);
   ok = p.npre == 0 || mbar_wait_bounded(&bars[1], par1);
   if (!__syncthreads_and(ok)) {
     if (tid == 0) atomicOr(c.err_flag, 1);
     return -1;
   }
   double emax = 0.0;
-  tile_epilogue<N, KT, MIXED, BT>(p, Xs, Us, PreBase, pre_off, coef, wmax, tile, n0, nt_here, ycur, emax);
-  if (p.mode == kModeRkf45 && p.stage == 5) tile_error_max<MIXED, BT>(p, emax, wmax);
-  tile_flags<N, KT, MIXED, BT>(p, Us, n0, nt_here, ycur);
+  tile_epilogue<N, KT, MIXED, BT, RKF>(p, m, in, PreBase, nullptr, wmax, tile, n0, 0, emax, dx);
+  tile_flags<N, KT, MIXED, BT, RKF>(p, Us, n0, nt_here, 0);
   return 0;
 }
 
-template <int N, int KT, bool MIXED, int BT = kTileThreads>
+template <int N, int KT, bool MIXED, int BT = kTileThreads, bool RKF = false>
 inline size_t tile_smem(int T, int npre, const int *pre_bytes) {
-  using S = TileShape<N, MIXED, KT, BT>;
-  using Lay = TileLayout<N, MIXED, KT, BT>;
+  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using Lay = TileLayout<N, MIXED, KT, BT, RKF>;
   size_t b = Lay::kPre;
-  for (int i = 0; i < npre; ++i)
-    b += ((size_t)S::NT * (pre_bytes[i] == 16 ? S::E : Lay::ES) * pre_bytes[i] + 127) / 128 * 128;
-  b += (size_t)S::E * Lay::XB;
-  b += (size_t)(S::NT + 36 + BT / 32) * sizeof(double);  // deph, coef (FP64 and FP32), warp maxima
-  b += (size_t)(2 * S::NT * T + 2 * T + S::E) * Lay::XB / 2;  // cn, cp, ccr, mats in the arithmetic type
-  b += (size_t)(S::NT * 3 * T) * sizeof(int);
-  b += 2 * S::P + 16;
+  for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, RKF>(pre_bytes[i]);
+  b += (size_t)(S::E + (S::E & 1)) * Lay::XB;
+  b += (size_t)(S::NT + (S::NT & 1) + tile_warp_slots(BT)) * sizeof(double);  // deph, warp sums
+  b += (size_t)S::NT * T * sizeof(typename TileIn<N, KT, MIXED, BT, RKF>::C);
+  b += (size_t)(S::E + (S::E & 1)) * Lay::XB / 2;                     // mats
+  b += (size_t)S::NT * T * sizeof(int2);                              // ids
+  b += 16;
   return b;
 }
 
+// Threads per CTA of the single-instance kernel: 320 for the 24-site mixed
+// kernel (a node's 300 pairs in one pass, two nodes per tile: timed on B200,
+// its RKF45 step 1.65 -> 1.56 ms), 256 otherwise (320 everywhere was slower
+// on the 7-site and the batched workloads).  The batched kernel always runs
+// 256, so its tile counts (tile_count) use that.
+template <int N, bool MIXED>
+struct TileBlock {
+  static constexpr int threads = (MIXED && N == 24) ? 320 : kTileThreads;
+  // The autotuner's alternative block size (heom_tile.cu, tile_autotune).
+  static constexpr int alt = threads == kTileThreads ? 320 : kTileThreads;
+};
+
 // The tile parameters of one stage launch (host; heom_tile.cu).
 TileParams tile_params_for(const StageLaunch &L);
+
+// Launches of the single-instance kernel (heom_tile_*_*.cu); *per_sm
+// (optional) receives the resident CTAs per SM before the schedule's cap.
+cudaError_t launch_tile_fp64_rk4(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_fp64_rkf45(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_mixed_rk4(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_mixed_rkf45(const TileParams &p, cudaStream_t stream, int *per_sm);
 
 }  // namespace tile_detail
 }  // namespace phi

@@ -1,0 +1,10 @@
+// The tile kernel's mixed-precision instantiations: RKF45 stages.
+#include "heom_tile_pipe.cuh"
+
+namespace phi {
+namespace tile_detail {
+cudaError_t launch_tile_mixed_rkf45(const TileParams &p, cudaStream_t stream, int *per_sm) {
+  return launch_tile_dispatch<true, true>(p, stream, per_sm);
+}
+}  // namespace tile_detail
+}  // namespace phi

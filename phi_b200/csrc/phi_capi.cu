@@ -280,9 +280,15 @@ void set_create_error(const std::string &msg) { g_create_error = msg; }
 namespace {
 
 // Tile-kernel schedules chosen so far in this process, per (device, N, K+1,
-// arithmetic, log2 of the node count).
+// arithmetic and kind of stage, log2 of the node count).
 std::mutex g_sched_mu;
 std::map<std::tuple<int, int, int, int, int>, phi::TileSchedule> g_sched;
+
+std::tuple<int, int, int, int, int> sched_key(const phi_ctx *ctx, bool rkf45) {
+  int lg = 0;
+  for (long long m = ctx->hier.M; m > 1; m >>= 1) ++lg;
+  return std::make_tuple(ctx->desc.device, ctx->desc.num_states, ctx->c.K1, (ctx->mixed() ? 1 : 0) + (rkf45 ? 2 : 0), lg);
+}
 constexpr long long kTuneMinElements = 1ll << 20;  // smaller problems keep the default schedule
 
 // The tile-shape autotuner: for a tile-eligible problem of at least
@@ -294,9 +300,7 @@ int tune_tile_schedule(phi_ctx *ctx) {
   if (!phi::tile_kernel_available(ctx->c)) return PHI_OK;
   const int N = ctx->desc.num_states;
   if (ctx->hier.M * N * N < kTuneMinElements) return PHI_OK;
-  int lg = 0;
-  for (long long m = ctx->hier.M; m > 1; m >>= 1) ++lg;
-  const auto key = std::make_tuple(ctx->desc.device, N, ctx->c.K1, ctx->mixed() ? 1 : 0, lg);
+  const auto key = sched_key(ctx, false);
   {
     std::lock_guard<std::mutex> lock(g_sched_mu);
     auto it = g_sched.find(key);
@@ -337,6 +341,37 @@ int tune_tile_schedule(phi_ctx *ctx) {
   g_sched[key] = sched;
   return PHI_OK;
 }
+
+}  // namespace
+
+// The schedule of the RKF45 stages, chosen before the first RKF45 step of a
+// context: the same choice as at creation, timed on `stage` (a launch whose
+// outputs the run overwrites).
+int phi_ctx::tune_rkf45(const phi::StageLaunch &stage) {
+  if (rkf45_tuned) return PHI_OK;
+  rkf45_tuned = true;
+  if (!phi::tile_kernel_available(c) || hier.M * c.N * c.N < kTuneMinElements) return PHI_OK;
+  const auto key = sched_key(this, true);
+  phi::TileSchedule sched;
+  bool known = false;
+  {
+    std::lock_guard<std::mutex> lock(g_sched_mu);
+    auto it = g_sched.find(key);
+    known = it != g_sched.end();
+    if (known) sched = it->second;
+  }
+  if (!known) {
+    const cudaError_t e = phi::tile_autotune(stage, stream, &sched);
+    if (e != cudaSuccess) return cuda_fail(this, e, "tile schedule");
+    std::lock_guard<std::mutex> lock(g_sched_mu);
+    g_sched[key] = sched;
+  }
+  c.tile_variant_rkf = sched.variant;
+  c.tile_cps_rkf = sched.cps;
+  return PHI_OK;
+}
+
+namespace {
 
 }  // namespace
 
@@ -820,8 +855,9 @@ extern "C" int phi_gpu_set_tile_schedule(phi_ctx *ctx, int32_t threads, int32_t 
                  " and ctas_per_sm >= 0";
     return PHI_E_INVALID;
   }
-  ctx->c.tile_variant = variant;
-  ctx->c.tile_cps = ctas_per_sm;
+  ctx->c.tile_variant = ctx->c.tile_variant_rkf = variant;
+  ctx->c.tile_cps = ctx->c.tile_cps_rkf = ctas_per_sm;
+  ctx->rkf45_tuned = true;
   ctx->release_graphs();  // captured launches carry the old schedule
   return PHI_OK;
 }

@@ -116,6 +116,8 @@ struct phi_ctx {
   // problems of at least kTuneMinElements elements; the choice is also in
   // c.tile_variant / c.tile_cps).
   phi::TileSchedule tile_sched{};
+  bool rkf45_tuned = false;  // the RKF45 stages' schedule is chosen (or set)
+  int tune_rkf45(const phi::StageLaunch &stage);
 
   double time = 0.0;
   std::string error;

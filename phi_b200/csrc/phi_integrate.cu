@@ -146,7 +146,8 @@ cudaError_t enqueue_rk4_step(phi_ctx *ctx, double dt, double2 *traj, int par, cu
   return cudaSuccess;
 }
 
-cudaError_t enqueue_rkf45_step(phi_ctx *ctx, cudaStream_t s) {
+// The launch parameters the RKF45 stages share.
+phi::StageLaunch rkf45_launch(phi_ctx *ctx) {
   phi::StageLaunch L;
   L.c = ctx->c;
   L.mode = phi::kModeRkf45;
@@ -162,6 +163,11 @@ cudaError_t enqueue_rkf45_step(phi_ctx *ctx, cudaStream_t s) {
     L.k[i] = ctx->kbuf[i].as<double2>();
     L.kv[i] = ctx->kbuf[i].ptr;
   }
+  return L;
+}
+
+cudaError_t enqueue_rkf45_step(phi_ctx *ctx, cudaStream_t s) {
+  phi::StageLaunch L = rkf45_launch(ctx);
   double2 *xa = ctx->xa.as<double2>(), *xb = ctx->xb.as<double2>();
   const double2 *in[6] = {nullptr, xa, xb, xa, xb, xa};
   double2 *outb[6] = {xa, xb, xa, xb, xa, nullptr};
@@ -382,6 +388,14 @@ int run_rkf45(phi_ctx *ctx, double dt0, double t_end, double tol, double min_dt,
   if (ctx->mixed())  // stage-0 input of the first step: complex64 copy of y (ycur = 0)
     PHI_CK(phi::launch_to_c64(ctx->y.as<double2>(), ctx->y32.as<float2>(), ctx->hier.M,
                               ctx->desc.num_states * ctx->desc.num_states, ctx->work_stride(), ctx->stream));
+  if (!ctx->rkf45_tuned && !hc.done) {  // stage 4 (its outputs are scratch until the run writes them)
+    phi::StageLaunch L = rkf45_launch(ctx);
+    L.stage = 4;
+    L.xv = L.x = ctx->xb.as<double2>();
+    L.outv = L.out = ctx->xa.as<double2>();
+    rc = ctx->tune_rkf45(L);
+    if (rc != PHI_OK) return rc;
+  }
   if (!ctx->rkf45_graph) {
     PHI_CK(capture(ctx->stream, [&]() {
       for (int i = 0; i < kGraphSteps; ++i) {
