@@ -415,10 +415,9 @@ __device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileI
 // and a run can then end past t_end instead of at it (PHI's clamp does not
 // see a grown step).
 //
-// A_US: the products are already in Us (computed on the tensor cores).
-// Barriers: every thread of the CTA calls; Us must be free (or hold the
-// products, visible) on entry, and is free again after the CTA's next barrier.
-template <int N, int KT, bool MIXED, int BT, bool RKF, bool A_US = false>
+// Barriers: every thread of the CTA calls; Us must be free on entry, and is
+// free again after the CTA's next barrier.
+template <int N, int KT, bool MIXED, int BT, bool RKF>
 __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, RKF> &m,
                                                 const TileIn<N, KT, MIXED, BT, RKF> &in,
                                                 typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
@@ -431,7 +430,6 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
   const TX zero = mk<TX>(0.0, 0.0);
   TX *Us = in.Us;
   if constexpr (S::kPairs) {
-    static_assert(!A_US, "the tensor-core kernel maps by element");
     // Every neighbour value the pairs need, as independent predicated loads,
     // issued before the products, whose work hides their latency, where the
     // registers hold them.
@@ -536,12 +534,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int r = 0; r < RR; ++r) gather(r);
     }
-    if constexpr (A_US) {
-#pragma unroll
-      for (int r = 0; r < RR; ++r) dx[r] = Us[m.uo(r)];
-    } else {
-      tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
-    }
+    tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
       if constexpr (!kHoist) gather(r);
