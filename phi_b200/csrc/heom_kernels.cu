@@ -1,21 +1,33 @@
-// heom_kernels.cu -- the per-node Liouvillian and the fused RK stage kernels.
+// heom_kernels.cu -- the Liouvillian and the fused RK stages for every bath
+// coupling at any N (FP64); identity-site independent baths of the tiled sizes
+// run on heom_tile.cu instead.
 //
-// One "group" of GROUP threads owns one hierarchy node at a time; a 256-thread
-// CTA holds 256/GROUP groups and walks the node range grid-stride.  Per node:
+// A CTA owns a tile of nt consecutive nodes.  Thread t < CS * N works on row
+// i = t % N of the tile's columns t / N, t / N + CS, ... (elements t, t + CS N,
+// ... of the tile), so its reads of ADOs -- its own tile's and the linked
+// ones -- run along contiguous memory.  Per element
+//   B_ij = -i/hbar (H X)_ij + sum_b (V_b M_b)_ij
+//   M_b  = sum_k (-i s X+ - i c sp X-)  over the K + 1 terms of bath b
+//          (+ Delta_b [X, V_b] for full couplings: FullBath::DoMatsubara)
+// and, every ADO being Hermitian,
+//   dX_ij = B_ij + conj(B_ji) - (dephasing + Matsubara_ij) X_ij :
+// PHI's commutators -i/hbar [H, X], -p [V, X+], -pr V X- - pc X- V and
+// -Delta [V, [V, X]] are each a product plus its Hermitian conjugate, and the
+// two factors of a term differ only in V's side, so the terms of a bath are
+// summed before the one product with V_b (a 3-bath full coupling with K = 1
+// takes 10 products per node instead of 37).  An independent bath's V_b is
+// |m><m|: V_b M_b is row m of M_b, the conjugate of its column m, so element
+// (i, j) adds the terms of site j; a diagonal V_b scales row i.  The tile
+// exchanges B through shared memory; the RK stage combine follows in
+// registers.
 //
-//   1. metadata: next/prev ids for every term, the multi-index n_t;
-//   2. own ADO X_n -> shared memory (coalesced, node-major contiguous);
-//      IndependentBath: column m = site(t) of every linked ADO -> shared memory
-//      (a Hermitian ADO's row m is the conjugate of its column m, so the
-//      neighbour terms of PHI's DoNext/DoPrevious, which touch row m and
-//      column m, read only contiguous columns);
-//   3. A = H X_n (the one complex N x N product of the node);
-//   4. upper-triangle pairs (i <= j):
-//        dX_ij = -i/hbar (A_ij - conj(A_ji))         (= -i/hbar [H, X]_ij)
-//                - (dephasing_n + matsubara_ij) X_ij
-//                + neighbour terms
-//      and dX_ji = conj(dX_ij), so every output ADO is exactly Hermitian;
-//   5. an epilogue that is the RK stage combine (RK4 / RKF45) or a plain store.
+// What bounds it (B200): latency.  A stage of these hierarchies is a few
+// thousand nodes or fewer, i.e. one chain of node records -> gathers ->
+// products -> exchange -> combine per CTA.  So the records are read before
+// the wait on the previous stage's kernel (programmatic dependent launch:
+// they are constant), the combine's operands are copied to shared memory
+// asynchronously while the derivative runs, and tiles are cut down until
+// there are two CTAs per SM.
 //
 // Reference: HierarchyUpdater::Get and the IndependentBath / DiagonalBath /
 // FullBath / Vacuum terms (hierarchy_updater.h:36-75,
@@ -24,6 +36,8 @@
 // control (:2010-2482).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "heom_device.cuh"
@@ -34,53 +48,41 @@
 namespace phi {
 namespace {
 
-__device__ __forceinline__ double2 c_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 c_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 c_mul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 c_conj(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double2 c_scale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-// a + b * s for real s.
 __device__ __forceinline__ double2 c_axpy(double2 a, double2 b, double s) {
   return make_double2(fma(b.x, s, a.x), fma(b.y, s, a.y));
 }
-// acc + i * s * b
-__device__ __forceinline__ double2 c_add_i(double2 acc, double2 b, double s) {
-  return make_double2(acc.x - s * b.y, acc.y + s * b.x);
+// Data that a preceding stage kernel wrote: past L1, which may hold lines of a
+// kernel that ran beside this one's preamble.
+__device__ __forceinline__ double2 ld_global(const double2 *p) { return __ldcg(p); }
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
 }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Programmatic dependent launch: the next kernel may start its preamble; this
+// one continues once the previous kernel's writes are visible (both no-ops in
+// a launch without the attribute).
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <int GROUP>
-__device__ __forceinline__ void group_sync(int g) {
-  if (GROUP == 32) {
-    __syncwarp();
-  } else {
-    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(GROUP) : "memory");
-  }
-}
+constexpr int kNodeThreads = 512;   // at most
+constexpr int kNodeRounds = 2;      // elements of a thread whose neighbour sums stay in registers
+constexpr int kNodeMaxOps = 5;      // combine operands
 
-// Shared-memory plan (doubles of complex = 16 B units).
-struct SmemPlan {
-  int E;         // N*N
-  int gcols;     // 2*T*N (independent) or 2*N*N (diagonal/full scratch)
-  int per_group; // complex slots per group
-  int ints_per_group;
+// Shape of a launch and its shared-memory plan (bytes, every region 16-byte
+// aligned).
+struct NodePlan {
+  int threads;   // CTA size
+  int nt;        // nodes per tile
+  int cs;        // columns per round: threads / N
+  int bc;        // full couplings: baths whose M_b are in shared memory at once
+  int stage_ops; // combine operands staged in shared memory (0: read directly)
+  uint32_t x, u, m, v, ops, cf, ids, bytes;
 };
-
-__host__ __device__ inline SmemPlan smem_plan(int N, int T, int kind) {
-  SmemPlan p;
-  p.E = N * N;
-  p.gcols = kind == kIndependent ? 2 * T * N : 2 * N * N;
-  p.per_group = 3 * p.E + p.gcols;
-  // ids[2T], nts[T], then three 8-byte slots at an even int offset (the
-  // node's dephasing rate, its max |y|^2 when filtering, and whether it is
-  // in the deepest tier, for time-local truncation).
-  p.ints_per_group = ((3 * T + 1) & ~1) + 6;
-  return p;
-}
 
 struct StageParams {
   HeomConsts c;
+  NodePlan plan;
   int mode;          // StageMode
   int stage;         // RK stage index
   const double2 *x;  // stage input (node-major)
@@ -96,6 +98,10 @@ struct StageParams {
   double2 *k[5];
   double2 *ybuf[2];
   Rkf45Ctl *ctl;
+  // Combine operands in the order the epilogue reads them; RKF45's operand 0
+  // is the state, chosen on the device.
+  int nops;
+  const double2 *op[kNodeMaxOps];
   // filtering (see StageLaunch)
   uint8_t *act[2];
   int act_par;
@@ -104,403 +110,409 @@ struct StageParams {
   long long x_bstride, out_bstride;
 };
 
-template <int GROUP, int KIND>
-__global__ void __launch_bounds__(256) heom_stage_kernel(StageParams p) {
+// s: next prefactor magnitude; a = (previous scale) * c_t.
+struct alignas(16) NodeCoef {
+  double s, pad, ax, ay;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_constant__ StageParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const HeomConsts &c = p.c;
-  const int N = c.N, E = N * N, T = c.T;
-  constexpr int NG = 256 / GROUP;
-  const int g = threadIdx.x / GROUP, lane = threadIdx.x % GROUP;
-
-  const SmemPlan plan = smem_plan(N, T, KIND);
+  const NodePlan &pl = p.plan;
+  const int N = c.N, E = N * N, T = c.T, tid = threadIdx.x, nth = blockDim.x;
+  const int NP = N | 1;  // odd column stride of the exchange tile: transposed reads in distinct banks
   double2 *Hs = reinterpret_cast<double2 *>(smem_raw);
-  double2 *Xs = Hs + E + (size_t)g * plan.per_group;
-  double2 *As = Xs + E;
-  double2 *Us = As + E;
-  double2 *Gs = Us + E;
-  double *coef_s = reinterpret_cast<double *>(Hs + E + (size_t)NG * plan.per_group);
-  int *ids = reinterpret_cast<int *>(coef_s + 32) + (size_t)g * plan.ints_per_group;
-  int *nts = ids + 2 * T;
-  double *deph_s = reinterpret_cast<double *>(ids + ((3 * T + 1) & ~1));  // 8-byte aligned
-  unsigned long long *nmax_s = reinterpret_cast<unsigned long long *>(deph_s + 1);
-  int *tlf_s = reinterpret_cast<int *>(nmax_s + 1);
+  double2 *Xs = reinterpret_cast<double2 *>(smem_raw + pl.x);
+  double2 *Us = reinterpret_cast<double2 *>(smem_raw + pl.u);
+  double2 *Ms = reinterpret_cast<double2 *>(smem_raw + pl.m);
+  double *Vs = reinterpret_cast<double *>(smem_raw + pl.v);
+  double2 *Ops = reinterpret_cast<double2 *>(smem_raw + pl.ops);
+  NodeCoef *cfs = reinterpret_cast<NodeCoef *>(smem_raw + pl.cf);
+  int2 *ids = reinterpret_cast<int2 *>(smem_raw + pl.ids);
+
+  const long long n0 = (long long)blockIdx.x * pl.nt;
+  const int nt = (int)(c.M - n0 < pl.nt ? c.M - n0 : pl.nt);
+  const int ncols = nt * N, tile = nt * E, step = pl.cs * N;
+  const bool nb = !c.vacuum;
+  pdl_launch_dependents();
+  if (c.filtered) pdl_wait();  // the records read the previous stage's flags
+  const uint8_t *act_in = nullptr;
+  if (c.filtered) act_in = p.act[p.mode == kModeRkf45 ? *(volatile int *)&p.ctl->ycur : p.act_par];
+  // Records: neighbour ids (-1 absent; an inactive neighbour contributes
+  // nothing, hierarchy_updater.cc:256-303) and coefficients.
+  if (nb) {
+    for (int q = tid; q < nt * T; q += nth) {
+      const int t = q % T;
+      int nx = __ldg(c.next + n0 * T + q), pv = __ldg(c.prev + n0 * T + q);
+      const int occ = __ldg(c.mi + n0 * T + q);
+      const double2 ct = __ldg(c.corr + t);
+      if (act_in) {
+        if (nx >= 0 && !__ldcg(act_in + nx)) nx = -1;
+        if (pv >= 0 && !__ldcg(act_in + pv)) pv = -1;
+      }
+      // DiagonalBath is unnormalised (hierarchy_updater.cc:105-127).
+      const double s = KIND == kDiagonal ? 1.0 : __ldg(c.sq_next + t * (c.L + 2) + occ);
+      const double sp = KIND == kDiagonal ? (double)occ : __ldg(c.sq_prev + t * (c.L + 2) + occ);
+      ids[q] = make_int2(nx, pv);
+      cfs[q] = NodeCoef{s, 0.0, sp * ct.x, sp * ct.y};
+    }
+  }
+  if (!c.filtered) pdl_wait();
 
   int ycur = 0;
   if (p.mode == kModeRkf45) {
     if (*(volatile int *)&p.ctl->done) return;  // uniform for the whole grid
-    ycur = p.ctl->ycur;
-    for (int i = threadIdx.x; i < 24; i += blockDim.x) coef_s[i] = p.ctl->coef[i];
+    ycur = *(volatile int *)&p.ctl->ycur;
   }
-  for (int i = threadIdx.x; i < E; i += blockDim.x) Hs[i] = c.H[i];
+  const double2 *xin = (p.mode == kModeRkf45 && p.stage == 0) ? p.ybuf[ycur] : p.x + blockIdx.y * p.x_bstride;
+  // This thread's elements: e0 + r * step, row i, first column c0.
+  const int i = tid % N, c0 = tid / N;
+  const bool live = c0 < pl.cs;
+  for (int e = tid; e < tile; e += nth) cp_async16(Xs + e, xin + n0 * E + e);
+  if (pl.stage_ops && live) {
+    for (int o = 0; o < p.nops; ++o) {
+      const double2 *src = (p.mode == kModeRkf45 && o == 0) ? p.ybuf[ycur] : p.op[o];
+      double2 *dst = Ops + (size_t)o * pl.nt * E;
+      for (int e = tid; e < tile; e += step) cp_async16(dst + e, src + n0 * E + e);
+    }
+  }
+  // An annealing run rewrites H (and V) between stages.
+  double *Hr = reinterpret_cast<double *>(Hs);
+  if (c.h_real) {
+    for (int e = tid; e < E; e += nth) Hr[e] = __ldcg(c.H + e).x;
+  } else {
+    for (int e = tid; e < E; e += nth) Hs[e] = __ldcg(c.H + e);
+  }
+  if (KIND == kFull && nb)
+    for (int e = tid; e < c.nb * E; e += nth) Vs[e] = __ldcg(c.bath_V + e);
+  __syncthreads();  // records
+
+  // The tile's X (and H) before the first read of them.
+  bool have_x = false;
+  auto need_x = [&]() {
+    if (have_x) return;
+    have_x = true;
+    cp_async_wait();
+    __syncthreads();
+  };
+  const double ih = c.inv_hbar;
+  const int rounds = (ncols + pl.cs - 1) / pl.cs;
+  const int K1 = c.K1;
+  // The linked ADOs' values at offset off for `count` term records, four
+  // terms' loads in flight at a time: use(n, X+, X-, record n's coefficients),
+  // absent ADOs as zeros.
+  auto gather = [&](int count, int off, auto record, bool with_next, auto use) {
+    for (int n0t = 0; n0t < count; n0t += 4) {
+      double2 g[4], h[4];
+      int q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool on = n0t + u < count;
+        q[u] = on ? record(n0t + u) : -1;
+        const int2 id = on ? ids[q[u]] : make_int2(-1, -1);
+        g[u] = with_next && id.x >= 0 ? ld_global(xin + (long long)id.x * E + off) : make_double2(0.0, 0.0);
+        h[u] = id.y >= 0 ? ld_global(xin + (long long)id.y * E + off) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q[u] >= 0) use(n0t + u, g[u], h[u], cfs[q[u]]);
+    }
+  };
+  // m += -i (s X+ + a X-)
+  auto add_term = [](double2 &m, double2 g, double2 h, const NodeCoef &f) {
+    m.x = fma(f.s, g.y, m.x);
+    m.y = fma(-f.s, g.x, m.y);
+    m.x = fma(f.ax, h.y, fma(f.ay, h.x, m.x));
+    m.y = fma(f.ay, h.y, fma(-f.ax, h.x, m.y));
+  };
+  // (Q X - X Q^+)_ij of the deepest tier's time-local matrix Q_b.
+  auto tl_deepest = [&](int nd) {
+    int tier = 0;
+    for (int t = 0; t < T; ++t) tier += __ldg(c.mi + (n0 + nd) * T + t);
+    return tier == c.L;
+  };
+  auto tl_commutator = [&](int b, const double2 *X, int j) {
+    const double2 *Q = c.tl_q + (size_t)b * E;
+    double2 w = make_double2(0.0, 0.0);
+    for (int k = 0; k < N; ++k) {
+      const double2 qi = __ldcg(Q + i + k * N), qj = __ldcg(Q + j + k * N), xk = X[k + j * N], xi = X[i + k * N];
+      w.x += qi.x * xk.x - qi.y * xk.y - (xi.x * qj.x + xi.y * qj.y);
+      w.y += qi.x * xk.y + qi.y * xk.x - (xi.y * qj.x - xi.x * qj.y);
+    }
+    return w;
+  };
+
+  // Full couplings: the neighbour terms of baths b0 .. b0 + bn - 1 into Ms.
+  auto full_terms = [&](int b0, int bn) {
+    for (int r = 0; r < rounds; ++r) {
+      const int col = c0 + r * pl.cs;
+      if (!live || col >= ncols) continue;
+      const int nd = col / N, off = i + (col - nd * N) * N;
+      double2 m = make_double2(0.0, 0.0);
+      int left = K1, b = 0;
+      gather(bn * K1, off, [&](int n) { return nd * T + b0 * K1 + n; }, true,
+             [&](int, double2 g, double2 h, const NodeCoef &f) {
+               add_term(m, g, h, f);
+               if (--left == 0) {
+                 Ms[b * pl.nt * E + col * N + i] = m;
+                 m = make_double2(0.0, 0.0);
+                 left = K1;
+                 ++b;
+               }
+             });
+    }
+  };
+  if (KIND == kFull && nb) full_terms(0, c.nb < pl.bc ? c.nb : pl.bc);
+
+  for (int r0 = 0; r0 < rounds; r0 += kNodeRounds) {
+    double2 acc[kNodeRounds];
+#pragma unroll
+    for (int r = 0; r < kNodeRounds; ++r) {
+      acc[r] = make_double2(0.0, 0.0);
+      const int col = c0 + (r0 + r) * pl.cs;
+      if (KIND == kFull || !nb || !live || col >= ncols) continue;
+      const int nd = col / N, j = col - nd * N, off = i + j * N;
+      if (KIND == kIndependent) {
+        // Column j of the ADOs linked by the baths on site j: + i s X+ and
+        // + i conj(c) sp X- (the next terms cancel on the diagonal).
+        const int q0 = __ldg(c.site_ptr + j), nq = __ldg(c.site_ptr + j + 1) - q0;
+        gather(nq, off, [&](int n) { return nd * T + __ldg(c.site_terms + q0 + n); }, i != j,
+               [&](int, double2 g, double2 h, const NodeCoef &f) {
+                 acc[r].x = fma(-f.s, g.y, acc[r].x);
+                 acc[r].y = fma(f.s, g.x, acc[r].y);
+                 acc[r].x = fma(f.ay, h.x, fma(-f.ax, h.y, acc[r].x));
+                 acc[r].y = fma(f.ax, h.x, fma(f.ay, h.y, acc[r].y));
+               });
+      } else {
+        gather(T, off, [&](int n) { return nd * T + n; }, true,
+               [&](int n, double2 g, double2 h, const NodeCoef &f) {
+                 double2 m = make_double2(0.0, 0.0);
+                 add_term(m, g, h, f);
+                 acc[r] = c_axpy(acc[r], m, __ldg(c.bath_V + (size_t)(n / K1) * N + i));
+               });
+      }
+    }
+    need_x();
+    // A = H X: one H_ik serves the round's elements (elements past the tile
+    // repeat its last column).
+    int xo[kNodeRounds];
+    double2 a[kNodeRounds];
+#pragma unroll
+    for (int r = 0; r < kNodeRounds; ++r) {
+      const int col = c0 + (r0 + r) * pl.cs;
+      xo[r] = (col < ncols ? col : ncols - 1) * N;
+      a[r] = make_double2(0.0, 0.0);
+    }
+    if (c.h_real) {
+#pragma unroll 4
+      for (int k = 0; k < N; ++k) {
+        const double h = Hr[i + k * N];
+#pragma unroll
+        for (int r = 0; r < kNodeRounds; ++r) {
+          const double2 x = Xs[xo[r] + k];
+          a[r].x = fma(h, x.x, a[r].x);
+          a[r].y = fma(h, x.y, a[r].y);
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < N; ++k) {
+        const double2 h = Hs[i + k * N];
+#pragma unroll
+        for (int r = 0; r < kNodeRounds; ++r) {
+          const double2 x = Xs[xo[r] + k];
+          a[r].x = fma(h.x, x.x, fma(-h.y, x.y, a[r].x));
+          a[r].y = fma(h.x, x.y, fma(h.y, x.x, a[r].y));
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kNodeRounds; ++r) {
+      const int col = c0 + (r0 + r) * pl.cs;
+      if (!live || col >= ncols) continue;
+      if (KIND == kDiagonal && c.time_local && nb) {
+        const int nd = col / N, j = col - nd * N;
+        if (tl_deepest(nd))
+          for (int b = 0; b < c.nb; ++b)
+            acc[r] = c_axpy(acc[r], tl_commutator(b, Xs + nd * E, j), -__ldg(c.bath_V + (size_t)b * N + i));
+      }
+      Us[col * NP + i] = make_double2(fma(a[r].y, ih, acc[r].x), fma(-a[r].x, ih, acc[r].y));
+    }
+  }
+  if (KIND == kFull && nb) {
+    // M_b of up to bc baths at a time, then B += V_b M_b.
+    for (int b0 = 0; b0 < c.nb; b0 += pl.bc) {
+      const int bn = c.nb - b0 < pl.bc ? c.nb - b0 : pl.bc;
+      if (b0 > 0) {
+        __syncthreads();  // the previous baths' M_b are read
+        full_terms(b0, bn);
+      }
+      for (int r = 0; r < rounds; ++r) {
+        const int col = c0 + r * pl.cs;
+        if (!live || col >= ncols) continue;
+        const int nd = col / N, j = col - nd * N;
+        const double2 *X = Xs + nd * E;
+        const bool tl = c.time_local && tl_deepest(nd);
+        for (int b = 0; b < bn; ++b) {
+          // + Delta_b [X, V_b]
+          const double *V = Vs + (size_t)(b0 + b) * E;
+          double2 w = make_double2(0.0, 0.0), z = w;
+#pragma unroll 4
+          for (int k = 0; k < N; ++k) {
+            w = c_axpy(w, X[i + k * N], V[k + j * N]);
+            z = c_axpy(z, X[k + j * N], V[i + k * N]);
+          }
+          double2 &m = Ms[b * pl.nt * E + col * N + i];
+          double2 v = c_axpy(m, make_double2(w.x - z.x, w.y - z.y), __ldg(c.mats_bath + b0 + b));
+          if (tl) v = c_axpy(v, tl_commutator(b0 + b, X, j), -1.0);
+          m = v;
+        }
+      }
+      __syncthreads();
+      for (int r = 0; r < rounds; ++r) {
+        const int col = c0 + r * pl.cs;
+        if (!live || col >= ncols) continue;
+        double2 u = Us[col * NP + i], w = make_double2(0.0, 0.0);
+        for (int b = 0; b < bn; ++b) {
+          const double *V = Vs + (size_t)(b0 + b) * E + i;
+          const double2 *M = Ms + b * pl.nt * E + col * N;
+          int k = 0;
+#pragma unroll 2
+          for (; k + 1 < N; k += 2) {
+            u = c_axpy(u, M[k], V[k * N]);
+            w = c_axpy(w, M[k + 1], V[(k + 1) * N]);
+          }
+          if (k < N) u = c_axpy(u, M[k], V[k * N]);
+        }
+        Us[col * NP + i] = make_double2(u.x + w.x, u.y + w.y);
+      }
+    }
+  }
   __syncthreads();
 
-  const double ih = c.inv_hbar;
+  // dX of each element and its combine.
+  const double *coef = p.mode == kModeRkf45 ? p.ctl->coef : nullptr;
+  auto cf = [&](int q) { return __ldcg(coef + q); };
+  auto operand = [&](int o, int e) -> double2 {
+    if (pl.stage_ops) return Ops[(size_t)o * pl.nt * E + e];
+    const double2 *src = (p.mode == kModeRkf45 && o == 0) ? p.ybuf[ycur] : p.op[o];
+    return ld_global(src + n0 * E + e);
+  };
+  const bool flags = c.filtered && ((p.mode == kModeRk4 && p.stage == 3) || (p.mode == kModeRkf45 && p.stage == 5));
+  long long row = -1;  // rho_0 row this step writes
+  if (p.mode == kModeRk4 && p.stage == 3 && n0 == 0 && p.traj) {
+    const volatile Rk4Ctl *rc = p.rk4;
+    if (rc->out_factor > 0 && rc->step % rc->out_factor == 0 && rc->nout < rc->capacity) row = rc->nout;
+  }
   double emax = 0.0;
-  // RKF45 stage 0 reads the current state, whose buffer only the device knows.
-  if (gridDim.y > 1) {
-    p.x += blockIdx.y * p.x_bstride;
-    p.out += blockIdx.y * p.out_bstride;
-  }
-  const double2 *xin = (p.mode == kModeRkf45 && p.stage == 0) ? p.ybuf[ycur] : p.x;
-  const double2 *yin = p.mode == kModeRkf45 ? p.ybuf[ycur] : p.y;
-  // Filtering: flags of the current state, and of the state this launch
-  // writes (RK4 stage 3, RKF45 stage 5 -- the candidate, kept on accept).
-  const uint8_t *act_in = nullptr;
-  uint8_t *act_out = nullptr;
-  if (c.filtered) {
-    const int ap = p.mode == kModeRkf45 ? ycur : p.act_par;
-    act_in = p.act[ap];
-    act_out = p.act[ap ^ 1];
-  }
-  const bool flag_stage = act_in && act_out &&
-                          ((p.mode == kModeRk4 && p.stage == 3) || (p.mode == kModeRkf45 && p.stage == 5));
-
-  for (long long n = (long long)blockIdx.x * NG + g; n < c.M; n += (long long)gridDim.x * NG) {
-    // 1. metadata
-    for (int s = lane; s < 2 * T; s += GROUP) {
-      const int id = s < T ? __ldg(c.next + n * T + s) : __ldg(c.prev + n * T + (s - T));
-      // an inactive neighbour contributes nothing (hierarchy_updater.cc:256-303)
-      ids[s] = (id >= 0 && act_in && !__ldg(act_in + id)) ? -1 : id;
+  for (int r = 0; r < rounds; ++r) {
+    const int col = c0 + r * pl.cs;
+    if (!live || col >= ncols) continue;
+    const int nd = col / N, j = col - nd * N, e = tid + r * step;
+    const long long g = n0 * E + e;
+    const double2 *X = Xs + nd * E;
+    const double2 b = Us[col * NP + i], bt = Us[(nd * N + i) * NP + j];
+    double2 kv = make_double2(b.x + bt.x, i == j ? 0.0 : b.y - bt.y);
+    if (nb) {
+      // The upper triangle's X (a lower element is its conjugate).
+      const double2 x = X[i <= j ? i + j * N : j + i * N];
+      const double fac = __ldg(c.deph_node + n0 + nd) + __ldg(c.mats_elem + i + j * N);
+      kv.x = fma(-fac, x.x, kv.x);
+      kv.y = fma(i == j ? 0.0 : (i < j ? -fac : fac), x.y, kv.y);
     }
-    for (int t = lane; t < T; t += GROUP) nts[t] = __ldg(c.mi + n * T + t);
-    // 2. own ADO
-    const double2 *xn = xin + n * E;
-    for (int e = lane; e < E; e += GROUP) Xs[e] = __ldg(xn + e);
-    group_sync<GROUP>(g);
-    if (lane == 0) {
-      double d = 0.0;
-      for (int t = 0; t < T; ++t) d += nts[t] * __ldg(c.nu + t);
-      deph_s[0] = d;
-      nmax_s[0] = 0ull;
-      int tier = 0;
-      for (int t = 0; t < T; ++t) tier += nts[t];
-      tlf_s[0] = c.time_local && tier == c.L;
+    if (KIND == kIndependent && c.time_local && i != j && tl_deepest(nd)) {
+      const double2 tv = tl_pair_term<double2>(X, c.tl_q, N, i < j ? i : j, i < j ? j : i);
+      kv.x += tv.x;
+      kv.y += i < j ? tv.y : -tv.y;
     }
-    if (KIND == kIndependent && !c.vacuum) {
-      for (int idx = lane; idx < 2 * T * N; idx += GROUP) {
-        const int s = idx / N, k = idx - s * N;
-        const int id = ids[s];
-        if (id >= 0) {
-          const int t = s < T ? s : s - T;
-          const int m = __ldg(c.term_site + t);
-          Gs[idx] = __ldg(xin + (long long)id * E + k + m * N);
-        }
-      }
-    }
-    // 3. A = H X
-    for (int e = lane; e < E; e += GROUP) {
-      const int i = e % N, j = e / N;
-      double2 a = make_double2(0.0, 0.0);
-      for (int k = 0; k < N; ++k) {
-        const double2 h = Hs[i + k * N], x = Xs[k + j * N];
-        a.x = fma(h.x, x.x, a.x);
-        a.x = fma(-h.y, x.y, a.x);
-        a.y = fma(h.x, x.y, a.y);
-        a.y = fma(h.y, x.x, a.y);
-      }
-      As[e] = a;
-    }
-    if (KIND != kIndependent) {
-      // Neighbour (and, for FullBath, Matsubara) terms into Gs[0..E) per element.
-      double2 *NB = Gs;
-      double2 *W = Gs + E;  // work matrix
-      for (int e = lane; e < E; e += GROUP) NB[e] = make_double2(0.0, 0.0);
-      group_sync<GROUP>(g);
-      if (!c.vacuum) {
-        if (KIND == kFull) {
-          // -Delta_b [V_b, [V_b, X]]  (FullBath::DoMatsubara, hierarchy_updater.cc:10-25)
-          for (int b = 0; b < c.nb; ++b) {
-            const double *V = c.bath_V + (size_t)b * E;
-            for (int e = lane; e < E; e += GROUP) {
-              const int i = e % N, j = e / N;
-              double2 w = make_double2(0.0, 0.0);
-              for (int k = 0; k < N; ++k) {
-                w = c_axpy(w, Xs[k + j * N], __ldg(V + i + k * N));
-                w = c_axpy(w, Xs[i + k * N], -__ldg(V + k + j * N));
-              }
-              W[e] = w;
-            }
-            group_sync<GROUP>(g);
-            const double dlt = __ldg(c.mats_bath + b);
-            for (int e = lane; e < E; e += GROUP) {
-              const int i = e % N, j = e / N;
-              double2 w = make_double2(0.0, 0.0);
-              for (int k = 0; k < N; ++k) {
-                w = c_axpy(w, W[k + j * N], __ldg(V + i + k * N));
-                w = c_axpy(w, W[i + k * N], -__ldg(V + k + j * N));
-              }
-              NB[e] = c_axpy(NB[e], w, -dlt);
-            }
-            group_sync<GROUP>(g);
-          }
-        }
-        for (int s = 0; s < 2 * T; ++s) {
-          const int id = ids[s];
-          if (id < 0) continue;
-          const bool is_next = s < T;
-          const int t = is_next ? s : s - T;
-          const int b = __ldg(c.term_site + t);
-          const int nt = nts[t];
-          const double2 *xo = xin + (long long)id * E;
-          if (KIND == kDiagonal) {
-            // DiagonalBath::DoNext / DoPrevious (hierarchy_updater.cc:105-127):
-            // next: -i (V_i - V_j) X+_ij ; prev: n_t (-i)(c V_i - c^* V_j) X-_ij
-            const double *V = c.bath_V + (size_t)b * N;
-            const double2 ct = __ldg(c.corr + t);
-            for (int e = lane; e < E; e += GROUP) {
-              const int i = e % N, j = e / N;
-              const double2 xv = __ldg(xo + e);
-              const double vi = __ldg(V + i), vj = __ldg(V + j);
-              double2 f;
-              if (is_next) {
-                f = make_double2(0.0, -(vi - vj));
-              } else {
-                // -i (c vi - conj(c) vj) * n_t
-                const double re = ct.x * vi - ct.x * vj;
-                const double im = ct.y * vi + ct.y * vj;
-                f = make_double2(im * nt, -re * nt);
-              }
-              NB[e] = c_add(NB[e], c_mul(f, xv));
-            }
-          } else {
-            // FullBath::DoNext: -p V X+ + p X+ V, p = i s;
-            // FullBath::DoPrevious: -pr V X- - pc X- V (hierarchy_updater.cc:46-82)
-            const double *V = c.bath_V + (size_t)b * E;
-            for (int e = lane; e < E; e += GROUP) W[e] = __ldg(xo + e);
-            group_sync<GROUP>(g);
-            double2 pl, pr;
-            if (is_next) {
-              const double sn = __ldg(c.sq_next + t * (c.L + 2) + nt);
-              pl = make_double2(0.0, -sn);  // -p
-              pr = make_double2(0.0, sn);   // +p
-            } else {
-              const double sp = __ldg(c.sq_prev + t * (c.L + 2) + nt);
-              const double2 ct = __ldg(c.corr + t);
-              pl = make_double2(ct.y * sp, -ct.x * sp);   // -pr = -i c sp
-              pr = make_double2(ct.y * sp, ct.x * sp);    // -pc = i conj(c) sp
-            }
-            for (int e = lane; e < E; e += GROUP) {
-              const int i = e % N, j = e / N;
-              double2 vx = make_double2(0.0, 0.0), xv = make_double2(0.0, 0.0);
-              for (int k = 0; k < N; ++k) {
-                vx = c_axpy(vx, W[k + j * N], __ldg(V + i + k * N));
-                xv = c_axpy(xv, W[i + k * N], __ldg(V + k + j * N));
-              }
-              NB[e] = c_add(NB[e], c_add(c_mul(pl, vx), c_mul(pr, xv)));
-            }
-            group_sync<GROUP>(g);
-          }
-        }
-        if (tlf_s[0]) {
-          // Time-local truncation on the deepest tier, DiagonalBath /
-          // FullBath::DoTimelocal (hierarchy_updater.cc:28-44, :93-104):
-          // W = Q_b X - X Q_b^+, then -[V_b, W] for every bath b.
-          for (int b = 0; b < c.nb; ++b) {
-            const double2 *Q = c.tl_q + (size_t)b * E;
-            group_sync<GROUP>(g);  // W is reused
-            for (int e = lane; e < E; e += GROUP) {
-              const int i = e % N, j = e / N;
-              double2 w = make_double2(0.0, 0.0);
-              for (int k = 0; k < N; ++k) {
-                w = c_add(w, c_mul(__ldg(Q + i + k * N), Xs[k + j * N]));
-                w = c_sub(w, c_mul(Xs[i + k * N], c_conj(__ldg(Q + j + k * N))));
-              }
-              W[e] = w;
-            }
-            group_sync<GROUP>(g);
-            if (KIND == kDiagonal) {
-              const double *V = c.bath_V + (size_t)b * N;
-              for (int e = lane; e < E; e += GROUP) {
-                const int i = e % N, j = e / N;
-                NB[e] = c_axpy(NB[e], W[e], -(__ldg(V + i) - __ldg(V + j)));
-              }
-            } else {
-              const double *V = c.bath_V + (size_t)b * E;
-              for (int e = lane; e < E; e += GROUP) {
-                const int i = e % N, j = e / N;
-                double2 vw = make_double2(0.0, 0.0);
-                for (int k = 0; k < N; ++k) {
-                  vw = c_axpy(vw, W[k + j * N], __ldg(V + i + k * N));
-                  vw = c_axpy(vw, W[i + k * N], -__ldg(V + k + j * N));
-                }
-                NB[e] = c_sub(NB[e], vw);
-              }
-            }
-          }
-        }
-      }
-    }
-    group_sync<GROUP>(g);
-
-    // 4. upper-triangle pairs
-    const double deph = deph_s[0];
-    const bool tl_node = tlf_s[0] != 0;
-    const int npairs = N * (N + 1) / 2;
-    for (int u = lane; u < npairs; u += GROUP) {
-      const int i = __ldg(c.pair_i + u), j = __ldg(c.pair_j + u);
-      const double2 aij = As[i + j * N], aji = As[j + i * N];
-      double2 v = make_double2((aij.y + aji.y) * ih, -(aij.x - aji.x) * ih);
-      const double2 xij = Xs[i + j * N];
-      if (!c.vacuum) {
-        const double fac = deph + __ldg(c.mats_elem + i + j * N);
-        v = c_axpy(v, xij, -fac);
-        if (KIND == kIndependent && tl_node && i != j) v = c_add(v, tl_pair_term<double2>(Xs, c.tl_q, N, i, j));
-        if (KIND == kIndependent) {
-          if (i != j) {
-            for (int q = __ldg(c.site_ptr + j); q < __ldg(c.site_ptr + j + 1); ++q) {
-              const int t = __ldg(c.site_terms + q);
-              const int nt = nts[t];
-              if (ids[t] >= 0) {  // + p X+_ij, p = i sqrt((n+1)|c|)
-                v = c_add_i(v, Gs[t * N + i], __ldg(c.sq_next + t * (c.L + 2) + nt));
-              }
-              if (ids[T + t] >= 0) {  // - pc X-_ij = i conj(c) sp X-_ij
-                const double sp = __ldg(c.sq_prev + t * (c.L + 2) + nt);
-                const double2 ct = __ldg(c.corr + t);
-                v = c_add_i(v, c_mul(c_conj(ct), Gs[(T + t) * N + i]), sp);
-              }
-            }
-            for (int q = __ldg(c.site_ptr + i); q < __ldg(c.site_ptr + i + 1); ++q) {
-              const int t = __ldg(c.site_terms + q);
-              const int nt = nts[t];
-              if (ids[t] >= 0) {  // - p X+_ij, X+_ij = conj(X+_ji)
-                v = c_add_i(v, c_conj(Gs[t * N + j]), -__ldg(c.sq_next + t * (c.L + 2) + nt));
-              }
-              if (ids[T + t] >= 0) {  // - pr X-_ij = -i c sp X-_ij
-                const double sp = __ldg(c.sq_prev + t * (c.L + 2) + nt);
-                const double2 ct = __ldg(c.corr + t);
-                v = c_add_i(v, c_mul(ct, c_conj(Gs[(T + t) * N + j])), -sp);
-              }
-            }
-          } else {
-            // diagonal (m, m): next terms cancel; prev gives -(pc + pr) X-_mm
-            //   = 2 sp Im(c) X-_mm
-            for (int q = __ldg(c.site_ptr + i); q < __ldg(c.site_ptr + i + 1); ++q) {
-              const int t = __ldg(c.site_terms + q);
-              if (ids[T + t] >= 0) {
-                const double sp = __ldg(c.sq_prev + t * (c.L + 2) + nts[t]);
-                const double2 ct = __ldg(c.corr + t);
-                v.x = fma(2.0 * sp * ct.y, Gs[(T + t) * N + i].x, v.x);
-              }
-            }
-          }
-        } else {
-          v = c_add(v, Gs[i + j * N]);
-        }
-      }
-      if (i == j) {
-        v.y = 0.0;
-        Us[i + j * N] = v;
-      } else {
-        Us[i + j * N] = v;
-        Us[j + i * N] = c_conj(v);
-      }
-    }
-    group_sync<GROUP>(g);
-
-    // 5. epilogue
-    const long long base = n * E;
-    double fl_m = 0.0;  // filtering: max |y_new|^2 of this lane's elements
+    double2 yn = kv;  // the new state, in the stages that write it
     if (p.mode == kModeApply) {
-      for (int e = lane; e < E; e += GROUP) p.out[base + e] = Us[e];
+      p.out[blockIdx.y * p.out_bstride + g] = kv;
     } else if (p.mode == kModeRk4) {
       const int s = p.stage;
-      for (int e = lane; e < E; e += GROUP) {
-        const double2 kv = Us[e];
-        if (s == 0) {
-          const double2 ys = Xs[e];
-          p.out[base + e] = c_axpy(ys, kv, p.a_next);
-          p.acc[base + e] = c_axpy(ys, kv, p.w_acc);
-        } else if (s < 3) {
-          const double2 ys = __ldg(p.y + base + e);
-          p.out[base + e] = c_axpy(ys, kv, p.a_next);
-          p.acc[base + e] = c_axpy(p.acc[base + e], kv, p.w_acc);
-        } else {
-          const double2 yn = c_axpy(p.acc[base + e], kv, p.w_acc);
-          p.y[base + e] = yn;
-          const double m2 = fma(yn.x, yn.x, yn.y * yn.y);
-          fl_m = m2 > fl_m ? m2 : fl_m;
-          if (n == 0 && p.traj) Xs[e] = yn;
-        }
+      if (s < 3) {
+        const double2 ys = s == 0 ? X[i + j * N] : operand(0, e);
+        p.out[g] = c_axpy(ys, kv, p.a_next);
+        p.acc[g] = c_axpy(s == 0 ? ys : operand(1, e), kv, p.w_acc);
+      } else {
+        yn = c_axpy(operand(0, e), kv, p.w_acc);
+        p.y[g] = yn;
+        if (row >= 0 && e < E) p.traj[row * E + e] = yn;
       }
-      if (n == 0 && p.stage == 3 && p.traj) {
-        group_sync<GROUP>(g);
-        Rk4Ctl *rc = p.rk4;
-        const long long step = rc->step;
-        if (rc->out_factor > 0 && step % rc->out_factor == 0) {
-          const long long row = rc->nout;
-          if (row < rc->capacity)
-            for (int e = lane; e < E; e += GROUP) p.traj[row * E + e] = Xs[e];
-        }
-        group_sync<GROUP>(g);
-        if (lane == 0) {
-          if (rc->out_factor > 0 && step % rc->out_factor == 0) rc->nout = rc->nout + 1;
-          rc->step = step + 1;
-        }
-      }
-    } else {  // RKF45
-      const int s = p.stage;
-      const double *cf = coef_s;
-      for (int e = lane; e < E; e += GROUP) {
-        const double2 kv = Us[e];
-        const double2 ys = s == 0 ? Xs[e] : __ldg(yin + base + e);
-        if (s < 5) {
-          if (s < 5) p.k[s][base + e] = kv;
-          // X_{s+1} = y + sum_{r<=s} b_{s+1,r} k_r  (left to right, as :2015-2200)
-          const int row = s * (s + 1) / 2;
-          double2 xv = ys;
-          for (int r = 0; r < s; ++r) xv = c_axpy(xv, __ldg(p.k[r] + base + e), cf[row + r]);
-          xv = c_axpy(xv, kv, cf[row + s]);
-          p.out[base + e] = xv;
-        } else {
-          const double2 k0 = __ldg(p.k[0] + base + e), k2 = __ldg(p.k[2] + base + e);
-          const double2 k3 = __ldg(p.k[3] + base + e), k4 = __ldg(p.k[4] + base + e);
-          double2 y4 = c_axpy(ys, k0, cf[15]);
-          y4 = c_axpy(y4, k2, cf[16]);
-          y4 = c_axpy(y4, k3, cf[17]);
-          y4 = c_axpy(y4, k4, cf[18]);
-          double2 y5 = c_axpy(ys, k0, cf[19]);
-          y5 = c_axpy(y5, k2, cf[20]);
-          y5 = c_axpy(y5, k3, cf[21]);
-          y5 = c_axpy(y5, k4, cf[22]);
-          y5 = c_axpy(y5, kv, cf[23]);
-          p.ybuf[ycur ^ 1][base + e] = y5;
-          const double m2 = fma(y5.x, y5.x, y5.y * y5.y);
-          fl_m = m2 > fl_m ? m2 : fl_m;
-          const double err = hypot(y4.x - y5.x, y4.y - y5.y);
-          emax = (err > emax || err != err) ? err : emax;
-        }
-      }
+    } else if (p.stage < 5) {
+      // X_{s+1} = y + sum_{r<=s} b_{s+1,r} k_r  (left to right, :2015-2200)
+      const int s = p.stage, co = s * (s + 1) / 2;
+      p.k[s][g] = kv;
+      double2 xv = s == 0 ? X[i + j * N] : operand(0, e);
+      for (int q = 0; q < s; ++q) xv = c_axpy(xv, operand(1 + q, e), cf(co + q));
+      p.out[g] = c_axpy(xv, kv, cf(co + s));
+    } else {
+      const double2 ys = operand(0, e), k0 = operand(1, e), k2 = operand(2, e), k3 = operand(3, e),
+                    k4 = operand(4, e);
+      double2 y4 = c_axpy(ys, k0, cf(15));
+      y4 = c_axpy(y4, k2, cf(16));
+      y4 = c_axpy(y4, k3, cf(17));
+      y4 = c_axpy(y4, k4, cf(18));
+      yn = c_axpy(ys, k0, cf(19));
+      yn = c_axpy(yn, k2, cf(20));
+      yn = c_axpy(yn, k3, cf(21));
+      yn = c_axpy(yn, k4, cf(22));
+      yn = c_axpy(yn, kv, cf(23));
+      p.ybuf[ycur ^ 1][g] = yn;
+      const double err = hypot(y4.x - yn.x, y4.y - yn.y);
+      emax = (err > emax || err != err) ? err : emax;
     }
-    if (flag_stage) {
-      // New flags of the state just written (hierarchy_integrator.cc:2827-2850,
-      // :2359-2384): below the tolerance -> inactive, above -> active, equal
-      // -> unchanged.  A NaN never wins the `>` above, as in PHI's scan.
-      if (fl_m > 0.0) atomicMax(nmax_s, (unsigned long long)__double_as_longlong(fl_m));
-      group_sync<GROUP>(g);
-      if (lane == 0) {
-        const double mx = sqrt(__longlong_as_double((long long)nmax_s[0]));
-        const uint8_t old = act_in[n];
-        act_out[n] = mx < c.filter_tol ? (uint8_t)0 : (mx > c.filter_tol ? (uint8_t)1 : old);
-      }
-    }
-    group_sync<GROUP>(g);
+    // X's own slot is free: no other thread reads it after the exchange
+    // barrier except as the upper triangle above, so the norms wait below.
+    if (flags) Ops[e] = make_double2(fma(yn.x, yn.x, yn.y * yn.y), 0.0);
   }
-
+  if (p.mode == kModeRk4 && p.stage == 3 && n0 == 0 && p.traj) {
+    __syncthreads();
+    if (tid == 0) {
+      Rk4Ctl *rc = p.rk4;
+      if (row >= 0) rc->nout = rc->nout + 1;
+      rc->step = rc->step + 1;
+    }
+  }
+  if (flags) {
+    // New flags of the state just written (hierarchy_integrator.cc:2827-2850,
+    // :2359-2384): below the tolerance -> inactive, above -> active, equal
+    // -> unchanged.  A NaN never wins the `>`, as in PHI's scan.
+    __syncthreads();
+    const int ap = p.mode == kModeRkf45 ? ycur : p.act_par;
+    for (int nd = tid >> 5; nd < nt; nd += nth >> 5) {
+      double m = 0.0;
+      for (int w = tid & 31; w < E; w += 32) {
+        const double v = Ops[nd * E + w].x;
+        m = v > m ? v : m;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v > m ? v : m;
+      }
+      if ((tid & 31) == 0) {
+        const double mx = sqrt(m);
+        p.act[ap ^ 1][n0 + nd] =
+            mx < c.filter_tol ? (uint8_t)0 : (mx > c.filter_tol ? (uint8_t)1 : __ldcg(p.act[ap] + n0 + nd));
+      }
+    }
+  }
   if (p.mode == kModeRkf45 && p.stage == 5) {
     // max-reduce |y4 - y5| (hierarchy_integrator.cc:2317-2351); the bit
     // pattern of a non-negative double orders like the value (NaN above inf).
+    // One atomic per CTA.
     unsigned long long bits = (unsigned long long)__double_as_longlong(emax);
     for (int off = 16; off > 0; off >>= 1) {
       const unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
       bits = o > bits ? o : bits;
     }
-    // one atomic per CTA (every CTA updates the same error word)
-    __shared__ unsigned long long wmax[8];
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = bits;
+    __shared__ unsigned long long wmax[kNodeThreads / 32];
+    if ((tid & 31) == 0) wmax[tid >> 5] = bits;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       unsigned long long m = wmax[0];
-      for (int w = 1; w < 8; ++w) m = wmax[w] > m ? wmax[w] : m;
+      for (int w = 1; w < nth / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
       if (m) atomicMax(&p.ctl->err_bits, m);
     }
   }
@@ -564,45 +576,101 @@ __global__ void rkf45_control_kernel(Rkf45Ctl *ctl) {
   }
 }
 
-template <int GROUP, int KIND>
-cudaError_t launch_group(const StageParams &p, size_t smem, int grid, int batch, cudaStream_t stream) {
-  auto kern = heom_stage_kernel<GROUP, KIND>;
+constexpr uint32_t kNodeMaxSmem = 224 * 1024;
+
+uint32_t align16(uint32_t b) { return (b + 15u) & ~15u; }
+
+// Shared-memory plan of nt nodes per tile with the combine's nops operands
+// staged (or not) and bc baths' M_b at once.
+void node_layout(const HeomConsts &c, int nops, bool flags, NodePlan *pl) {
+  const uint32_t E = c.N * c.N, tile = (uint32_t)pl->nt * E * 16;
+  uint32_t b = E * 16;  // H
+  pl->x = b;
+  b += tile;
+  pl->u = b;
+  b += (uint32_t)pl->nt * c.N * (c.N | 1) * 16;
+  pl->m = b;
+  if (c.kind == kFull && !c.vacuum) b += (uint32_t)pl->bc * tile;
+  pl->v = b;
+  if (c.kind == kFull && !c.vacuum) b += align16((uint32_t)c.nb * E * 8);
+  pl->ops = b;
+  b += std::max<uint32_t>(pl->stage_ops ? nops : 0, flags ? 1 : 0) * tile;
+  pl->cf = b;
+  b += (uint32_t)pl->nt * c.T * sizeof(NodeCoef);
+  pl->ids = b;
+  b += align16((uint32_t)pl->nt * c.T * sizeof(int2));
+  pl->bytes = b;
+}
+
+// Tile and CTA size: the cheapest of whole rounds of elements per thread (1 to
+// 4) and CTA sizes under
+//   waves * (2 + rounds) + CTAs per SM * (threads * rounds / 512 + 1/2):
+// a CTA's chain of latencies (a round takes about as long as half the fixed
+// part), the SM's element slots, and a CTA's fixed work.  Fitted to a sweep of
+// 17 problems on B200 (N = 3 .. 20, 84 to 20,000 nodes): within 10 % of the
+// best shape of the sweep, where a fixed 256-thread tile was up to 1.6 times
+// slower.
+NodePlan node_plan(const HeomConsts &c, int nops, bool flags, int num_sms) {
+  const int N = c.N;
+  NodePlan best{};
+  double best_cost = 1e300;
+  for (int threads = 64; threads <= kNodeThreads; threads += 32) {
+    const int cs = threads / N;
+    if (cs < 1) continue;
+    for (int want = 1; want <= 4; ++want) {
+      NodePlan pl{};
+      pl.nt = std::max(1, std::min<int>(want * cs / N, 64));
+      const int rounds = (pl.nt * N + cs - 1) / cs;
+      if (rounds < want && want > 1) continue;
+      pl.threads = threads;
+      pl.cs = cs;
+      pl.bc = std::min(c.nb, 8);
+      pl.stage_ops = nops > 0;
+      node_layout(c, nops, flags, &pl);
+      // Larger nodes: first read the operands directly, then take fewer
+      // baths at once.
+      if (pl.bytes > kNodeMaxSmem / 2 && pl.stage_ops) {
+        pl.stage_ops = 0;
+        node_layout(c, nops, flags, &pl);
+      }
+      while (pl.bytes > kNodeMaxSmem && pl.bc > 1 && c.kind == kFull) {
+        --pl.bc;
+        node_layout(c, nops, flags, &pl);
+      }
+      if (pl.bytes > kNodeMaxSmem && pl.nt > 1) continue;
+      const int resident = std::max(1, std::min<int>(768 / threads, (int)(kNodeMaxSmem / pl.bytes)));
+      const double tiles = (double)((c.M + pl.nt - 1) / pl.nt);
+      const double per_sm = std::ceil(tiles / num_sms);
+      const double cost = std::ceil(per_sm / resident) * (2.0 + rounds) + per_sm * (threads * rounds / 512.0 + 0.5);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = pl;
+      }
+    }
+  }
+  return best;
+}
+
+template <int KIND>
+cudaError_t launch_node(const StageParams &p, int batch, cudaStream_t stream) {
+  auto kern = heom_node_kernel<KIND>;
   static thread_local int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(kern, smem, configured);
+  cudaError_t e = raise_smem_limit(kern, p.plan.bytes, configured);
   if (e != cudaSuccess) return e;
-  kern<<<dim3(grid, batch), 256, smem, stream>>>(p);
-  return cudaGetLastError();
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch);
+  cfg.blockDim = dim3(p.plan.threads);
+  cfg.dynamicSmemBytes = p.plan.bytes;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 }  // namespace
-
-int choose_group(int N) {
-  if (N <= 11) return 32;
-  if (N <= 22) return 128;
-  return 256;
-}
-
-size_t stage_smem_bytes(int N, int T, int kind) {
-  const SmemPlan plan = smem_plan(N, T, kind);
-  const int NG = 256 / choose_group(N);
-  size_t bytes = (size_t)(plan.E + (size_t)NG * plan.per_group) * sizeof(double2);
-  bytes += 32 * sizeof(double);
-  bytes += (size_t)NG * plan.ints_per_group * sizeof(int);
-  return bytes + 16;
-}
-
-int stage_grid(const HeomConsts &c, int num_sms) {
-  const int NG = 256 / choose_group(c.N);
-  long long need = (c.M + NG - 1) / NG;
-  const size_t smem = stage_smem_bytes(c.N, c.T, c.kind);
-  int per_sm = (int)((200 * 1024) / (smem + 1024));
-  if (per_sm < 1) per_sm = 1;
-  if (per_sm > 8) per_sm = 8;
-  long long cap = (long long)num_sms * per_sm;
-  if (need > cap) need = cap;
-  if (need < 1) need = 1;
-  return (int)need;
-}
 
 cudaError_t launch_stage(const StageLaunch &L, cudaStream_t stream) {
   if (!L.generic && tile_kernel_available(L.c)) {
@@ -637,23 +705,32 @@ cudaError_t launch_stage(const StageLaunch &L, cudaStream_t stream) {
   p.out_bstride = L.out_bstride;
   const int batch = L.batch;
   if (batch < 1 || batch > 65535 || (batch > 1 && L.mode != kModeApply)) return cudaErrorInvalidValue;
-  const size_t smem = stage_smem_bytes(L.c.N, L.c.T, L.c.kind);
-  const int grid = L.grid;
-  const int group = choose_group(L.c.N);
-#define PHI_DISPATCH(G)                                                      \
-  switch (L.c.kind) {                                                        \
-    case kIndependent: return launch_group<G, kIndependent>(p, smem, grid, batch, stream); \
-    case kDiagonal: return launch_group<G, kDiagonal>(p, smem, grid, batch, stream); \
-    default: return launch_group<G, kFull>(p, smem, grid, batch, stream); \
+  // The combine's operands (see the kernel's epilogue).
+  p.nops = 0;
+  if (L.mode == kModeRk4) {
+    if (L.stage == 1 || L.stage == 2) {
+      p.op[p.nops++] = L.y;
+      p.op[p.nops++] = L.acc;
+    } else if (L.stage == 3) {
+      p.op[p.nops++] = L.acc;
+    }
+  } else if (L.mode == kModeRkf45 && L.stage > 0) {
+    p.op[p.nops++] = nullptr;  // the current state
+    if (L.stage < 5)
+      for (int r = 0; r < L.stage; ++r) p.op[p.nops++] = L.k[r];
+    else
+      for (int r : {0, 2, 3, 4}) p.op[p.nops++] = L.k[r];
   }
-  if (group == 32) {
-    PHI_DISPATCH(32)
-  } else if (group == 128) {
-    PHI_DISPATCH(128)
-  } else {
-    PHI_DISPATCH(256)
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return cudaErrorInvalidDevice;
+  const bool flags = L.c.filtered && L.mode != kModeApply;
+  p.plan = node_plan(L.c, p.nops, flags, sms);
+  switch (L.c.kind) {
+    case kIndependent: return launch_node<kIndependent>(p, batch, stream);
+    case kDiagonal: return launch_node<kDiagonal>(p, batch, stream);
+    default: return launch_node<kFull>(p, batch, stream);
   }
-#undef PHI_DISPATCH
 }
 
 namespace {

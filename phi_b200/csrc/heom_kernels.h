@@ -14,7 +14,6 @@ struct StageLaunch {
   HeomConsts c;
   int mode = kModeApply;
   int stage = 0;
-  int grid = 1;
   const double2 *x = nullptr;   // stage input
   double2 *out = nullptr;       // apply output / next stage input
   double2 *y = nullptr;         // RK4 state
@@ -54,9 +53,6 @@ struct StageLaunch {
   void *y32buf[2] = {nullptr, nullptr};
 };
 
-int choose_group(int N);
-size_t stage_smem_bytes(int N, int T, int kind);
-int stage_grid(const HeomConsts &c, int num_sms);
 cudaError_t launch_stage(const StageLaunch &L, cudaStream_t stream);
 cudaError_t launch_rkf45_control(Rkf45Ctl *ctl, cudaStream_t stream);
 // complex128 (node stride N*N) <-> complex64 (node stride `padded`).

@@ -84,7 +84,6 @@ namespace {
 phi::StageLaunch stage_launch(phi_ctx *c, int st, double dt) {
   phi::StageLaunch L;
   L.c = c->c;
-  L.grid = c->grid;
   L.mixed = c->mixed();
   L.y = c->y.as<double2>();
   L.acc = c->acc.as<double2>();

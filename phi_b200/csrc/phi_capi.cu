@@ -316,7 +316,6 @@ int tune_tile_schedule(phi_ctx *ctx) {
   phi::StageLaunch L;
   L.c = ctx->c;
   L.mode = phi::kModeApply;
-  L.grid = ctx->grid;
   L.mixed = ctx->mixed();
   if (L.mixed) {  // complex64 input from the state, output to the other stage buffer
     PHI_CUDA(ctx, phi::launch_to_c64(ctx->y.as<double2>(), ctx->xa.as<float2>(), ctx->hier.M, N * N,
@@ -565,7 +564,6 @@ extern "C" int phi_gpu_create(const phi_problem_desc *desc, phi_ctx **out) {
     return fail(nullptr, PHI_E_INVALID,
                 "mixed precision is built for independent baths on PHI's identity site map, K+1 <= 3 and "
                 "N in {2..8, 10, 12, 16, 24}");
-  ctx->grid = phi::stage_grid(ctx->c, ctx->num_sms);
   const size_t state_bytes = (size_t)ctx->hier.M * N * N * sizeof(double2);
   e = ctx->y.alloc(state_bytes);
   if (e != cudaSuccess) return fail(nullptr, PHI_E_OOM, "state allocation failed: " + std::to_string(state_bytes) + " bytes");
@@ -924,7 +922,6 @@ extern "C" int phi_gpu_apply_device(phi_ctx *ctx, const void *d_in, void *d_out,
   phi::StageLaunch L;
   L.c = ctx->c;
   L.mode = phi::kModeApply;
-  L.grid = ctx->grid;
   L.x = static_cast<const double2 *>(d_in);
   L.out = static_cast<double2 *>(d_out);
   L.xv = d_in;

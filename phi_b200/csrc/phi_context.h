@@ -32,7 +32,6 @@ struct phi_ctx {
 
   cudaStream_t stream = nullptr;
   int num_sms = 148;
-  int grid = 1;
   phi::DeviceHierarchy hier;
   PhiConstBuffers cbuf;
   phi::HeomConsts c{};

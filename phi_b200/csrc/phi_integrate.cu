@@ -98,7 +98,6 @@ cudaError_t enqueue_rk4_step(phi_ctx *ctx, double dt, double2 *traj, int par, cu
   L.c = ctx->c;
   ctx->bind_filter(L, par);
   L.mode = phi::kModeRk4;
-  L.grid = ctx->grid;
   L.y = ctx->y.as<double2>();
   L.acc = ctx->acc.as<double2>();
   L.rk4 = ctx->ctl.as<phi::Rk4Ctl>();
@@ -151,7 +150,6 @@ phi::StageLaunch rkf45_launch(phi_ctx *ctx) {
   phi::StageLaunch L;
   L.c = ctx->c;
   L.mode = phi::kModeRkf45;
-  L.grid = ctx->grid;
   L.ctl = ctx->ctl.as<phi::Rkf45Ctl>();
   ctx->bind_filter(L, 0);  // the kernels index the flags by ycur
   L.ybuf[0] = ctx->y.as<double2>();

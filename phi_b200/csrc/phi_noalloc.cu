@@ -115,7 +115,6 @@ extern "C" int phi_gpu_rk4_step_noalloc(phi_ctx *ctx, const void *d_in, void *d_
     phi::StageLaunch L;
     L.c = ctx->c;
     L.mode = phi::kModeRk4;
-    L.grid = ctx->grid;
     ctx->bind_filter(L, 0);
     const double a[4] = {dt / 2, dt / 2, dt, 0.0};
     const double w[4] = {dt / 6, dt / 3, dt / 3, dt / 6};

@@ -37,7 +37,6 @@ cudaError_t apply_fp64(phi_ctx *ctx, const double2 *in, double2 *out, cudaStream
   L.dot_part = dot_part;
   L.c = ctx->c;
   L.mode = phi::kModeApply;
-  L.grid = ctx->grid;
   L.x = in;
   L.out = out;
   L.xv = in;
@@ -163,7 +162,6 @@ cudaError_t build_deflation(phi_ctx *ctx, const phi::DeflView &D, const DeflPlan
   L.c.M = plan.rows_nodes;
   L.mode = phi::kModeApply;
   L.generic = true;
-  L.grid = phi::stage_grid(L.c, ctx->num_sms);
   L.x = D.units;
   L.out = D.AZ;
   L.batch = D.k;
