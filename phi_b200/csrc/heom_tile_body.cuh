@@ -164,7 +164,11 @@ __device__ __forceinline__ double2 cfma(double2 acc, double2 b, double s) {
 }
 template <class TX> __device__ __forceinline__ void st_stream(TX *p, TX v) { __stcs(p, v); }
 
-template <int N, bool MIXED, int KT, int BT = kTileThreads, bool RKF = false>
+// Which kernel a tile shape is for: the single-instance apply and RK4 stages,
+// the RKF45 stages, the batched stages.
+enum TileKind : int { kTileRk4 = 0, kTileRkf45 = 1, kTileBatch = 2 };
+
+template <int N, bool MIXED, int KT, int BT = kTileThreads, int ST = kTileRk4>
 struct TileShape {
   static constexpr int E = N * N;
   static constexpr int EP = E + (E & 1);  // complex64 node stride (16-byte aligned nodes)
@@ -172,16 +176,23 @@ struct TileShape {
   static constexpr int P = N * (N + 1) / 2;
   // How the neighbour terms are mapped (tile_derivative): by upper-triangle
   // pair, or by element.
-  static constexpr bool kPairs = RKF && N < 10;
+  static constexpr bool kPairs = ST == kTileRkf45 && N < 10;
   // Thread t < CS * N works on row t % N of the tile's columns t / N, t / N +
   // CS, ...: one H_ik serves all of a thread's elements, and a warp's
   // gathers and stores run along whole columns.
   static constexpr int CS = BT / N;
   // Nodes per tile: one pair per thread, or 32 bytes of elements per thread
-  // and operand; FP64 halves tiles of more than 40 nodes (sites <= 3), which
-  // would leave a small hierarchy too few CTAs (84-node trimer, 256 RK4
-  // steps: 4.35 -> 3.80 ms).
-  static constexpr int NT0 = kPairs ? BT / P : (MIXED ? 4 : (2 * CS / N > 40 ? 1 : 2)) * CS / N;
+  // and operand.  A single hierarchy halves tiles of more than 40 nodes
+  // (few sites), which would leave a small one too few CTAs (84-node trimer,
+  // 256 RK4 steps: FP64 4.35 -> 3.80 ms, mixed 4.83 -> 4.07; 4-site mixed
+  // apply over 125,970 nodes 29.9 -> 26.9 us); a batch has tiles enough and
+  // takes the large ones (48 instances: 30.1 -> 28.1 ms).
+  static constexpr int R1 = MIXED ? 4 : 2;
+  static constexpr int kRounds = ST == kTileBatch  ? (!MIXED && R1 * CS / N > 40 ? 1 : R1)
+                                 : R1 * CS / N <= 40 ? R1
+                                 : 2 * CS / N <= 40  ? 2
+                                                     : 1;
+  static constexpr int NT0 = kPairs ? BT / P : kRounds * CS / N;
   static constexpr int NT = NT0 < 1 ? 1 : (NT0 > 64 ? 64 : NT0);
   static constexpr int RR = (NT * N + CS - 1) / CS;  // elements per thread
   static constexpr int PR = (NT * P + BT - 1) / BT;  // pairs per thread
@@ -191,9 +202,9 @@ struct TileShape {
   static constexpr int EU = (N & 1) ? ES : N * NP;
 };
 
-template <int N, bool MIXED, int KT, int BT = kTileThreads, bool RKF = false>
+template <int N, bool MIXED, int KT, int BT = kTileThreads, int ST = kTileRk4>
 struct TileLayout {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   static constexpr int ES = S::ES;
   static constexpr int XB = MIXED ? 8 : 16;        // bytes per element of X / k
   // byte offsets in dynamic shared memory
@@ -281,9 +292,9 @@ __host__ __device__ constexpr int tile_warp_slots(int threads) { return (threads
 // This thread's share of a tile, the same in every tile: element r is row i
 // of column j of node nd.  Offsets of elements past the tile repeat its last
 // column, so every read stays inside the tile's buffers.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 struct TileMap {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   int i;
   int xo[S::RR];   // element in X (and k buffers): nd * ES + i + j * N
   int ut[S::RR];   // its transpose in the exchange tile
@@ -327,12 +338,12 @@ struct TileMap {
 // A = H X of this thread's elements, from shared memory: k runs outside, so
 // one H_ik serves all of the thread's elements and a warp's reads of X are
 // broadcasts along its columns.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
-__device__ __forceinline__ void tile_products(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, RKF> &m,
+template <int N, int KT, bool MIXED, int BT, int ST>
+__device__ __forceinline__ void tile_products(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, ST> &m,
                                               const typename TileArith<MIXED>::TX *Xs,
                                               const typename TileArith<MIXED>::TX *Hs,
-                                              typename TileArith<MIXED>::TX (&a)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+                                              typename TileArith<MIXED>::TX (&a)[TileShape<N, MIXED, KT, BT, ST>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
   using R = typename TileArith<MIXED>::R;
 #pragma unroll
@@ -367,11 +378,11 @@ __device__ __forceinline__ void tile_products(const HeomConsts &c, const TileMap
 }
 
 // What a tile's derivative is computed from (shared memory, except xin).
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 struct TileIn {
   using TX = typename TileArith<MIXED>::TX;
   using R = typename TileArith<MIXED>::R;
-  using C = TileCoef<R, TileShape<N, MIXED, KT, BT, RKF>::kPairs>;
+  using C = TileCoef<R, TileShape<N, MIXED, KT, BT, ST>::kPairs>;
   const TX *Xs;         // the tile's stage input
   TX *Us;               // exchange tile
   const TX *Hs;         // H
@@ -385,10 +396,10 @@ struct TileIn {
 };
 
 // The deepest tier's time-local term of element (i, j), i < j, of node nd.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
-__device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileIn<N, KT, MIXED, BT, RKF> &in, int nd, int i,
+template <int N, int KT, bool MIXED, int BT, int ST>
+__device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileIn<N, KT, MIXED, BT, ST> &in, int nd, int i,
                                                 int j, typename TileArith<MIXED>::TX &tv) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   int tier = 0;  // deepest tier only (is_timelocal_truncated)
   for (int t = 0; t < N * KT; ++t) tier += in.mi[nd * N * KT + t];
   if (tier != c.L) return false;
@@ -417,11 +428,11 @@ __device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileI
 //
 // Barriers: every thread of the CTA calls; Us must be free on entry, and is
 // free again after the CTA's next barrier.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
-__device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, RKF> &m,
-                                                const TileIn<N, KT, MIXED, BT, RKF> &in,
-                                                typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+template <int N, int KT, bool MIXED, int BT, int ST>
+__device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, ST> &m,
+                                                const TileIn<N, KT, MIXED, BT, ST> &in,
+                                                typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, ST>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
   using R = typename TileArith<MIXED>::R;
   constexpr int ES = S::ES, NP = S::NP, EU = S::EU, RR = S::RR, T = N * KT;
@@ -452,7 +463,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int r = 0; r < S::PR; ++r) gather(r);
     }
-    tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
+    tile_products<N, KT, MIXED, BT, ST>(c, m, in.Xs, in.Hs, dx);
 #pragma unroll
     for (int r = 0; r < RR; ++r)
       if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
@@ -502,7 +513,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
       TX v = mk<TX>(vx, vy);
       if (c.time_local && i != j) {
         TX tv;
-        if (tile_time_local<N, KT, MIXED, BT, RKF>(c, in, nd, i, j, tv)) {
+        if (tile_time_local<N, KT, MIXED, BT, ST>(c, in, nd, i, j, tv)) {
           v.x += tv.x;
           v.y += tv.y;
         }
@@ -517,7 +528,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
   } else {
     const int i = m.i;
     // FP64 issues the gathers after the products (registers).
-    constexpr bool kHoist = MIXED || KT == 1 || (KT == 2 && RKF);
+    constexpr bool kHoist = MIXED || KT == 1 || (KT == 2 && ST == kTileRkf45);
     TX gn[RR][KT], gp[RR][KT];
     auto gather = [&](int r) {
       const bool on = nb && m.on(r, in.nt_here);
@@ -534,7 +545,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int r = 0; r < RR; ++r) gather(r);
     }
-    tile_products<N, KT, MIXED, BT, RKF>(c, m, in.Xs, in.Hs, dx);
+    tile_products<N, KT, MIXED, BT, ST>(c, m, in.Xs, in.Hs, dx);
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
       if constexpr (!kHoist) gather(r);
@@ -581,7 +592,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
             nd = m.nd(q);
           }
         TX tv;
-        if (i == j || !tile_time_local<N, KT, MIXED, BT, RKF>(c, in, nd, i < j ? i : j, i < j ? j : i, tv)) continue;
+        if (i == j || !tile_time_local<N, KT, MIXED, BT, ST>(c, in, nd, i < j ? i : j, i < j ? j : i, tv)) continue;
 #pragma unroll
         for (int q = 0; q < RR; ++q)
           if (q == r) {
@@ -595,15 +606,15 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 
 // Byte offset of prefetched epilogue operand b: operand 0, then the others,
 // one size apart (each padded to 128 bytes).
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 __host__ __device__ __forceinline__ uint32_t tile_pre_size(int bytes) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   return ((uint32_t)S::NT * (bytes == 16 ? S::E : S::ES) * bytes + 127) / 128 * 128;
 }
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 __host__ __device__ __forceinline__ uint32_t tile_pre_off(const TileParams &p, int b) {
   return b == 0 ? 0
-                : tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[0]) + (b - 1) * tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[1]);
+                : tile_pre_size<N, KT, MIXED, BT, ST>(p.pre_bytes[0]) + (b - 1) * tile_pre_size<N, KT, MIXED, BT, ST>(p.pre_bytes[1]);
 }
 
 // Phase 3: the epilogue of this thread's elements (plain store, RK4 or RKF45
@@ -611,22 +622,23 @@ __host__ __device__ __forceinline__ uint32_t tile_pre_off(const TileParams &p, i
 // Pre; the RKF45 stage-5 error is folded into emax (max of |y4 - y5|, or of
 // its square in mixed precision).  coef holds the 24 RKF45 coefficients in
 // FP64 followed by the same 24 in FP32.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
-__device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap<N, KT, MIXED, BT, RKF> &m,
-                                              const TileIn<N, KT, MIXED, BT, RKF> &in, const unsigned char *Pre,
+template <int N, int KT, bool MIXED, int BT, int ST>
+__device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap<N, KT, MIXED, BT, ST> &m,
+                                              const TileIn<N, KT, MIXED, BT, ST> &in, const unsigned char *Pre,
                                               const double *coef, unsigned long long *wmax, long long tile,
                                               long long n0, int ycur, double &emax,
-                                              const typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, RKF>::RR]) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+                                              const typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, ST>::RR]) {
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
   using R = typename TileArith<MIXED>::R;
   constexpr int E = S::E, ES = S::ES, RR = S::RR;
+  constexpr bool RKF = ST == kTileRkf45;
   const int tid = threadIdx.x;
   // Element r of this thread: m.xo[r] in the tile's X / k ranges, m.eo(r) in
   // its complex128 ranges (and in the operands staged from either).
   const long long gx0 = n0 * ES, gd0 = n0 * E;
-  const uint32_t off1 = tile_pre_off<N, KT, MIXED, BT, RKF>(p, 1);
-  const uint32_t offs = tile_pre_size<N, KT, MIXED, BT, RKF>(p.pre_bytes[1]);
+  const uint32_t off1 = tile_pre_off<N, KT, MIXED, BT, ST>(p, 1);
+  const uint32_t offs = tile_pre_size<N, KT, MIXED, BT, ST>(p.pre_bytes[1]);
   const double2 *pre0d = reinterpret_cast<const double2 *>(Pre);
   const TX *pre0x = reinterpret_cast<const TX *>(Pre);
   // New filter flags follow: |y_new|^2 of every element goes to its slot of
@@ -820,12 +832,13 @@ __device__ __forceinline__ void tile_error_max(const TileParams &p, double emax,
 
 // New filter flags of a tile's nodes after the stage that writes the new
 // state (RK4 stage 3, RKF45 stage 5).
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 __device__ __forceinline__ void tile_flags(const TileParams &p, const typename TileArith<MIXED>::TX *Us, long long n0,
                                            int nt_here, int ycur) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
   const HeomConsts &c = p.c;
+  constexpr bool RKF = ST == kTileRkf45;
   if (!(c.filtered && p.stage == (RKF ? 5 : 3) && (RKF || p.mode == kModeRk4))) return;
   // Below the tolerance -> inactive, above -> active, equal -> unchanged
   // (hierarchy_integrator.cc:2827-2850, :2359-2384).
@@ -846,20 +859,20 @@ __device__ __forceinline__ void tile_flags(const TileParams &p, const typename T
 template <int N, int KT, bool MIXED, int BT = kTileThreads>
 __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, unsigned char *smem_raw,
                                          uint32_t par0, uint32_t par1) {
-  constexpr bool RKF = false;  // apply and RK4 stages
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
-  using Lay = TileLayout<N, MIXED, KT, BT, RKF>;
+  constexpr int ST = kTileBatch;  // apply and RK4 stages
+  using S = TileShape<N, MIXED, KT, BT, ST>;
+  using Lay = TileLayout<N, MIXED, KT, BT, ST>;
   using TX = typename std::conditional<MIXED, float2, double2>::type;
   using R = typename std::conditional<MIXED, float, double>::type;
   constexpr int E = S::E, NT = S::NT, ES = Lay::ES;
-  using In = TileIn<N, KT, MIXED, BT, RKF>;
+  using In = TileIn<N, KT, MIXED, BT, ST>;
   const HeomConsts &c = p.c;
   constexpr int T = N * KT;  // PHI's identity site map: K+1 terms per site
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + Lay::kBars);
   TX *Xs = reinterpret_cast<TX *>(smem_raw + Lay::kX);   // NT*ES
   TX *Us = reinterpret_cast<TX *>(smem_raw + Lay::kU);   // NT*EU (column stride NP)
   unsigned char *PreBase = smem_raw + Lay::kPre;
-  const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, RKF>(p, p.npre) : 0);
+  const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, ST>(p, p.npre) : 0);
   TX *Hs = reinterpret_cast<TX *>(smem_raw + tail);                 // E
   double *deph = reinterpret_cast<double *>(Hs + E + (E & 1));       // NT (16-aligned)
   unsigned long long *wmax = reinterpret_cast<unsigned long long *>(deph + NT + (NT & 1));  // per-warp sums
@@ -891,7 +904,7 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
       const unsigned char *src = static_cast<const unsigned char *>(p.pre[b]);
       const int stride = p.pre_bytes[b] == 16 ? E : ES;
       const uint32_t bytes = (uint32_t)(nt_here * stride * p.pre_bytes[b]);
-      bulk_g2s(PreBase + tile_pre_off<N, KT, MIXED, BT, RKF>(p, b), src + (size_t)n0 * stride * p.pre_bytes[b], bytes, &bars[1]);
+      bulk_g2s(PreBase + tile_pre_off<N, KT, MIXED, BT, ST>(p, b), src + (size_t)n0 * stride * p.pre_bytes[b], bytes, &bars[1]);
     }
   }
   // A real Hamiltonian (every in-scope workload) is kept as E reals in the
@@ -934,30 +947,31 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
     return -1;
   }
 
-  const TileMap<N, KT, MIXED, BT, RKF> m(c);
+  const TileMap<N, KT, MIXED, BT, ST> m(c);
   const In in{Xs, Us, Hs, mats, ids, cfs, deph, c.mi + n0 * T, xin, nt_here};
   TX dx[S::RR];
-  tile_derivative<N, KT, MIXED, BT, RKF>(c, m, in, dx);
+  tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
   ok = p.npre == 0 || mbar_wait_bounded(&bars[1], par1);
   if (!__syncthreads_and(ok)) {
     if (tid == 0) atomicOr(c.err_flag, 1);
     return -1;
   }
   double emax = 0.0;
-  tile_epilogue<N, KT, MIXED, BT, RKF>(p, m, in, PreBase, nullptr, wmax, tile, n0, 0, emax, dx);
-  tile_flags<N, KT, MIXED, BT, RKF>(p, Us, n0, nt_here, 0);
+  tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, nullptr, wmax, tile, n0, 0, emax, dx);
+  tile_flags<N, KT, MIXED, BT, ST>(p, Us, n0, nt_here, 0);
   return 0;
 }
 
-template <int N, int KT, bool MIXED, int BT = kTileThreads, bool RKF = false>
+// Shared memory of a batched tile.
+template <int N, int KT, bool MIXED, int BT = kTileThreads, int ST = kTileBatch>
 inline size_t tile_smem(int T, int npre, const int *pre_bytes) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
-  using Lay = TileLayout<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
+  using Lay = TileLayout<N, MIXED, KT, BT, ST>;
   size_t b = Lay::kPre;
-  for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, RKF>(pre_bytes[i]);
+  for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, ST>(pre_bytes[i]);
   b += (size_t)(S::E + (S::E & 1)) * Lay::XB;
   b += (size_t)(S::NT + (S::NT & 1) + tile_warp_slots(BT)) * sizeof(double);  // deph, warp sums
-  b += (size_t)S::NT * T * sizeof(typename TileIn<N, KT, MIXED, BT, RKF>::C);
+  b += (size_t)S::NT * T * sizeof(typename TileIn<N, KT, MIXED, BT, ST>::C);
   b += (size_t)(S::E + (S::E & 1)) * Lay::XB / 2;                     // mats
   b += (size_t)S::NT * T * sizeof(int2);                              // ids
   b += 16;

@@ -36,12 +36,12 @@ namespace {
 // exchange tile) took longer, because the operands' shared memory and two
 // barriers cost more than the 28 k FMAs of a node: 24-site RKF45 step 1.20 ms
 // against 0.87, and rho_0 after 47 steps 1.0e-6 off against 1.8e-7.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 struct PipeLayout {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   static constexpr int T = N * KT;
   static constexpr int ES = S::ES;
-  using C = typename TileIn<N, KT, MIXED, BT, RKF>::C;
+  using C = typename TileIn<N, KT, MIXED, BT, ST>::C;
   static constexpr int XB = MIXED ? 8 : 16;
   static constexpr int RB = MIXED ? 4 : 8;  // bytes of the arithmetic type
   static constexpr size_t r16(size_t b) { return (b + 15) / 16 * 16; }
@@ -60,12 +60,12 @@ struct PipeLayout {
   static constexpr size_t kPre = kUs + r128((size_t)S::NT * S::EU * XB);
 };
 
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 size_t pipe_smem(int T, int L, int npre, const int *pre_bytes) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
-  using Lay = PipeLayout<N, KT, MIXED, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
+  using Lay = PipeLayout<N, KT, MIXED, BT, ST>;
   size_t b = Lay::kPre;
-  for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, RKF>(pre_bytes[i]);
+  for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, ST>(pre_bytes[i]);
   const int W = L + 2, TW = T * W + ((T * W) & 1), E2 = S::E + (S::E & 1);
   b += (size_t)E2 * Lay::XB;                                          // H
   b += (size_t)(36 + tile_warp_slots(BT)) * sizeof(double);           // coef (FP64, FP32), warp maxima
@@ -77,13 +77,14 @@ size_t pipe_smem(int T, int L, int npre, const int *pre_bytes) {
   return b;
 }
 
-template <int N, int KT, bool MIXED, int BT, bool RKF>
-__global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, MIXED, KT, BT, RKF>::kPairs>::value) heom_tile_pipe_kernel(TileParams p) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
-  using Lay = PipeLayout<N, KT, MIXED, BT, RKF>;
+template <int N, int KT, bool MIXED, int BT, int ST>
+__global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, MIXED, KT, BT, ST>::kPairs>::value) heom_tile_pipe_kernel(TileParams p) {
+  using S = TileShape<N, MIXED, KT, BT, ST>;
+  using Lay = PipeLayout<N, KT, MIXED, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
   using R = typename TileArith<MIXED>::R;
   using C = typename Lay::C;
+  constexpr bool RKF = ST == kTileRkf45;
   constexpr int E = S::E, E2 = E + (E & 1), NT = S::NT, ES = Lay::ES, T = N * KT;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const HeomConsts &c = p.c;
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
   TX *Us = reinterpret_cast<TX *>(smem_raw + Lay::kUs);
   unsigned char *PreBase = smem_raw + Lay::kPre;
-  const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, RKF>(p, p.npre) : 0);
+  const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, ST>(p, p.npre) : 0);
   const int W = c.L + 2, TW = T * W + ((T * W) & 1);
   TX *Hs = reinterpret_cast<TX *>(smem_raw + tail);                           // E
   double *coef = reinterpret_cast<double *>(Hs + E2);                         // 24, then 24 floats
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
       if (RKF && b == 0)
         src = static_cast<const unsigned char *>(p.pre_bytes[0] == 8 ? p.y32buf[ycur] : (const void *)p.ybuf[ycur]);
       const int stride = p.pre_bytes[b] == 16 ? E : ES;
-      bulk_g2s(PreBase + tile_pre_off<N, KT, MIXED, BT, RKF>(p, b), src + (size_t)n0 * stride * p.pre_bytes[b],
+      bulk_g2s(PreBase + tile_pre_off<N, KT, MIXED, BT, ST>(p, b), src + (size_t)n0 * stride * p.pre_bytes[b],
                (uint32_t)(nt * stride * p.pre_bytes[b]), &bars[2]);
     }
   };
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     }
   };
 
-  const TileMap<N, KT, MIXED, BT, RKF> m(c);
+  const TileMap<N, KT, MIXED, BT, ST> m(c);
   double emax = 0.0;
   int i = 0;
   // ok: this thread's waits so far; checked by the whole CTA at the barrier
@@ -247,10 +248,10 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     const TX *Xs = reinterpret_cast<const TX *>(sb);
     const double *deph =
         reinterpret_cast<const double *>(sb + Lay::kSlotX + 2 * Lay::kSlotIds + Lay::kSlotMi) + (n0 & 1);
-    const TileIn<N, KT, MIXED, BT, RKF> in{Xs,   Us,   Hs, mats, ids + s * NT * T, cfs + s * NT * T,
+    const TileIn<N, KT, MIXED, BT, ST> in{Xs,   Us,   Hs, mats, ids + s * NT * T, cfs + s * NT * T,
                                       deph, slot_mi(s, n0), xin, nt_here};
     TX dx[S::RR];
-    tile_derivative<N, KT, MIXED, BT, RKF>(c, m, in, dx);
+    tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
     // The operands have had the derivative's time to land.  A wait that gave
     // up skips the stores; the tile's last barrier then ends the CTA.
     ok = p.npre == 0 || mbar_wait_bounded(&bars[2], (uint32_t)i & 1u);
@@ -261,8 +262,8 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
         break;
       }
     }
-    if (ok) tile_epilogue<N, KT, MIXED, BT, RKF>(p, m, in, PreBase, coef, wmax, tile, n0, ycur, emax, dx);
-    tile_flags<N, KT, MIXED, BT, RKF>(p, Us, n0, nt_here, ycur);
+    if (ok) tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, coef, wmax, tile, n0, ycur, emax, dx);
+    tile_flags<N, KT, MIXED, BT, ST>(p, Us, n0, nt_here, ycur);
     if (next_issued) {
       const bool got = mbar_wait_bounded(&bars[s ^ 1], (uint32_t)((i + 1) >> 1) & 1u, polls0);
       if (got) records(tile + gridDim.x, s ^ 1);
@@ -314,17 +315,17 @@ int persistent_grid(const void *fn, int threads, size_t smem) {
 // this launch's shared-memory size (capped at tile_cps CTAs per SM when the
 // schedule sets it) and never more than the tiles.  *per_sm (optional)
 // receives the resident CTAs per SM before the cap.
-template <int N, int KT, bool MIXED, int BT, bool RKF>
+template <int N, int KT, bool MIXED, int BT, int ST>
 cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
-  using S = TileShape<N, MIXED, KT, BT, RKF>;
+  using S = TileShape<N, MIXED, KT, BT, ST>;
   const long long tiles = (p.c.M + S::NT - 1) / S::NT;
   const int max_bytes[kMaxPre] = {16, 16, 16, 16, 16};
-  const size_t smem_max = pipe_smem<N, KT, MIXED, BT, RKF>(p.c.T, p.c.L, kMaxPre, max_bytes);
-  auto kern = heom_tile_pipe_kernel<N, KT, MIXED, BT, RKF>;
+  const size_t smem_max = pipe_smem<N, KT, MIXED, BT, ST>(p.c.T, p.c.L, kMaxPre, max_bytes);
+  auto kern = heom_tile_pipe_kernel<N, KT, MIXED, BT, ST>;
   static thread_local int configured[kSmemLimitDevices] = {};
   cudaError_t e = raise_smem_limit(kern, smem_max, configured);
   if (e != cudaSuccess) return e;
-  const size_t smem = pipe_smem<N, KT, MIXED, BT, RKF>(p.c.T, p.c.L, p.npre, p.pre_bytes);
+  const size_t smem = pipe_smem<N, KT, MIXED, BT, ST>(p.c.T, p.c.L, p.npre, p.pre_bytes);
   int cap = persistent_grid((const void *)kern, BT, smem);
   if (cap <= 0) return cudaErrorInvalidConfiguration;
   int sms = 0, dev = 0;
@@ -337,39 +338,39 @@ cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm
   return cudaGetLastError();
 }
 
-template <int N, int KT, bool MIXED, bool RKF>
+template <int N, int KT, bool MIXED, int ST>
 cudaError_t launch_tile_nk(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   // The steady-state apply writes one partial inner product per tile into
   // an array sized by tile_count, i.e. by the default block's tiles.
   if (p.c.tile_variant == 1 && !p.dot_w)
-    return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::alt, RKF>(p, stream, per_sm);
-  return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::threads, RKF>(p, stream, per_sm);
+    return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::alt, ST>(p, stream, per_sm);
+  return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::threads, ST>(p, stream, per_sm);
 }
 
-template <int N, bool MIXED, bool RKF>
+template <int N, bool MIXED, int ST>
 cudaError_t launch_tile_n(const TileParams &p, cudaStream_t stream, int *per_sm) {
   switch (p.c.K1) {
-    case 1: return launch_tile_nk<N, 1, MIXED, RKF>(p, stream, per_sm);
-    case 2: return launch_tile_nk<N, 2, MIXED, RKF>(p, stream, per_sm);
-    case 3: return launch_tile_nk<N, 3, MIXED, RKF>(p, stream, per_sm);
+    case 1: return launch_tile_nk<N, 1, MIXED, ST>(p, stream, per_sm);
+    case 2: return launch_tile_nk<N, 2, MIXED, ST>(p, stream, per_sm);
+    case 3: return launch_tile_nk<N, 3, MIXED, ST>(p, stream, per_sm);
     default: return cudaErrorInvalidValue;
   }
 }
 
-template <bool MIXED, bool RKF>
+template <bool MIXED, int ST>
 cudaError_t launch_tile_dispatch(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   switch (p.c.N) {
-    case 2: return launch_tile_n<2, MIXED, RKF>(p, stream, per_sm);
-    case 3: return launch_tile_n<3, MIXED, RKF>(p, stream, per_sm);
-    case 4: return launch_tile_n<4, MIXED, RKF>(p, stream, per_sm);
-    case 5: return launch_tile_n<5, MIXED, RKF>(p, stream, per_sm);
-    case 6: return launch_tile_n<6, MIXED, RKF>(p, stream, per_sm);
-    case 7: return launch_tile_n<7, MIXED, RKF>(p, stream, per_sm);
-    case 8: return launch_tile_n<8, MIXED, RKF>(p, stream, per_sm);
-    case 10: return launch_tile_n<10, MIXED, RKF>(p, stream, per_sm);
-    case 12: return launch_tile_n<12, MIXED, RKF>(p, stream, per_sm);
-    case 16: return launch_tile_n<16, MIXED, RKF>(p, stream, per_sm);
-    case 24: return launch_tile_n<24, MIXED, RKF>(p, stream, per_sm);
+    case 2: return launch_tile_n<2, MIXED, ST>(p, stream, per_sm);
+    case 3: return launch_tile_n<3, MIXED, ST>(p, stream, per_sm);
+    case 4: return launch_tile_n<4, MIXED, ST>(p, stream, per_sm);
+    case 5: return launch_tile_n<5, MIXED, ST>(p, stream, per_sm);
+    case 6: return launch_tile_n<6, MIXED, ST>(p, stream, per_sm);
+    case 7: return launch_tile_n<7, MIXED, ST>(p, stream, per_sm);
+    case 8: return launch_tile_n<8, MIXED, ST>(p, stream, per_sm);
+    case 10: return launch_tile_n<10, MIXED, ST>(p, stream, per_sm);
+    case 12: return launch_tile_n<12, MIXED, ST>(p, stream, per_sm);
+    case 16: return launch_tile_n<16, MIXED, ST>(p, stream, per_sm);
+    case 24: return launch_tile_n<24, MIXED, ST>(p, stream, per_sm);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -230,7 +230,7 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
     }
   }
   if (phi::tile_kernel_available(ctx->c) && !ctx->bicg_parts.ptr) {
-    ctx->bicg_tiles = phi::tile_count(ctx->c, false);
+    ctx->bicg_tiles = phi::tile_count(ctx->c, false, false);
     if (ctx->bicg_tiles > 0 &&
         ctx->bicg_parts.alloc((size_t)2 * (ctx->bicg_tiles + 1) * sizeof(double)) != cudaSuccess) {
       ctx->error = "steady_state: allocation of the per-tile partial sums failed";
