@@ -39,6 +39,33 @@ inline cudaError_t raise_smem_limit(Kernel kern, size_t bytes, int (&seen)[kSmem
   return e;
 }
 
+// Programmatic dependent launch: the next kernel may start its preamble; this
+// one continues once the previous kernel's writes are visible (both no-ops in
+// a launch without the attribute).  A kernel reads what a preceding kernel
+// wrote only after pdl_wait, and never through the read-only path (__ldg):
+// such memory changes while the kernel is resident.
+__device__ __forceinline__ void pdl_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches kern(args...) with that attribute.
+template <class Kernel, class... Args>
+inline cudaError_t launch_dependent(Kernel kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    const Args &...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // Read-only problem constants, built on the host once per context.  Mirrors
 // what PHI keeps per node (HierarchyNode prefactors, hierarchy_node.h:139-208)
 // but stores it per term: the per-node values are recomputed in registers.
@@ -52,6 +79,7 @@ struct HeomConsts {
   int vacuum;       // truncation_level == 1: unitary part only
   int identity_sites;  // independent baths: bath m couples to |m><m|
   int h_real;       // every Hamiltonian element has a zero imaginary part
+  int h_dynamic;    // H changes between stages (annealing)
   int64_t M;        // nodes
   double inv_hbar;  // 1 / hbar
   const uint8_t *mi;     // M*T

@@ -51,20 +51,13 @@ namespace {
 __device__ __forceinline__ double2 c_axpy(double2 a, double2 b, double s) {
   return make_double2(fma(b.x, s, a.x), fma(b.y, s, a.y));
 }
-// Data that a preceding stage kernel wrote: past L1, which may hold lines of a
-// kernel that ran beside this one's preamble.
+// Data that a preceding stage kernel wrote.
 __device__ __forceinline__ double2 ld_global(const double2 *p) { return __ldcg(p); }
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Programmatic dependent launch: the next kernel may start its preamble; this
-// one continues once the previous kernel's writes are visible (both no-ops in
-// a launch without the attribute).
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 constexpr int kNodeThreads = 512;   // at most
 constexpr int kNodeRounds = 2;      // elements of a thread whose neighbour sums stay in registers
 constexpr int kNodeMaxOps = 5;      // combine operands
@@ -657,17 +650,8 @@ cudaError_t launch_node(const StageParams &p, int batch, cudaStream_t stream) {
   static thread_local int configured[kSmemLimitDevices] = {};
   cudaError_t e = raise_smem_limit(kern, p.plan.bytes, configured);
   if (e != cudaSuccess) return e;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch);
-  cfg.blockDim = dim3(p.plan.threads);
-  cfg.dynamicSmemBytes = p.plan.bytes;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  return launch_dependent(kern, dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch), dim3(p.plan.threads),
+                          p.plan.bytes, stream, p);
 }
 
 }  // namespace

@@ -70,6 +70,7 @@ TileParams tile_params_for(const StageLaunch &L) {
   const bool mixed = L.mixed;
   const int xb = mixed ? 8 : 16;
   // Epilogue operands of this (mode, stage), in the order the epilogue reads them.
+  p.dependent = 0;  // set by the launch
   p.npre = 0;
   for (int b = 0; b < kMaxPre; ++b) {
     p.pre[b] = nullptr;

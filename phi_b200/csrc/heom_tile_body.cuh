@@ -88,6 +88,7 @@ struct TileParams {
   int act_par;
   const double2 *dot_w;          // FP64 apply: <dot_w, out> per tile (see StageLaunch)
   double *dot_part;
+  int dependent;                 // launched as a dependent of the previous kernel
   int npre;                      // epilogue operands prefetched
   const void *pre[kMaxPre];      // sources; slot 0 of RKF45 is chosen on the device
   int pre_bytes[kMaxPre];        // 16 (complex128) or 8 (complex64)
@@ -453,10 +454,10 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int q = 0; q < KT; ++q) {
         const int2 idj = in.ids[ndr * T + j * KT + q], idi = in.ids[ndr * T + i * KT + q];
-        gn_c[r][q] = (on && idj.x >= 0 && i != j) ? __ldg(in.xin + idj.x + oij) : zero;
-        gp_c[r][q] = (on && idj.y >= 0 && i != j) ? __ldg(in.xin + idj.y + oij) : zero;
-        gn_r[r][q] = (on && idi.x >= 0 && i != j) ? __ldg(in.xin + idi.x + oji) : zero;
-        gp_r[r][q] = (on && idi.y >= 0) ? __ldg(in.xin + idi.y + oji) : zero;
+        gn_c[r][q] = (on && idj.x >= 0 && i != j) ? *(in.xin + idj.x + oij) : zero;
+        gp_c[r][q] = (on && idj.y >= 0 && i != j) ? *(in.xin + idj.y + oij) : zero;
+        gn_r[r][q] = (on && idi.x >= 0 && i != j) ? *(in.xin + idi.x + oji) : zero;
+        gp_r[r][q] = (on && idi.y >= 0) ? *(in.xin + idi.y + oji) : zero;
       }
     };
     if constexpr (kHoist) {
@@ -537,8 +538,8 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int q = 0; q < KT; ++q) {
         const int2 id = in.ids[m.rec[r] + q];
-        gn[r][q] = (on && id.x >= 0 && !diag) ? __ldg(in.xin + id.x + off) : zero;
-        gp[r][q] = (on && id.y >= 0) ? __ldg(in.xin + id.y + off) : zero;
+        gn[r][q] = (on && id.x >= 0 && !diag) ? *(in.xin + id.x + off) : zero;
+        gp[r][q] = (on && id.y >= 0) ? *(in.xin + id.y + off) : zero;
       }
     };
     if constexpr (kHoist) {
@@ -668,7 +669,7 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap
           TX v = dx[r];
           if (gx0 + m.xo[r] == 0) v = mk<TX>(0.0, 0.0);
           st_stream(out + m.xo[r], v);
-          const double2 w = __ldg(p.dot_w + gx0 + m.xo[r]);
+          const double2 w = __ldcg(p.dot_w + gx0 + m.xo[r]);
           dsum = fma(w.x, v.x, fma(w.y, v.y, dsum));
         }
       for (int off = 16; off > 0; off >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
@@ -745,7 +746,7 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap
       } else if (MIXED || p.pre_bytes[0] != 0) {
         xv[r] = pre0x[x];
       } else {
-        xv[r] = m.on(r, in.nt_here) ? from_d2<TX>(__ldg(p.ybuf[ycur] + gd0 + x)) : mk<TX>(0.0, 0.0);
+        xv[r] = m.on(r, in.nt_here) ? from_d2<TX>(__ldcg(p.ybuf[ycur] + gd0 + x)) : mk<TX>(0.0, 0.0);
       }
     }
     const TX *kb = reinterpret_cast<const TX *>(Pre + off1);
@@ -778,7 +779,7 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap
       if (!m.on(r, in.nt_here)) continue;
       const int x = m.xo[r], e = m.eo(r);
       const double2 kv = to_d2(dx[r]);
-      const double2 ys = p.pre_bytes[0] == 0 ? __ldg(p.ybuf[ycur] + gd0 + e) : pre0d[e];
+      const double2 ys = p.pre_bytes[0] == 0 ? __ldcg(p.ybuf[ycur] + gd0 + e) : pre0d[e];
       const double2 k0 = to_d2(kb[x]), k2 = to_d2(kb[ksz + x]);
       const double2 k3 = to_d2(kb[2 * ksz + x]), k4 = to_d2(kb[3 * ksz + x]);
       double2 y4 = cfma(ys, k0, cf[15]);

@@ -25,8 +25,9 @@ namespace {
 // epilogue operands of tile i (y, accumulator, k_r) are issued when tile i
 // starts and land while its derivative runs; tile i+1's neighbour offsets and
 // coefficients are prepared at the end of tile i, so one barrier ends a tile
-// and starts the next.  The first tile's copies are issued before H, the
-// Matsubara factors, c_t and the prefactor tables are staged (once per CTA).
+// and starts the next.  H, the Matsubara factors, c_t and the prefactor tables
+// are staged once per CTA: while the first tile's copies run, or, in a
+// dependent launch, before the wait on the previous stage's kernel.
 // mbarriers: one per slot (phase parity (i >> 1) & 1 for the CTA's i-th
 // tile) and one for the epilogue operands (parity i & 1).
 //
@@ -89,7 +90,6 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const HeomConsts &c = p.c;
   const int tid = threadIdx.x;
-  if (RKF && *(volatile int *)&p.ctl->done) return;  // uniform across the grid
 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
   TX *Us = reinterpret_cast<TX *>(smem_raw + Lay::kUs);
@@ -112,18 +112,10 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     mbar_init(&bars[2], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const int ycur = RKF ? p.ctl->ycur : 0;
   const long long ntiles = (c.M + NT - 1) / NT;
-  const TX *xin;
-  if (RKF && p.stage == 0)
-    xin = MIXED ? static_cast<const TX *>(p.y32buf[ycur]) : reinterpret_cast<const TX *>(p.ybuf[ycur]);
-  else
-    xin = static_cast<const TX *>(p.x);
-  // Filtering: an inactive neighbour contributes nothing (the DoNext /
-  // DoPrevious overrides of IndependentBathAdaptiveTruncation,
-  // hierarchy_updater.cc:256-303).
-  const uint8_t *act_in = c.filtered ? p.act[RKF ? ycur : p.act_par] : nullptr;
-  const long long polls0 = c.first_wait_polls == 0 ? kMaxPolls : (c.first_wait_polls < 0 ? 0 : c.first_wait_polls);
+  long long tile = blockIdx.x;
+  int ycur = 0;
+  const TX *xin = static_cast<const TX *>(p.x);
 
   // Thread 0: the X and neighbour records of `tile` into slot s.
   auto issue_slot = [&](long long tile, int s) {
@@ -142,27 +134,51 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     bulk_g2s(b + Lay::kSlotX + 2 * Lay::kSlotIds, c.mi + a16, mibytes, &bars[s]);
     bulk_g2s(b + Lay::kSlotX + 2 * Lay::kSlotIds + Lay::kSlotMi, c.deph_node + a2, dbytes, &bars[s]);
   };
-  // The first tile's copies run while the constants are staged (the barriers
-  // reach the other threads at the barrier below).
-  long long tile = blockIdx.x;
-  if (tid == 0 && tile < ntiles) issue_slot(tile, 0);
-  if (RKF && tid < 24) {
-    const double v = p.ctl->coef[tid];
-    coef[tid] = v;
-    reinterpret_cast<float *>(coef + 24)[tid] = (float)v;
+  // What needs the previous kernel's results: false once the RKF45 run is done
+  // (uniform across the grid), else the first tile's copies.
+  auto begin = [&]() {
+    if (RKF) {
+      if (*(volatile int *)&p.ctl->done) return false;
+      ycur = *(volatile int *)&p.ctl->ycur;
+      if (p.stage == 0)
+        xin = MIXED ? static_cast<const TX *>(p.y32buf[ycur]) : reinterpret_cast<const TX *>(p.ybuf[ycur]);
+    }
+    if (tid == 0 && tile < ntiles) issue_slot(tile, 0);
+    return true;
+  };
+  if (p.dependent) {
+    pdl_launch_dependents();
+    if (c.h_dynamic) pdl_wait();  // H is read below
+  } else if (!begin()) {
+    return;
   }
   const bool hreal = c.h_real;
   R *Hr = reinterpret_cast<R *>(Hs);
   if (hreal) {
-    for (int i = tid; i < E; i += BT) Hr[i] = (R)__ldg(c.H + i).x;
+    for (int i = tid; i < E; i += BT) Hr[i] = (R)__ldcg(c.H + i).x;
   } else {
-    for (int i = tid; i < E; i += BT) Hs[i] = from_d2<TX>(__ldg(c.H + i));
+    for (int i = tid; i < E; i += BT) Hs[i] = from_d2<TX>(__ldcg(c.H + i));
   }
   for (int i = tid; i < E; i += BT) mats[i] = (R)__ldg(c.mats_elem + i);
   for (int t = tid; t < T; t += BT) ccs[t] = __ldg(c.corr + t);
   for (int q = tid; q < T * W; q += BT) {
     sqn[q] = (R)__ldg(c.sq_next + q);
     sqp[q] = (R)__ldg(c.sq_prev + q);
+  }
+  if (p.dependent) {
+    pdl_wait();
+    if (!begin()) return;
+  }
+  // Filtering: an inactive neighbour contributes nothing (the DoNext /
+  // DoPrevious overrides of IndependentBathAdaptiveTruncation,
+  // hierarchy_updater.cc:256-303).
+  const uint8_t *act_in = c.filtered ? p.act[RKF ? ycur : p.act_par] : nullptr;
+  const long long polls0 = c.first_wait_polls == 0 ? kMaxPolls : (c.first_wait_polls < 0 ? 0 : c.first_wait_polls);
+
+  if (RKF && tid < 24) {
+    const double v = __ldcg(&p.ctl->coef[tid]);
+    coef[tid] = v;
+    reinterpret_cast<float *>(coef + 24)[tid] = (float)v;
   }
   __syncthreads();  // barriers initialised, constants visible
 
@@ -212,8 +228,8 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     for (int q = tid; q < nt * T; q += BT) {
       const int t = q % T;
       const int nx = nx_s[q], pv = pv_s[q], occ = mi_s[q];
-      const bool nx_on = nx >= 0 && (!act_in || __ldg(act_in + nx));
-      const bool pv_on = pv >= 0 && (!act_in || __ldg(act_in + pv));
+      const bool nx_on = nx >= 0 && (!act_in || __ldcg(act_in + nx));
+      const bool pv_on = pv >= 0 && (!act_in || __ldcg(act_in + pv));
       ids[s * NT * T + q] = make_int2(nx_on ? nx * ES : -1, pv_on ? pv * ES : -1);
       cfs[s * NT * T + q] = tile_coef<C, R>(sqn[t * W + occ], sqp[t * W + occ], ccs[t]);
     }
@@ -334,6 +350,16 @@ cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm
   if (per_sm) *per_sm = cap / sms;
   if (p.c.tile_cps > 0 && p.c.tile_cps * sms < cap) cap = p.c.tile_cps * sms;
   const long long grid = tiles < cap ? tiles : cap;
+  // Dependent launch (the preamble overlaps the previous kernel) for the
+  // apply and where every CTA has one tile: 8-site mixed RK4 stage 6.5 -> 5.5
+  // us, 84-node trimer 4.0 -> 3.0 us, 4-site apply 37.2 -> 34.5 us.  Stages
+  // of several tiles per CTA gained up to 10 % (24 sites) but lost up to 22 %
+  // (7-site mixed RKF45), so they keep the plain launch.
+  if (p.mode == kModeApply || tiles <= cap) {
+    TileParams d = p;
+    d.dependent = 1;
+    return launch_dependent(kern, dim3((unsigned)grid), dim3(BT), smem, stream, d);
+  }
   kern<<<(unsigned)grid, BT, smem, stream>>>(p);
   return cudaGetLastError();
 }

@@ -595,6 +595,7 @@ extern "C" int phi_gpu_create(const phi_problem_desc *desc, phi_ctx **out) {
     ctx->c.h_real = 1;
     for (int k = 0; k < N * N; ++k)
       if (d.annealing_h_x[2 * k + 1] != 0.0 || d.annealing_h_z[2 * k + 1] != 0.0) ctx->c.h_real = 0;
+    ctx->c.h_dynamic = 1;
     if (e == cudaSuccess) e = ctx->reset_annealing();
   }
   if (e == cudaSuccess && ctx->c.time_local) {
