@@ -35,6 +35,7 @@
 #include <cstdint>
 
 #include "heom_bicgstab.h"
+#include "heom_device.cuh"
 
 namespace phi {
 namespace {
@@ -103,6 +104,11 @@ __device__ __forceinline__ bool grid_sum(double (&v)[K], double (&tot)[K], doubl
 #define GRID_LOOP(i, n) \
   for (long long i = blockIdx.x * (long long)kBlock + threadIdx.x; i < (n); i += (long long)gridDim.x * kBlock)
 
+// The passes over the Krylov vectors run from the end to the start where the
+// kernel before them ran forward (the applies do, the minimal-residual update
+// does): the part of the vectors still in L2 is then read first.  They are
+// bound by memory bandwidth: 4-site chain, 32 MB per vector, 126 MB of L2.
+
 __device__ __forceinline__ bool solve_done(const BicgScalars *sc) { return *(volatile const int *)&sc->done; }
 
 __device__ __forceinline__ void fail(BicgScalars *sc, int code) {
@@ -154,6 +160,8 @@ __global__ void init_kernel(BicgVectors V, long long n, BicgScalars *sc) {
 // BiCG step j >= 1: rho1 = <rhat, r_j>, beta = alpha rho1 / rho0, rho0 = rho1.
 // Also drops element 0 of r_j = A r_{j-1}.
 __global__ void rho_kernel(BicgVectors V, long long n, BicgScalars *sc, int j) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (solve_done(sc)) return;
   double2 *rj = V.r[j];
   double acc[1] = {0.0}, tot[1];
@@ -176,20 +184,58 @@ __global__ void rho_kernel(BicgVectors V, long long n, BicgScalars *sc, int j) {
   }
 }
 
-// u_i = r_i - beta u_i for i = 0..j.
-__global__ void u_update_kernel(BicgVectors V, long long n, const BicgScalars *sc, int j) {
-  if (solve_done(sc)) return;
-  const double beta = sc->beta;
-  GRID_LOOP(e, n) {
-    for (int i = 0; i <= j; ++i) {
-      const double2 r = V.r[i][e], u = V.u[i][e];
-      V.u[i][e] = make_double2(r.x - beta * u.x, r.y - beta * u.y);
+// u_i = r_i - beta u_i for i = 0..j; for j >= 1 also the x += alpha u_0 of BiCG
+// step j - 1, which this pass reads u_0 for anyway (the last step's is in
+// mr_update_kernel).
+template <int J>
+__device__ __forceinline__ void u_update_pass(const BicgVectors &V, long long n, const BicgScalars *sc) {
+  const double beta = sc->beta, alpha = sc->alpha;
+  constexpr int U = J == 0 ? 4 : (J == 1 ? 2 : 1);  // elements whose loads are in flight together
+  const long long stride = (long long)gridDim.x * kBlock;
+  for (long long e0 = n - 1 - (blockIdx.x * (long long)kBlock + threadIdx.x); e0 >= 0; e0 -= U * stride) {
+    double2 r[U][J + 1], u[U][J + 1], x[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long e = e0 - q * stride;
+      if (e < 0) break;
+#pragma unroll
+      for (int i = 0; i <= J; ++i) {
+        r[q][i] = V.r[i][e];
+        u[q][i] = V.u[i][e];
+      }
+      if (J >= 1) x[q] = V.x[e];
     }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long e = e0 - q * stride;
+      if (e < 0) break;
+#pragma unroll
+      for (int i = 0; i <= J; ++i)
+        V.u[i][e] = make_double2(r[q][i].x - beta * u[q][i].x, r[q][i].y - beta * u[q][i].y);
+      if (J >= 1) V.x[e] = make_double2(x[q].x + alpha * u[q][0].x, x[q].y + alpha * u[q][0].y);
+    }
+  }
+}
+__global__ void __launch_bounds__(kBlock) u_update_kernel(BicgVectors V, long long n, const BicgScalars *sc, int j) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (solve_done(sc)) return;
+  switch (j) {
+    case 0: return u_update_pass<0>(V, n, sc);
+    case 1: return u_update_pass<1>(V, n, sc);
+    case 2: return u_update_pass<2>(V, n, sc);
+    case 3: return u_update_pass<3>(V, n, sc);
+    case 4: return u_update_pass<4>(V, n, sc);
+    case 5: return u_update_pass<5>(V, n, sc);
+    case 6: return u_update_pass<6>(V, n, sc);
+    default: return u_update_pass<7>(V, n, sc);
   }
 }
 
 // alpha = rho0 / <rhat, u_{j+1}>; drops element 0 of u_{j+1} = A u_j.
 __global__ void gamma_kernel(BicgVectors V, long long n, BicgScalars *sc, int j) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (solve_done(sc)) return;
   double2 *uj = V.u[j + 1];
   double acc[1] = {0.0}, tot[1];
@@ -207,10 +253,12 @@ __global__ void gamma_kernel(BicgVectors V, long long n, BicgScalars *sc, int j)
   }
 }
 
-// rho_kernel / gamma_kernel's scalar steps from per-tile partial sums of
+// rho_kernel / gamma_kernel's scalar steps from per-CTA partial sums of
 // <rhat, .> (the apply zeroed element 0 and summed them); one block, summed
-// in tile order (deterministic).
+// in order (deterministic).
 __global__ void dot_finish_kernel(const double *parts, long long nparts, BicgScalars *sc, int which) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (solve_done(sc)) return;
   double v[1] = {0.0};
   for (long long b = threadIdx.x; b < nparts; b += kBlock) v[0] += parts[b];
@@ -219,17 +267,47 @@ __global__ void dot_finish_kernel(const double *parts, long long nparts, BicgSca
   bicg_dot_step(sc, v[0], which);
 }
 
-// r_i -= alpha u_{i+1} for i = 0..j; x += alpha u_0.
-__global__ void r_update_kernel(BicgVectors V, long long n, const BicgScalars *sc, int j) {
-  if (solve_done(sc)) return;
+// r_i -= alpha u_{i+1} for i = 0..j.
+template <int J>
+__device__ __forceinline__ void r_update_pass(const BicgVectors &V, long long n, const BicgScalars *sc) {
   const double a = sc->alpha;
-  GRID_LOOP(e, n) {
-    for (int i = 0; i <= j; ++i) {
-      const double2 r = V.r[i][e], u = V.u[i + 1][e];
-      V.r[i][e] = make_double2(r.x - a * u.x, r.y - a * u.y);
+  constexpr int U = J == 0 ? 4 : (J == 1 ? 2 : 1);
+  const long long stride = (long long)gridDim.x * kBlock;
+  for (long long e0 = n - 1 - (blockIdx.x * (long long)kBlock + threadIdx.x); e0 >= 0; e0 -= U * stride) {
+    double2 r[U][J + 1], u[U][J + 1];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long e = e0 - q * stride;
+      if (e < 0) break;
+#pragma unroll
+      for (int i = 0; i <= J; ++i) {
+        r[q][i] = V.r[i][e];
+        u[q][i] = V.u[i + 1][e];
+      }
     }
-    const double2 x = V.x[e], u0 = V.u[0][e];
-    V.x[e] = make_double2(x.x + a * u0.x, x.y + a * u0.y);
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long e = e0 - q * stride;
+      if (e < 0) break;
+#pragma unroll
+      for (int i = 0; i <= J; ++i)
+        V.r[i][e] = make_double2(r[q][i].x - a * u[q][i].x, r[q][i].y - a * u[q][i].y);
+    }
+  }
+}
+__global__ void __launch_bounds__(kBlock) r_update_kernel(BicgVectors V, long long n, const BicgScalars *sc, int j) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (solve_done(sc)) return;
+  switch (j) {
+    case 0: return r_update_pass<0>(V, n, sc);
+    case 1: return r_update_pass<1>(V, n, sc);
+    case 2: return r_update_pass<2>(V, n, sc);
+    case 3: return r_update_pass<3>(V, n, sc);
+    case 4: return r_update_pass<4>(V, n, sc);
+    case 5: return r_update_pass<5>(V, n, sc);
+    case 6: return r_update_pass<6>(V, n, sc);
+    default: return r_update_pass<7>(V, n, sc);
   }
 }
 
@@ -241,26 +319,36 @@ __host__ __device__ constexpr int gram_index(int i, int k) { return (k - 1) * k 
 // r_ell = A r_{ell-1}.
 template <int ELL>
 __global__ void gram_kernel(BicgVectors V, long long n, BicgScalars *sc) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (solve_done(sc)) return;
   constexpr int NG = ELL * (ELL + 1) / 2;
   constexpr int ND = NG + ELL;
   double acc[ND], tot[ND];
 #pragma unroll
   for (int k = 0; k < ND; ++k) acc[k] = 0.0;
-  GRID_LOOP(e, n) {
-    if (e == 0) {
-      V.r[ELL][0] = make_double2(0.0, 0.0);
-      continue;
+  constexpr int U = ELL <= 2 ? 4 : 1;  // elements whose loads are in flight together
+  const long long stride = (long long)gridDim.x * kBlock;
+  for (long long e0 = n - 1 - (blockIdx.x * (long long)kBlock + threadIdx.x); e0 >= 0; e0 -= U * stride) {
+    double2 r[U][ELL + 1];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long e = e0 - q * stride;
+#pragma unroll
+      for (int i = 0; i <= ELL; ++i) r[q][i] = e >= 0 ? V.r[i][e] : make_double2(0.0, 0.0);
+      if (e == 0) {
+        V.r[ELL][0] = make_double2(0.0, 0.0);
+        r[q][ELL] = make_double2(0.0, 0.0);
+      }
     }
-    double2 r[ELL + 1];
 #pragma unroll
-    for (int i = 0; i <= ELL; ++i) r[i] = V.r[i][e];
+    for (int q = 0; q < U; ++q)
 #pragma unroll
-    for (int k = 1; k <= ELL; ++k) {
+      for (int k = 1; k <= ELL; ++k) {
 #pragma unroll
-      for (int i = 1; i <= k; ++i) acc[gram_index(i, k)] += cdot_re(r[i], r[k]);
-      acc[NG + k - 1] += cdot_re(r[0], r[k]);
-    }
+        for (int i = 1; i <= k; ++i) acc[gram_index(i, k)] += cdot_re(r[q][i], r[q][k]);
+        acc[NG + k - 1] += cdot_re(r[q][0], r[q][k]);
+      }
   }
   if (grid_sum<ND>(acc, tot, sc->partials, &sc->counter) && threadIdx.x == 0) {
     double G[ELL][ELL], c[ELL];
@@ -326,20 +414,26 @@ __global__ void gram_kernel(BicgVectors V, long long n, BicgScalars *sc) {
   }
 }
 
-// x += sum_j gamma_j r_{j-1}; r_0 -= sum_j gamma_j r_j; u_0 -= sum_j gamma_j u_j;
+// x += alpha u_0 (the last BiCG step) + sum_j gamma_j r_{j-1};
+// r_0 -= sum_j gamma_j r_j; u_0 -= sum_j gamma_j u_j;
 // then rr = <r_0, r_0>, the stopping test, and the first BiCG step of the
 // next outer iteration (rho0 = -omega rho0; rho1 = <rhat, r_0>;
 // beta = alpha rho1 / rho0; rho0 = rho1).
 template <int ELL>
 __global__ void mr_update_kernel(BicgVectors V, long long n, BicgScalars *sc) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (solve_done(sc)) return;
   double g[ELL + 1];
 #pragma unroll
   for (int j = 1; j <= ELL; ++j) g[j] = sc->gamma[j];
   const bool restart = sc->restart;
+  const double alpha = sc->alpha;
   double acc[2] = {0.0, 0.0}, tot[2];
   GRID_LOOP(e, n) {
     double2 x = V.x[e], r0 = V.r[0][e], u0 = V.u[0][e];
+    x.x += alpha * u0.x;
+    x.y += alpha * u0.y;
 #pragma unroll
     for (int j = 1; j <= ELL; ++j) {
       const double2 rp = V.r[j - 1][e], rj = V.r[j][e], uj = V.u[j][e];
@@ -421,13 +515,11 @@ __global__ void guess_clear_kernel(double2 *x) { x[0] = make_double2(0.0, 0.0); 
 
 template <int ELL>
 cudaError_t launch_gram_t(const BicgVectors &V, long long n, BicgScalars *sc, int grid, cudaStream_t s) {
-  gram_kernel<ELL><<<grid, kBlock, 0, s>>>(V, n, sc);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), gram_kernel<ELL>, dim3(grid), dim3(kBlock), 0, s, V, n, sc);
 }
 template <int ELL>
 cudaError_t launch_mr_t(const BicgVectors &V, long long n, BicgScalars *sc, int grid, cudaStream_t s) {
-  mr_update_kernel<ELL><<<grid, kBlock, 0, s>>>(V, n, sc);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), mr_update_kernel<ELL>, dim3(grid), dim3(kBlock), 0, s, V, n, sc);
 }
 
 }  // namespace
@@ -448,27 +540,22 @@ cudaError_t bicg_launch_init(const BicgVectors &V, long long n, BicgScalars *sc,
   return cudaGetLastError();
 }
 cudaError_t bicg_launch_rho(const BicgVectors &V, long long n, BicgScalars *sc, int j, int grid, cudaStream_t s) {
-  rho_kernel<<<grid, kBlock, 0, s>>>(V, n, sc, j);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), rho_kernel, dim3(grid), dim3(kBlock), 0, s, V, n, sc, j);
 }
 cudaError_t bicg_launch_dot_finish(const double *parts, long long nparts, BicgScalars *sc, int which,
-                                   cudaStream_t s) {
-  dot_finish_kernel<<<1, kBlock, 0, s>>>(parts, nparts, sc, which);
-  return cudaGetLastError();
+                                   bool dependent, cudaStream_t s) {
+  return launch_dependent(dependent, dot_finish_kernel, dim3(1), dim3(kBlock), 0, s, parts, nparts, sc, which);
 }
 cudaError_t bicg_launch_u_update(const BicgVectors &V, long long n, const BicgScalars *sc, int j, int grid,
                                  cudaStream_t s) {
-  u_update_kernel<<<grid, kBlock, 0, s>>>(V, n, sc, j);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), u_update_kernel, dim3(grid), dim3(kBlock), 0, s, V, n, sc, j);
 }
 cudaError_t bicg_launch_gamma(const BicgVectors &V, long long n, BicgScalars *sc, int j, int grid, cudaStream_t s) {
-  gamma_kernel<<<grid, kBlock, 0, s>>>(V, n, sc, j);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), gamma_kernel, dim3(grid), dim3(kBlock), 0, s, V, n, sc, j);
 }
 cudaError_t bicg_launch_r_update(const BicgVectors &V, long long n, const BicgScalars *sc, int j, int grid,
                                  cudaStream_t s) {
-  r_update_kernel<<<grid, kBlock, 0, s>>>(V, n, sc, j);
-  return cudaGetLastError();
+  return launch_dependent(bicg_dependent(n), r_update_kernel, dim3(grid), dim3(kBlock), 0, s, V, n, sc, j);
 }
 cudaError_t bicg_launch_gram(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid, cudaStream_t s) {
   switch (ell) {

@@ -67,6 +67,11 @@ __device__ inline void bicg_dot_step(BicgScalars *sc, double tot, int which) {
 #endif
 
 int bicg_grid(int num_sms);
+// Whether the solver's kernels on vectors of n elements are launched as
+// dependents of one another: yes where they are short (a BiCG step of 70 to
+// 3,003 nodes takes 40 -> 36 us), not where they run at memory bandwidth
+// (125,970 nodes of 4x4: 201 us, 218 as dependents).
+constexpr bool bicg_dependent(long long n) { return n <= (1ll << 18); }
 // b = -b with element (0,0) of node 0 zeroed (b holds L(E00) on entry).
 cudaError_t bicg_launch_rhs(double2 *b, long long n, int grid, cudaStream_t s);
 // x /= x[0] (the guess scaled to x_0[0,0] = 1), then x[0] = 0.
@@ -81,11 +86,11 @@ cudaError_t bicg_launch_gamma(const BicgVectors &V, long long n, BicgScalars *sc
 cudaError_t bicg_launch_r_update(const BicgVectors &V, long long n, const BicgScalars *sc, int j, int grid,
                                  cudaStream_t s);
 // The same two inner products when the apply that produced the vector
-// already summed <rhat, .> per tile (the tiled kernel, dot_part of a stage
+// already summed <rhat, .> per CTA (the tiled kernel, dot_part of a stage
 // launch): one block adds the nparts partials in order and runs the scalar
 // step of rho (which = 0) or gamma (which = 1).
 cudaError_t bicg_launch_dot_finish(const double *parts, long long nparts, BicgScalars *sc, int which,
-                                   cudaStream_t s);
+                                   bool dependent, cudaStream_t s);
 // Minimal-residual step over r_1..r_ell and the end-of-iteration control.
 cudaError_t bicg_launch_gram(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid, cudaStream_t s);
 cudaError_t bicg_launch_mr_update(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid,

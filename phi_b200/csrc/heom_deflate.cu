@@ -16,8 +16,10 @@
 // so the stopping test is unchanged (Nicolaides, SIAM J. Numer. Anal. 24,
 // 1987; the DEF1 form of Tang, Nabben, Vuik and Erlangga, J. Sci. Comput. 39,
 // 2009).  Z is a set of unit vectors, so Z^T v is a gather of k coordinates
-// and A Z is supported on the nodes of tiers 0..tiers: a projection is one
-// small solve with E and one rows x k product, both L2-resident.  A Z is
+// and A Z is supported on the nodes of tiers 0..tiers: with W = A Z E^-1 formed
+// once per solve, a projection is that gather and one rows x k product,
+// L2-resident (the solve with E's factors in one CTA took 15 us of every
+// operator product on the 4-site chain; the gather takes 5).  A Z is
 // built once per solve by one batched launch of the generic Liouvillian
 // kernel over those nodes (k unit inputs).  First-tier nodes are not
 // neighbours of one another, so E = [[A00, A01], [A10, D]] with D block
@@ -34,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include "heom_bicgstab.h"
+#include "heom_device.cuh"
 #include "heom_deflate.h"
 
 namespace phi {
@@ -44,8 +47,6 @@ constexpr int kSolveBlock = 1024;
 // Matrices of the factorisation up to this many doubles are inverted in
 // shared memory, larger ones in the global work buffer (L2).
 constexpr int kSmemDoubles = 16384;
-// The projection's factors are staged in shared memory up to this size.
-constexpr int kStageDoubles = 24576;
 
 __device__ __forceinline__ double cdot_re(double2 a, double2 b) { return a.x * b.x + a.y * b.y; }
 
@@ -98,15 +99,6 @@ __global__ void units_kernel(DeflView D) {
     *ab = make_double2(0.0, 1.0);
     *ba = make_double2(0.0, -1.0);
   }
-}
-
-// AZr = A Z row-major, element (0,0) of node 0 (row 0) zeroed.
-__global__ void transpose_kernel(DeflView D) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= D.rows * D.k) return;
-  const long long r = idx / D.k;
-  const int j = (int)(idx - r * D.k);
-  D.AZr[idx] = r == 0 ? make_double2(0.0, 0.0) : D.AZ[(long long)j * D.rows + r];
 }
 
 // In-place inverse of the n x n row-major matrix A (shared or global
@@ -311,34 +303,92 @@ __global__ void __launch_bounds__(kSolveBlock) factor_kernel(DeflView D) {
   if (tid == 0) *D.status = 0;
 }
 
-// g_j = <rhat, A Z_j>: one warp per column, lanes in row order.
-__global__ void g_kernel(DeflView D, const double2 *rhat) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= D.k) return;
-  const double2 *col = D.AZ + (long long)warp * D.rows;
+// W = A Z E^-1, row-major, row 0 (element (0,0) of node 0, whose equation is
+// dropped) zero: with it a projection is v -= W Z^T v, without a solve.  One
+// CTA per row a = (a0, a1) of A Z: t = (a0 - a1 F) S^-1, W = (t,
+// (a1 - t A01) D^-1).
+__global__ void w_kernel(DeflView D) {
+  __shared__ double2 a[kMaxDeflK], t0[kMaxDeflK], t[kMaxDeflK];
+  const long long r = blockIdx.x;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int E = D.E, k0 = D.k0, n1 = D.n1, k = D.k;
+  double2 *out = D.W + r * k;
+  if (r == 0) {
+    for (int j = tid; j < k; j += nt) out[j] = make_double2(0.0, 0.0);
+    return;
+  }
+  for (int j = tid; j < k; j += nt) a[j] = D.AZ[(long long)j * D.rows + r];
+  __syncthreads();
+  for (int q = warp; q < k0; q += nw) {
+    double2 s = make_double2(0.0, 0.0);
+    for (int i = lane; i < n1; i += 32) {
+      const double f = D.F[(long long)i * k0 + q];
+      s.x = fma(a[k0 + i].x, f, s.x);
+      s.y = fma(a[k0 + i].y, f, s.y);
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, off);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, off);
+    }
+    if (lane == 0) t0[q] = make_double2(a[q].x - s.x, a[q].y - s.y);
+  }
+  __syncthreads();
+  for (int q = tid; q < k0; q += nt) {
+    double2 s = make_double2(0.0, 0.0);
+    for (int p = 0; p < k0; ++p) {
+      const double f = D.Si[(long long)p * k0 + q];
+      s.x = fma(t0[p].x, f, s.x);
+      s.y = fma(t0[p].y, f, s.y);
+    }
+    t[q] = s;
+    out[q] = s;
+  }
+  __syncthreads();
+  for (int i = tid; i < n1; i += nt) {
+    double2 s = a[k0 + i];
+    for (int q = 0; q < k0; ++q) {
+      const double f = D.A01[(long long)q * n1 + i];
+      s.x = fma(-t[q].x, f, s.x);
+      s.y = fma(-t[q].y, f, s.y);
+    }
+    a[k0 + i] = s;
+  }
+  __syncthreads();
+  for (int i = tid; i < n1; i += nt) {
+    const int o = i / E * E, l = i - o;
+    double2 s = make_double2(0.0, 0.0);
+    for (int p = 0; p < E; ++p) {
+      const double f = D.Dinv[(long long)(o + p) * E + l];
+      s.x = fma(a[k0 + o + p].x, f, s.x);
+      s.y = fma(a[k0 + o + p].y, f, s.y);
+    }
+    out[k0 + i] = s;
+  }
+}
+
+// g_j = <rhat, W_j>: one thread per column (a warp reads along the rows), the
+// rows split over the CTA's warps' groups and added in order.
+constexpr int kGroups = 16;
+__global__ void __launch_bounds__(32 * kGroups) g_kernel(DeflView D, const double2 *rhat) {
+  __shared__ double part[kGroups][32];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (long long r = lane; r < D.rows; r += 32) s += cdot_re(rhat[r], col[r]);
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) D.g[warp] = s;
+  if (j < D.k)
+    for (long long r = grp; r < D.rows; r += kGroups) s += cdot_re(rhat[r], D.W[r * D.k + j]);
+  part[grp][lane] = s;
+  __syncthreads();
+  if (grp != 0 || j >= D.k) return;
+  s = 0.0;
+  for (int q = 0; q < kGroups; ++q) s += part[q][lane];
+  D.g[j] = s;
 }
 
 // c = E^-1 Z^T (v - b) through the factors: w = D^-1 z1,
-// c0 = S^-1 (z0 - A01 w), c1 = w - F c0; *part = -<g, c>.  One CTA.
-// The factors (Dinv, F, A01, Si: one contiguous run of doubles) are first
-// copied into shared memory when they fit (stage = true).
-__device__ __forceinline__ void coeff_body(DeflView D, const double2 *v, const double2 *b, double *part,
-                                           bool stage, double *fac_s) {
+// c0 = S^-1 (z0 - A01 w), c1 = w - F c0.  One CTA (the final correction).
+__global__ void __launch_bounds__(kSolveBlock) coeff_kernel(DeflView D, const double2 *v, const double2 *b) {
   __shared__ double z[kMaxDeflK], w[kMaxDeflK], cs[kMaxDeflK];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   const int E = D.E, k0 = D.k0, n1 = D.n1, k = D.k;
-  if (stage) {
-    const long long total = (long long)n1 * E + 2ll * n1 * k0 + (long long)k0 * k0;
-    for (long long i = tid; i < total; i += nt) fac_s[i] = D.Dinv[i];
-    D.Dinv = fac_s;
-    D.F = D.Dinv + (long long)n1 * E;
-    D.A01 = D.F + (long long)n1 * k0;
-    D.Si = D.A01 + (long long)k0 * n1;
-  }
   for (int p = tid; p < k; p += nt) {
     const Coord c = coord_of(p + 1, D.N);
     z[p] = zcoord(v, c, D.N) - (b ? zcoord(b, c, D.N) : 0.0);
@@ -376,57 +426,63 @@ __device__ __forceinline__ void coeff_body(DeflView D, const double2 *v, const d
   }
   __syncthreads();
   for (int j = tid; j < k; j += nt) D.c[j] = cs[j];
-  if (part && warp == 0) {
-    double s = 0.0;
-    for (int j = lane; j < k; j += 32) s = fma(D.g[j], cs[j], s);
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) *part = -s;
+}
+
+// z = Z^T (v - b) for the projection's update; with part != NULL also
+// *part = -<g, z>, the change of <rhat, v> that the update makes, and the BiCG
+// scalar step of the inner product whose per-CTA partials the apply left in
+// parts[0 .. nparts - 1] (*part is the last of them), summed in order.
+constexpr int kCoordBlock = 512;
+__global__ void __launch_bounds__(kCoordBlock) coords_kernel(DeflView D, const double2 *v, const double2 *b,
+                                                           double *part, const double *parts, long long nparts,
+                                                           BicgScalars *sc, int which) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ double red[2][kCoordBlock / 32];
+  if (D.done && *(volatile const int *)D.done) return;  // uniform: the solve has stopped
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double s = 0.0, d = 0.0;
+  if (tid < D.k) {
+    const Coord c = coord_of(tid + 1, D.N);
+    const double z = zcoord(v, c, D.N) - (b ? zcoord(b, c, D.N) : 0.0);
+    D.z[tid] = z;
+    if (part) d = -D.g[tid] * z;
   }
-}
-
-__global__ void __launch_bounds__(kSolveBlock) coeff_kernel(DeflView D, const double2 *v, const double2 *b,
-                                                          double *part, bool stage) {
-  extern __shared__ double fac_s[];
-  if (D.done && *(volatile const int *)D.done) return;  // uniform: the solve has stopped
-  coeff_body(D, v, b, part, stage, fac_s);
-}
-
-// The coefficients of v's projection, then the BiCG scalar step of the
-// inner product whose per-tile partials the apply left in parts[0..nparts-1]
-// (the projection's change is parts[nparts-1] = *part): one launch instead
-// of a coefficient kernel and a one-block finish.  Summed in part order.
-__global__ void __launch_bounds__(kSolveBlock) coeff_finish_kernel(DeflView D, const double2 *v, double *part,
-                                                                 const double *parts, long long nparts,
-                                                                 BicgScalars *sc, int which, bool stage) {
-  extern __shared__ double fac_s[];
-  __shared__ double red[kSolveBlock / 32];
-  if (D.done && *(volatile const int *)D.done) return;  // uniform: the solve has stopped
-  coeff_body(D, v, nullptr, part, stage, fac_s);
-  __syncthreads();  // *part is visible to the whole CTA
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double s = 0.0;
-  for (long long i = threadIdx.x; i < nparts; i += blockDim.x) s += parts[i];
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) red[warp] = s;
+  if (!part) return;
+  for (long long i = tid; i < nparts - 1; i += kCoordBlock) s += parts[i];
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, off);
+    d += __shfl_xor_sync(0xffffffffu, d, off);
+  }
+  if (lane == 0) {
+    red[0][warp] = s;
+    red[1][warp] = d;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red[i];
-    bicg_dot_step(sc, tot, which);
+  if (tid == 0) {
+    s = d = 0.0;
+    for (int w = 0; w < kCoordBlock / 32; ++w) {
+      s += red[0][w];
+      d += red[1][w];
+    }
+    *part = d;
+    bicg_dot_step(sc, s + d, which);
   }
 }
 
-// v[r] -= sum_j A Z[r, j] c_j for the rows of tiers 0..tiers: one warp per
-// row of the row-major copy, lanes over j.
+// v[r] -= sum_j W[r, j] z_j for the rows of tiers 0..tiers: one warp per row,
+// lanes over j.
 __global__ void update_kernel(DeflView D, double2 *v) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ double cs[kMaxDeflK];
   if (D.done && *(volatile const int *)D.done) return;
-  for (int j = threadIdx.x; j < D.k; j += blockDim.x) cs[j] = D.c[j];
+  for (int j = threadIdx.x; j < D.k; j += blockDim.x) cs[j] = D.z[j];
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= D.rows) return;
-  const double2 *row = D.AZr + r * D.k;
+  const double2 *row = D.W + r * D.k;
   double sx = 0.0, sy = 0.0;
   for (int j = lane; j < D.k; j += 32) {
     const double2 a = row[j];
@@ -472,59 +528,41 @@ cudaError_t defl_launch_units(const DeflView &D, cudaStream_t st) {
 
 cudaError_t defl_launch_factor(const DeflView &D, cudaStream_t st) {
   if (D.k < 1 || D.k > kMaxDeflK || D.k0 + D.n1 != D.k || (D.n1 && D.n1 % D.E)) return cudaErrorInvalidValue;
-  const long long total = D.rows * D.k;
-  transpose_kernel<<<(unsigned)((total + kBlock - 1) / kBlock), kBlock, 0, st>>>(D);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   const int big = D.E > D.k0 ? D.E : D.k0;
   const int t1 = D.n1 / D.E, regions = t1 < kSolveBlock / 32 ? t1 : kSolveBlock / 32;
   long long need = (long long)big * big;
   if (D.E <= 32 && (long long)regions * D.E * D.E <= kSmemDoubles && (long long)regions * D.E * D.E > need)
     need = (long long)regions * D.E * D.E;  // one region per warp for the first-tier blocks
   const size_t smem = (size_t)(need < kSmemDoubles ? need : kSmemDoubles) * sizeof(double);
-  e = cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   factor_kernel<<<1, kSolveBlock, smem, st>>>(D);
+  w_kernel<<<(unsigned)D.rows, kBlock, 0, st>>>(D);
   return cudaGetLastError();
 }
 
 cudaError_t defl_launch_g(const DeflView &D, const double2 *rhat, cudaStream_t st) {
-  const int warps_per_block = kBlock / 32;
-  g_kernel<<<(D.k + warps_per_block - 1) / warps_per_block, kBlock, 0, st>>>(D, rhat);
+  g_kernel<<<(D.k + 31) / 32, 32 * kGroups, 0, st>>>(D, rhat);
   return cudaGetLastError();
 }
 
-cudaError_t defl_launch_coeff(const DeflView &D, const double2 *v, const double2 *b, double *part, cudaStream_t st) {
-  const long long total = (long long)D.n1 * D.E + 2ll * D.n1 * D.k0 + (long long)D.k0 * D.k0;
-  const bool stage = total <= kStageDoubles;
-  const size_t smem = stage ? (size_t)total * sizeof(double) : 0;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(coeff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kStageDoubles * sizeof(double)));
-    if (e != cudaSuccess) return e;
-  }
-  coeff_kernel<<<1, kSolveBlock, smem, st>>>(D, v, b, part, stage);
+cudaError_t defl_launch_coeff(const DeflView &D, const double2 *v, const double2 *b, cudaStream_t st) {
+  coeff_kernel<<<1, kSolveBlock, 0, st>>>(D, v, b);
   return cudaGetLastError();
 }
 
-cudaError_t defl_launch_coeff_finish(const DeflView &D, const double2 *v, double *part, const double *parts,
-                                     long long nparts, BicgScalars *sc, int which, cudaStream_t st) {
-  const long long total = (long long)D.n1 * D.E + 2ll * D.n1 * D.k0 + (long long)D.k0 * D.k0;
-  const bool stage = total <= kStageDoubles;
-  const size_t smem = stage ? (size_t)total * sizeof(double) : 0;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(coeff_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kStageDoubles * sizeof(double)));
-    if (e != cudaSuccess) return e;
-  }
-  coeff_finish_kernel<<<1, kSolveBlock, smem, st>>>(D, v, part, parts, nparts, sc, which, stage);
-  return cudaGetLastError();
+cudaError_t defl_launch_coords(const DeflView &D, const double2 *v, const double2 *b, cudaStream_t st) {
+  return launch_dependent(D.dependent, coords_kernel, dim3(1), dim3(kCoordBlock), 0, st, D, v, b, nullptr, nullptr, 0, nullptr, 0);
+}
+
+cudaError_t defl_launch_coords_finish(const DeflView &D, const double2 *v, double *part, const double *parts,
+                                      long long nparts, BicgScalars *sc, int which, cudaStream_t st) {
+  return launch_dependent(D.dependent, coords_kernel, dim3(1), dim3(kCoordBlock), 0, st, D, v, nullptr, part, parts, nparts, sc, which);
 }
 
 cudaError_t defl_launch_update(const DeflView &D, double2 *v, cudaStream_t st) {
   const int rows_per_block = kBlock / 32;
-  update_kernel<<<(unsigned)((D.rows + rows_per_block - 1) / rows_per_block), kBlock, 0, st>>>(D, v);
-  return cudaGetLastError();
+  return launch_dependent(D.dependent, update_kernel, dim3((unsigned)((D.rows + rows_per_block - 1) / rows_per_block)), dim3(kBlock), 0, st, D, v);
 }
 
 cudaError_t defl_launch_correct(const DeflView &D, double2 *x, cudaStream_t st) {

@@ -49,10 +49,10 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches kern(args...) with that attribute.
+// Launches kern(args...) with that attribute (or, dependent false, without).
 template <class Kernel, class... Args>
-inline cudaError_t launch_dependent(Kernel kern, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    const Args &...args) {
+inline cudaError_t launch_dependent(bool dependent, Kernel kern, dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t stream, const Args &...args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -62,7 +62,7 @@ inline cudaError_t launch_dependent(Kernel kern, dim3 grid, dim3 block, size_t s
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 

@@ -650,7 +650,7 @@ cudaError_t launch_node(const StageParams &p, int batch, cudaStream_t stream) {
   static thread_local int configured[kSmemLimitDevices] = {};
   cudaError_t e = raise_smem_limit(kern, p.plan.bytes, configured);
   if (e != cudaSuccess) return e;
-  return launch_dependent(kern, dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch), dim3(p.plan.threads),
+  return launch_dependent(true, kern, dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch), dim3(p.plan.threads),
                           p.plan.bytes, stream, p);
 }
 

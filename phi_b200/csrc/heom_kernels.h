@@ -31,10 +31,12 @@ struct StageLaunch {
   uint8_t *act[2] = {nullptr, nullptr};
   int act_par = 0;
   // FP64 apply of the steady-state solver (tiled kernel): element (0,0) of
-  // node 0 of the output is zeroed and each tile writes its share of
-  // <dot_w, out> to dot_part[tile].
+  // node 0 of the output is zeroed and each CTA writes its share of
+  // <dot_w, out> to dot_part[CTA]; the dot_slots entries past the grid are
+  // zeroed.
   const double2 *dot_w = nullptr;
   double *dot_part = nullptr;
+  int dot_slots = 0;
   // The generic kernel even where the tiled one applies (with c.M lowered,
   // the rows of the first c.M nodes only; neighbour ids index the whole x).
   bool generic = false;

@@ -67,6 +67,7 @@ TileParams tile_params_for(const StageLaunch &L) {
   p.act_par = L.act_par;
   p.dot_w = (L.mode == kModeApply && !L.mixed) ? L.dot_w : nullptr;
   p.dot_part = p.dot_w ? L.dot_part : nullptr;
+  p.dot_slots = p.dot_w ? L.dot_slots : 0;
   const bool mixed = L.mixed;
   const int xb = mixed ? 8 : 16;
   // Epilogue operands of this (mode, stage), in the order the epilogue reads them.
@@ -75,6 +76,10 @@ TileParams tile_params_for(const StageLaunch &L) {
   for (int b = 0; b < kMaxPre; ++b) {
     p.pre[b] = nullptr;
     p.pre_bytes[b] = 16;
+  }
+  if (p.dot_w) {
+    p.pre[0] = p.dot_w;
+    p.npre = 1;
   }
   if (L.mode == kModeRk4) {
     if (L.stage == 0 && mixed) {
@@ -187,19 +192,17 @@ cudaError_t tile_autotune(const StageLaunch &L0, cudaStream_t stream, TileSchedu
 
 namespace {
 template <int N, int KT>
-long long tiles_of_k(long long M, bool mixed, bool batch) {
-  const long long nt =
-      batch ? (mixed ? TileShape<N, true, KT, kTileThreads, kTileBatch>::NT
-                     : TileShape<N, false, KT, kTileThreads, kTileBatch>::NT)
-            : (mixed ? TileShape<N, true, KT>::NT : TileShape<N, false, KT>::NT);
+long long tiles_of_k(long long M, bool mixed) {
+  const long long nt = mixed ? TileShape<N, true, KT, kTileThreads, kTileBatch>::NT
+                             : TileShape<N, false, KT, kTileThreads, kTileBatch>::NT;
   return (M + nt - 1) / nt;
 }
 template <int N>
-long long tiles_of(long long M, bool mixed, int K1, bool batch) {
+long long tiles_of(long long M, bool mixed, int K1) {
   switch (K1) {
-    case 1: return tiles_of_k<N, 1>(M, mixed, batch);
-    case 2: return tiles_of_k<N, 2>(M, mixed, batch);
-    case 3: return tiles_of_k<N, 3>(M, mixed, batch);
+    case 1: return tiles_of_k<N, 1>(M, mixed);
+    case 2: return tiles_of_k<N, 2>(M, mixed);
+    case 3: return tiles_of_k<N, 3>(M, mixed);
     default: return -1;
   }
 }
@@ -214,19 +217,19 @@ size_t stage_smem_n(const TileParams &p, bool mixed) {
 }
 }  // namespace
 
-long long tile_count(const HeomConsts &c, bool mixed, bool batch) {
+long long tile_count(const HeomConsts &c, bool mixed) {
   switch (c.N) {
-    case 2: return tiles_of<2>(c.M, mixed, c.K1, batch);
-    case 3: return tiles_of<3>(c.M, mixed, c.K1, batch);
-    case 4: return tiles_of<4>(c.M, mixed, c.K1, batch);
-    case 5: return tiles_of<5>(c.M, mixed, c.K1, batch);
-    case 6: return tiles_of<6>(c.M, mixed, c.K1, batch);
-    case 7: return tiles_of<7>(c.M, mixed, c.K1, batch);
-    case 8: return tiles_of<8>(c.M, mixed, c.K1, batch);
-    case 10: return tiles_of<10>(c.M, mixed, c.K1, batch);
-    case 12: return tiles_of<12>(c.M, mixed, c.K1, batch);
-    case 16: return tiles_of<16>(c.M, mixed, c.K1, batch);
-    case 24: return tiles_of<24>(c.M, mixed, c.K1, batch);
+    case 2: return tiles_of<2>(c.M, mixed, c.K1);
+    case 3: return tiles_of<3>(c.M, mixed, c.K1);
+    case 4: return tiles_of<4>(c.M, mixed, c.K1);
+    case 5: return tiles_of<5>(c.M, mixed, c.K1);
+    case 6: return tiles_of<6>(c.M, mixed, c.K1);
+    case 7: return tiles_of<7>(c.M, mixed, c.K1);
+    case 8: return tiles_of<8>(c.M, mixed, c.K1);
+    case 10: return tiles_of<10>(c.M, mixed, c.K1);
+    case 12: return tiles_of<12>(c.M, mixed, c.K1);
+    case 16: return tiles_of<16>(c.M, mixed, c.K1);
+    case 24: return tiles_of<24>(c.M, mixed, c.K1);
     default: return -1;
   }
 }

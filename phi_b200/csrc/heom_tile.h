@@ -29,9 +29,8 @@ int tile_block_threads(const HeomConsts &c, bool mixed, int variant);
 cudaError_t tile_autotune(const StageLaunch &L, cudaStream_t stream, TileSchedule *out);
 
 // ---- batched stages over many hierarchies (heom_tile_batch.cu) ----
-// Tiles of one hierarchy in the given arithmetic (-1 when N has no tile
-// kernel), of the single-instance apply (default block) or in a batch.
-long long tile_count(const HeomConsts &c, bool mixed, bool batch);
+// Tiles of one hierarchy in the given arithmetic (-1 when N has no tile kernel).
+long long tile_count(const HeomConsts &c, bool mixed);
 // Dynamic shared memory of one tile of stage launch L.
 size_t tile_stage_smem(const StageLaunch &L);
 // Size and host image of the per-instance tile parameters of stage launch L.

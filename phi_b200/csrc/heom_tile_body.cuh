@@ -86,8 +86,9 @@ struct TileParams {
   Rkf45Ctl *ctl;
   uint8_t *act[2];               // filtering: active flags (see StageLaunch)
   int act_par;
-  const double2 *dot_w;          // FP64 apply: <dot_w, out> per tile (see StageLaunch)
+  const double2 *dot_w;          // FP64 apply: <dot_w, out> per CTA (see StageLaunch)
   double *dot_part;
+  int dot_slots;
   int dependent;                 // launched as a dependent of the previous kernel
   int npre;                      // epilogue operands prefetched
   const void *pre[kMaxPre];      // sources; slot 0 of RKF45 is chosen on the device
@@ -621,13 +622,12 @@ __host__ __device__ __forceinline__ uint32_t tile_pre_off(const TileParams &p, i
 // Phase 3: the epilogue of this thread's elements (plain store, RK4 or RKF45
 // stage combine) from its derivatives dx and the prefetched operands at
 // Pre; the RKF45 stage-5 error is folded into emax (max of |y4 - y5|, or of
-// its square in mixed precision).  coef holds the 24 RKF45 coefficients in
+// its square in mixed precision), an apply's inner product added to it.  coef holds the 24 RKF45 coefficients in
 // FP64 followed by the same 24 in FP32.
 template <int N, int KT, bool MIXED, int BT, int ST>
 __device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap<N, KT, MIXED, BT, ST> &m,
                                               const TileIn<N, KT, MIXED, BT, ST> &in, const unsigned char *Pre,
-                                              const double *coef, unsigned long long *wmax, long long tile,
-                                              long long n0, int ycur, double &emax,
+                                              const double *coef, long long n0, int ycur, double &emax,
                                               const typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, ST>::RR]) {
   using S = TileShape<N, MIXED, KT, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
@@ -659,28 +659,19 @@ __device__ __forceinline__ void tile_epilogue(const TileParams &p, const TileMap
         if (m.on(r, in.nt_here)) st_stream(out + m.xo[r], dx[r]);
     } else if constexpr (!MIXED) {
       // Steady-state solve: the output's element (0,0) of node 0 is the
-      // eliminated unknown (zero), and the tile's share of <dot_w, out> (the
-      // real inner product of Hermitian states) goes to dot_part[tile] --
-      // the inner product the solver would otherwise read the vector for.
-      double dsum = 0.0;
+      // eliminated unknown (zero), and this thread's share of <dot_w, out>
+      // (the real inner product of Hermitian states; pre = {dot_w}) is added
+      // up over the CTA's tiles -- the inner product the solver would
+      // otherwise read the vector for.
 #pragma unroll
       for (int r = 0; r < RR; ++r)
         if (m.on(r, in.nt_here)) {
           TX v = dx[r];
           if (gx0 + m.xo[r] == 0) v = mk<TX>(0.0, 0.0);
           st_stream(out + m.xo[r], v);
-          const double2 w = __ldcg(p.dot_w + gx0 + m.xo[r]);
-          dsum = fma(w.x, v.x, fma(w.y, v.y, dsum));
+          const double2 w = pre0d[m.xo[r]];
+          emax = fma(w.x, v.x, fma(w.y, v.y, emax));
         }
-      for (int off = 16; off > 0; off >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
-      double *wsum = reinterpret_cast<double *>(wmax);
-      if ((tid & 31) == 0) wsum[tid >> 5] = dsum;
-      __syncthreads();
-      if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < BT / 32; ++w) t += wsum[w];
-        p.dot_part[tile] = t;
-      }
     }
   } else if (!RKF) {  // RK4
     const int s = p.stage;
@@ -831,6 +822,24 @@ __device__ __forceinline__ void tile_error_max(const TileParams &p, double emax,
     }
 }
 
+// An apply's inner product: the sum over the CTA's threads into its slot, in
+// warp order; CTA 0 zeroes the slots past the grid.
+template <int BT>
+__device__ __forceinline__ void tile_dot_sum(const TileParams &p, double dsum, unsigned long long *wmax) {
+  const int tid = threadIdx.x;
+  for (int off = 16; off > 0; off >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
+  double *wsum = reinterpret_cast<double *>(wmax);
+  if ((tid & 31) == 0) wsum[tid >> 5] = dsum;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < BT / 32; ++w) t += wsum[w];
+    p.dot_part[blockIdx.x] = t;
+  }
+  if (blockIdx.x == 0)
+    for (int q = (int)gridDim.x + tid; q < p.dot_slots; q += BT) p.dot_part[q] = 0.0;
+}
+
 // New filter flags of a tile's nodes after the stage that writes the new
 // state (RK4 stage 3, RKF45 stage 5).
 template <int N, int KT, bool MIXED, int BT, int ST>
@@ -876,8 +885,7 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
   const size_t tail = Lay::kPre + (p.npre > 0 ? tile_pre_off<N, KT, MIXED, BT, ST>(p, p.npre) : 0);
   TX *Hs = reinterpret_cast<TX *>(smem_raw + tail);                 // E
   double *deph = reinterpret_cast<double *>(Hs + E + (E & 1));       // NT (16-aligned)
-  unsigned long long *wmax = reinterpret_cast<unsigned long long *>(deph + NT + (NT & 1));  // per-warp sums
-  typename In::C *cfs = reinterpret_cast<typename In::C *>(wmax + tile_warp_slots(BT));  // NT*T neighbour coefficients
+  typename In::C *cfs = reinterpret_cast<typename In::C *>(deph + NT + (NT & 1));  // NT*T neighbour coefficients
   R *mats = reinterpret_cast<R *>(cfs + NT * T);                    // E    Matsubara factor per element
   int2 *ids = reinterpret_cast<int2 *>(mats + E + (E & 1));         // NT*T element offsets (next, prev)
 
@@ -958,7 +966,7 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
     return -1;
   }
   double emax = 0.0;
-  tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, nullptr, wmax, tile, n0, 0, emax, dx);
+  tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, nullptr, n0, 0, emax, dx);
   tile_flags<N, KT, MIXED, BT, ST>(p, Us, n0, nt_here, 0);
   return 0;
 }
@@ -971,7 +979,7 @@ inline size_t tile_smem(int T, int npre, const int *pre_bytes) {
   size_t b = Lay::kPre;
   for (int i = 0; i < npre; ++i) b += tile_pre_size<N, KT, MIXED, BT, ST>(pre_bytes[i]);
   b += (size_t)(S::E + (S::E & 1)) * Lay::XB;
-  b += (size_t)(S::NT + (S::NT & 1) + tile_warp_slots(BT)) * sizeof(double);  // deph, warp sums
+  b += (size_t)(S::NT + (S::NT & 1)) * sizeof(double);  // deph
   b += (size_t)S::NT * T * sizeof(typename TileIn<N, KT, MIXED, BT, ST>::C);
   b += (size_t)(S::E + (S::E & 1)) * Lay::XB / 2;                     // mats
   b += (size_t)S::NT * T * sizeof(int2);                              // ids

@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
         break;
       }
     }
-    if (ok) tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, coef, wmax, tile, n0, ycur, emax, dx);
+    if (ok) tile_epilogue<N, KT, MIXED, BT, ST>(p, m, in, PreBase, coef, n0, ycur, emax, dx);
     tile_flags<N, KT, MIXED, BT, ST>(p, Us, n0, nt_here, ycur);
     if (next_issued) {
       const bool got = mbar_wait_bounded(&bars[s ^ 1], (uint32_t)((i + 1) >> 1) & 1u, polls0);
@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     return;
   }
   if (RKF && p.stage == 5) tile_error_max<MIXED, BT>(p, emax, wmax);
+  if (!RKF && !MIXED && p.dot_w) tile_dot_sum<BT>(p, emax, wmax);
 }
 
 // Resident CTAs per SM of a kernel at a dynamic shared-memory size and the
@@ -349,26 +350,21 @@ cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm
     return cudaErrorInvalidDevice;
   if (per_sm) *per_sm = cap / sms;
   if (p.c.tile_cps > 0 && p.c.tile_cps * sms < cap) cap = p.c.tile_cps * sms;
+  if (p.dot_w && p.dot_slots < cap) cap = p.dot_slots;
   const long long grid = tiles < cap ? tiles : cap;
   // Dependent launch (the preamble overlaps the previous kernel) for the
   // apply and where every CTA has one tile: 8-site mixed RK4 stage 6.5 -> 5.5
   // us, 84-node trimer 4.0 -> 3.0 us, 4-site apply 37.2 -> 34.5 us.  Stages
   // of several tiles per CTA gained up to 10 % (24 sites) but lost up to 22 %
   // (7-site mixed RKF45), so they keep the plain launch.
-  if (p.mode == kModeApply || tiles <= cap) {
-    TileParams d = p;
-    d.dependent = 1;
-    return launch_dependent(kern, dim3((unsigned)grid), dim3(BT), smem, stream, d);
-  }
-  kern<<<(unsigned)grid, BT, smem, stream>>>(p);
-  return cudaGetLastError();
+  TileParams d = p;
+  d.dependent = p.mode == kModeApply || tiles <= cap;
+  return launch_dependent(d.dependent, kern, dim3((unsigned)grid), dim3(BT), smem, stream, d);
 }
 
 template <int N, int KT, bool MIXED, int ST>
 cudaError_t launch_tile_nk(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
-  // The steady-state apply writes one partial inner product per tile into
-  // an array sized by tile_count, i.e. by the default block's tiles.
-  if (p.c.tile_variant == 1 && !p.dot_w)
+  if (p.c.tile_variant == 1)
     return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::alt, ST>(p, stream, per_sm);
   return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::threads, ST>(p, stream, per_sm);
 }

@@ -3,6 +3,7 @@
 // propagation path, always in FP64.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <string>
@@ -35,6 +36,7 @@ cudaError_t apply_fp64(phi_ctx *ctx, const double2 *in, double2 *out, cudaStream
   phi::StageLaunch L;
   L.dot_w = dot_w;
   L.dot_part = dot_part;
+  L.dot_slots = (int)ctx->bicg_tiles;
   L.c = ctx->c;
   L.mode = phi::kModeApply;
   L.x = in;
@@ -46,10 +48,9 @@ cudaError_t apply_fp64(phi_ctx *ctx, const double2 *in, double2 *out, cudaStream
   return phi::launch_stage(L, s);
 }
 
-// v = P v after an operator apply (deflated solves): the coefficients, the
-// change of <rhat, v> into the extra partial slot (part, or NULL), the update.
-cudaError_t project(const phi::DeflView *D, double2 *v, double *part, cudaStream_t s) {
-  cudaError_t e = phi::defl_launch_coeff(*D, v, nullptr, part, s);
+// v = P v after an operator apply (deflated solves).
+cudaError_t project(const phi::DeflView *D, double2 *v, cudaStream_t s) {
+  cudaError_t e = phi::defl_launch_coords(*D, v, nullptr, s);
   return e == cudaSuccess ? phi::defl_launch_update(*D, v, s) : e;
 }
 
@@ -60,39 +61,39 @@ cudaError_t outer_iteration(phi_ctx *ctx, const phi::BicgVectors &V, long long n
                             int grid, cudaStream_t s, const phi::DeflView *D) {
   cudaError_t e = cudaSuccess;
   // With the tiled kernel the applies that produce u_{j+1} and r_{j+1} also
-  // zero their element (0,0) of node 0 and sum <rhat, .> per tile, so gamma
+  // zero their element (0,0) of node 0 and sum <rhat, .> per CTA, so gamma
   // and the next rho need only a one-block finish instead of a pass over
   // two state-size vectors each.  Each of the two partial arrays has one
-  // slot more than there are tiles: the projection's change of the sum.
+  // slot more than an apply has CTAs: the projection's change of the sum.
   const bool fused = ctx->bicg_parts.ptr != nullptr;
   const long long tiles = ctx->bicg_tiles;
   const long long nparts = tiles + (D ? 1 : 0);
   double *pu = fused ? ctx->bicg_parts.as<double>() : nullptr;
   double *pr = fused ? pu + tiles + 1 : nullptr;
-  // Deflated and fused, the projection's coefficient kernel also finishes
+  // Deflated and fused, the projection's coordinate kernel also finishes
   // the inner product (rho or gamma) before its update kernel runs.
   const bool fold = fused && D;
   for (int j = 0; j < ell && e == cudaSuccess; ++j) {
     if (j > 0 && !fold)
-      e = fused ? phi::bicg_launch_dot_finish(pr, nparts, sc, 0, s) : phi::bicg_launch_rho(V, n, sc, j, grid, s);
+      e = fused ? phi::bicg_launch_dot_finish(pr, nparts, sc, 0, phi::bicg_dependent(n), s) : phi::bicg_launch_rho(V, n, sc, j, grid, s);
     if (e == cudaSuccess) e = phi::bicg_launch_u_update(V, n, sc, j, grid, s);
     if (e == cudaSuccess) e = apply_fp64(ctx, V.u[j], V.u[j + 1], s, fused ? V.rhat : nullptr, pu);
     if (e == cudaSuccess && fold) {
-      e = phi::defl_launch_coeff_finish(*D, V.u[j + 1], pu + tiles, pu, nparts, sc, 1, s);
+      e = phi::defl_launch_coords_finish(*D, V.u[j + 1], pu + tiles, pu, nparts, sc, 1, s);
       if (e == cudaSuccess) e = phi::defl_launch_update(*D, V.u[j + 1], s);
     } else {
-      if (e == cudaSuccess && D) e = project(D, V.u[j + 1], nullptr, s);
+      if (e == cudaSuccess && D) e = project(D, V.u[j + 1], s);
       if (e == cudaSuccess)
-        e = fused ? phi::bicg_launch_dot_finish(pu, nparts, sc, 1, s) : phi::bicg_launch_gamma(V, n, sc, j, grid, s);
+        e = fused ? phi::bicg_launch_dot_finish(pu, nparts, sc, 1, phi::bicg_dependent(n), s) : phi::bicg_launch_gamma(V, n, sc, j, grid, s);
     }
     if (e == cudaSuccess) e = phi::bicg_launch_r_update(V, n, sc, j, grid, s);
     const bool rho_next = fused && j + 1 < ell;  // the last r_{j+1} goes to the Gram step instead
     if (e == cudaSuccess) e = apply_fp64(ctx, V.r[j], V.r[j + 1], s, rho_next ? V.rhat : nullptr, pr);
     if (e == cudaSuccess && fold && rho_next) {
-      e = phi::defl_launch_coeff_finish(*D, V.r[j + 1], pr + tiles, pr, nparts, sc, 0, s);
+      e = phi::defl_launch_coords_finish(*D, V.r[j + 1], pr + tiles, pr, nparts, sc, 0, s);
       if (e == cudaSuccess) e = phi::defl_launch_update(*D, V.r[j + 1], s);
     } else if (e == cudaSuccess && D) {
-      e = project(D, V.r[j + 1], nullptr, s);
+      e = project(D, V.r[j + 1], s);
     }
   }
   if (e == cudaSuccess) e = phi::bicg_launch_gram(V, n, sc, ell, grid, s);
@@ -230,10 +231,10 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
     }
   }
   if (phi::tile_kernel_available(ctx->c) && !ctx->bicg_parts.ptr) {
-    ctx->bicg_tiles = phi::tile_count(ctx->c, false, false);
-    if (ctx->bicg_tiles > 0 &&
-        ctx->bicg_parts.alloc((size_t)2 * (ctx->bicg_tiles + 1) * sizeof(double)) != cudaSuccess) {
-      ctx->error = "steady_state: allocation of the per-tile partial sums failed";
+    // At most 8 CTAs of 256 threads per SM, and a tile's worth of work each.
+    ctx->bicg_tiles = std::min<long long>(8ll * ctx->num_sms, std::max<long long>(64, n / 128));
+    if (ctx->bicg_parts.alloc((size_t)2 * (ctx->bicg_tiles + 1) * sizeof(double)) != cudaSuccess) {
+      ctx->error = "steady_state: allocation of the per-CTA partial sums failed";
       return PHI_E_OOM;
     }
   }
@@ -245,6 +246,7 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
   phi::DeflView D{};
   if (plan.tiers > 0) {
     D.N = N;
+    D.dependent = phi::bicg_dependent(n);
     D.E = N * N;
     D.k = plan.k;
     D.k0 = D.E - 1;
@@ -252,8 +254,8 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
     D.rows = plan.rows_nodes * D.E;
     D.unit_len = plan.unit_nodes * D.E;
     const int big = D.E > D.k0 ? D.E : D.k0;
-    // doubles: Dinv, F, A01, Si, g, c, work
-    const size_t dbl = (size_t)D.n1 * D.E + 2 * (size_t)D.n1 * D.k0 + (size_t)D.k0 * D.k0 + 2 * (size_t)D.k +
+    // doubles: Dinv, F, A01, Si, g, c, z, work
+    const size_t dbl = (size_t)D.n1 * D.E + 2 * (size_t)D.n1 * D.k0 + (size_t)D.k0 * D.k0 + 3 * (size_t)D.k +
                        (size_t)big * big;
     const size_t az = (size_t)D.rows * D.k * sizeof(double2);
     const size_t units = (size_t)D.k * D.unit_len * sizeof(double2);
@@ -271,7 +273,7 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
     }
     unsigned char *p = ctx->defl_buf.as<unsigned char>();
     D.AZ = reinterpret_cast<double2 *>(p);
-    D.AZr = reinterpret_cast<double2 *>(p + az);
+    D.W = reinterpret_cast<double2 *>(p + az);
     D.units = reinterpret_cast<double2 *>(p + 2 * az);
     double *d = reinterpret_cast<double *>(p + 2 * az + units);
     D.Dinv = d;
@@ -280,7 +282,8 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
     D.Si = D.A01 + (size_t)D.k0 * D.n1;
     D.g = D.Si + (size_t)D.k0 * D.k0;
     D.c = D.g + D.k;
-    D.work = D.c + D.k;
+    D.z = D.c + D.k;
+    D.work = D.z + D.k;
     D.status = reinterpret_cast<int *>(p + 2 * az + units + dbl_bytes);
   }
   if (!ctx->bicg_sc.ptr && ctx->bicg_sc.alloc(sizeof(phi::BicgScalars)) != cudaSuccess) {
@@ -341,7 +344,7 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
   PHI_SK(phi::bicg_launch_guess(V.x, n, grid, s));
   PHI_SK(apply_fp64(ctx, V.x, V.r[1], s));
   if (Dp) {  // r_1 -> r_1 + A Z E^-1 Z^T (b - r_1), so that b - r_1 = P (b - A x_0)
-    PHI_SK(phi::defl_launch_coeff(D, V.r[1], V.b, nullptr, s));
+    PHI_SK(phi::defl_launch_coords(D, V.r[1], V.b, s));
     PHI_SK(phi::defl_launch_update(D, V.r[1], s));
   }
   phi::BicgScalars init{};
@@ -404,7 +407,7 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
   if (result == PHI_OK && Dp) {
     // The coarse part: x = y + Z E^-1 Z^T (b - A y).
     cudaError_t e = apply_fp64(ctx, V.x, V.r[1], s);
-    if (e == cudaSuccess) e = phi::defl_launch_coeff(D, V.r[1], V.b, nullptr, s);
+    if (e == cudaSuccess) e = phi::defl_launch_coeff(D, V.r[1], V.b, s);
     if (e == cudaSuccess) e = phi::defl_launch_correct(D, V.x, s);
     if (e != cudaSuccess) result = steady_err(ctx, e, "coarse correction");
   }
