@@ -219,9 +219,9 @@ struct TileLayout {
 };
 
 // Resident warps per SM the register budget is fitted to.
-template <int KT, bool MIXED, int BT, bool PAIRS>
+template <int N, int KT, bool MIXED, int BT, bool PAIRS>
 struct TileMinBlocks {
-  static constexpr int warps = MIXED ? (PAIRS ? 32 : 24) : (KT == 1 ? 32 : 24);
+  static constexpr int warps = MIXED ? (PAIRS && KT == 2 && N >= 6 ? 32 : 24) : (KT == 1 && !PAIRS ? 32 : 24);
   static constexpr int value = warps / (BT / 32);
 };
 
@@ -265,9 +265,13 @@ struct TileArith {
 // one's scale sp and c_t (pairs), or a = sp * c_t (elements).
 template <class R, bool PAIRS>
 struct TileCoef;
-template <class R>
-struct alignas(16) TileCoef<R, true> {
-  R s, sp, cx, cy;
+template <>
+struct alignas(16) TileCoef<float, true> {
+  float s, sp, cx, cy;
+};
+template <>
+struct alignas(16) TileCoef<double, true> {  // c_t from its table: half the shared memory
+  double s, sp;
 };
 template <class R>
 struct alignas(16) TileCoef<R, false> {
@@ -279,8 +283,10 @@ __device__ __forceinline__ C tile_coef(R s, R sp, double2 c) {
   f.s = s;
   if constexpr (std::is_same<C, TileCoef<R, true>>::value) {
     f.sp = sp;
-    f.cx = (R)c.x;
-    f.cy = (R)c.y;
+    if constexpr (std::is_same<R, float>::value) {
+      f.cx = (R)c.x;
+      f.cy = (R)c.y;
+    }
   } else {
     f.pad = 0;
     f.ax = sp * (R)c.x;
@@ -391,6 +397,7 @@ struct TileIn {
   const R *mats;        // Matsubara factor per element
   const int2 *ids;      // neighbour element offsets (next, prev), -1 absent
   const C *cfs;         // neighbour coefficients
+  const double2 *ccs;   // c_t (FP64 pairs)
   const double *deph;   // dephasing rates
   const uint8_t *mi;    // occupations (time-local truncation)
   const TX *xin;        // the stage input of every node (HBM)
@@ -443,10 +450,17 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
   const TX zero = mk<TX>(0.0, 0.0);
   TX *Us = in.Us;
   if constexpr (S::kPairs) {
+    // FP64 of few sites: each pair forms its two products itself, which costs
+    // less than the exchange and its barrier (6-site RKF45 2.85 -> 2.37 ms).
+    constexpr bool kDirect = !MIXED && N <= 6;
+    auto coupling = [&](int t, const auto &f) {  // c_t
+      if constexpr (MIXED) return mk<TX>(f.cx, f.cy);
+      else return in.ccs[t];
+    };
     // Every neighbour value the pairs need, as independent predicated loads,
-    // issued before the products, whose work hides their latency, where the
-    // registers hold them.
-    constexpr bool kHoist = MIXED || KT <= 2;
+    // in mixed precision issued before the products, whose work hides their
+    // latency (FP64 would spill).
+    constexpr bool kHoist = MIXED;
     TX gn_c[S::PR][KT], gp_c[S::PR][KT], gn_r[S::PR][KT], gp_r[S::PR][KT];
     auto gather = [&](int r) {
       const int i = m.ij[r] & 255, j = m.ij[r] >> 8 & 255, nd = m.ij[r] >> 16;
@@ -465,18 +479,52 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int r = 0; r < S::PR; ++r) gather(r);
     }
-    tile_products<N, KT, MIXED, BT, ST>(c, m, in.Xs, in.Hs, dx);
+    if constexpr (!kDirect) {
+      tile_products<N, KT, MIXED, BT, ST>(c, m, in.Xs, in.Hs, dx);
 #pragma unroll
-    for (int r = 0; r < RR; ++r)
-      if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
-    __syncthreads();
+      for (int r = 0; r < RR; ++r)
+        if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
+      __syncthreads();
+    }
 #pragma unroll
     for (int r = 0; r < S::PR; ++r) {
-      if constexpr (!kHoist) gather(r);
       const int i = m.ij[r] & 255, j = m.ij[r] >> 8 & 255, nd = m.ij[r] >> 16;
       if (nd >= in.nt_here) continue;
       const int uij = nd * EU + i + j * NP, uji = nd * EU + j + i * NP;
-      const TX a = Us[uij], b = Us[uji];
+      TX a = zero, b = zero;  // A_ij, A_ji
+      if constexpr (!kDirect) {
+        a = Us[uij];
+        b = Us[uji];
+      } else {
+        const TX *X = in.Xs + nd * ES;
+        if (c.h_real) {
+          const R *Hr = reinterpret_cast<const R *>(in.Hs);
+#pragma unroll
+          for (int k = 0; k < N; ++k) {
+            const R hik = Hr[i + k * N], hjk = Hr[j + k * N];
+            const TX xkj = X[k + j * N], xik = X[i + k * N];  // X_ki = conj(X_ik)
+            a.x = fma(hik, xkj.x, a.x);
+            a.y = fma(hik, xkj.y, a.y);
+            b.x = fma(hjk, xik.x, b.x);
+            b.y = fma(-hjk, xik.y, b.y);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < N; ++k) {
+            const TX hik = in.Hs[i + k * N], xkj = X[k + j * N];
+            const TX hjk = in.Hs[j + k * N], xik = X[i + k * N];
+            a.x = fma(hik.x, xkj.x, a.x);
+            a.x = fma(-hik.y, xkj.y, a.x);
+            a.y = fma(hik.x, xkj.y, a.y);
+            a.y = fma(hik.y, xkj.x, a.y);
+            b.x = fma(hjk.x, xik.x, b.x);
+            b.x = fma(hjk.y, xik.y, b.x);
+            b.y = fma(-hjk.x, xik.y, b.y);
+            b.y = fma(hjk.y, xik.x, b.y);
+          }
+        }
+      }
+      if constexpr (!kHoist) gather(r);
       // -i/hbar (A_ij - conj(A_ji))
       R vx = (a.y + b.y) * ih, vy = -(a.x - b.x) * ih;
       if (nb) {
@@ -488,18 +536,19 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
           for (int q = 0; q < KT; ++q) {
             const auto fj = in.cfs[nd * T + j * KT + q], fi = in.cfs[nd * T + i * KT + q];
+            const TX cj = coupling(j * KT + q, fj), ci = coupling(i * KT + q, fi);
             // column part: + p X+_ij (p = i s), + i conj(c) sp X-_ij
             vx = fma(-fj.s, gn_c[r][q].y, vx);
             vy = fma(fj.s, gn_c[r][q].x, vy);
             const TX g = gp_c[r][q];
-            const R re = fj.cx * g.x + fj.cy * g.y, im = fj.cx * g.y - fj.cy * g.x;
+            const R re = cj.x * g.x + cj.y * g.y, im = cj.x * g.y - cj.y * g.x;
             vx = fma(-fj.sp, im, vx);
             vy = fma(fj.sp, re, vy);
             // row part: - p conj(X+_ji), - i c sp conj(X-_ji)
             vx = fma(-fi.s, gn_r[r][q].y, vx);
             vy = fma(-fi.s, gn_r[r][q].x, vy);
             const TX h = gp_r[r][q];
-            const R re2 = fi.cx * h.x + fi.cy * h.y, im2 = fi.cy * h.x - fi.cx * h.y;
+            const R re2 = ci.x * h.x + ci.y * h.y, im2 = ci.y * h.x - ci.x * h.y;
             vx = fma(fi.sp, im2, vx);
             vy = fma(-fi.sp, re2, vy);
           }
@@ -508,7 +557,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
           for (int q = 0; q < KT; ++q) {
             const auto fi = in.cfs[nd * T + i * KT + q];
-            vx = fma((R)2 * fi.sp * fi.cy, gp_r[r][q].x, vx);
+            vx = fma((R)2 * fi.sp * coupling(i * KT + q, fi).y, gp_r[r][q].x, vx);
           }
         }
       }
@@ -957,7 +1006,7 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
   }
 
   const TileMap<N, KT, MIXED, BT, ST> m(c);
-  const In in{Xs, Us, Hs, mats, ids, cfs, deph, c.mi + n0 * T, xin, nt_here};
+  const In in{Xs, Us, Hs, mats, ids, cfs, nullptr, deph, c.mi + n0 * T, xin, nt_here};
   TX dx[S::RR];
   tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
   ok = p.npre == 0 || mbar_wait_bounded(&bars[1], par1);

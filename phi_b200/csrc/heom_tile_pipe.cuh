@@ -79,7 +79,7 @@ size_t pipe_smem(int T, int L, int npre, const int *pre_bytes) {
 }
 
 template <int N, int KT, bool MIXED, int BT, int ST>
-__global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, MIXED, KT, BT, ST>::kPairs>::value) heom_tile_pipe_kernel(TileParams p) {
+__global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<N, MIXED, KT, BT, ST>::kPairs>::value) heom_tile_pipe_kernel(TileParams p) {
   using S = TileShape<N, MIXED, KT, BT, ST>;
   using Lay = PipeLayout<N, KT, MIXED, BT, ST>;
   using TX = typename TileArith<MIXED>::TX;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<KT, MIXED, BT, TileShape<N, 
     const double *deph =
         reinterpret_cast<const double *>(sb + Lay::kSlotX + 2 * Lay::kSlotIds + Lay::kSlotMi) + (n0 & 1);
     const TileIn<N, KT, MIXED, BT, ST> in{Xs,   Us,   Hs, mats, ids + s * NT * T, cfs + s * NT * T,
-                                      deph, slot_mi(s, n0), xin, nt_here};
+                                      ccs, deph, slot_mi(s, n0), xin, nt_here};
     TX dx[S::RR];
     tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
     // The operands have had the derivative's time to land.  A wait that gave
