@@ -10,6 +10,12 @@ namespace phi {
 // True when a compile-time-N tiled kernel exists for this problem.
 bool tile_kernel_available(const HeomConsts &c);
 cudaError_t launch_tile_stage(const StageLaunch &L, cudaStream_t stream);
+// A whole RK4 run of a small hierarchy in one launch (heom_tile_resident.cu):
+// `steps` steps of dt on L.y in place (mixed: with its complex64 copy L.y32),
+// stage inputs through L.xv and L.outv, rho_0 rows and counters as the stage
+// kernels keep them.  cudaErrorNotSupported, nothing launched, where the
+// hierarchy has more tiles than a cluster or needs the launch-per-stage path.
+cudaError_t launch_tile_resident_rk4(const StageLaunch &L, double dt, long long steps, cudaStream_t stream);
 // Node stride of complex64 buffers (N*N rounded up to even).
 int mixed_node_stride(int N);
 

@@ -167,8 +167,10 @@ __device__ __forceinline__ double2 cfma(double2 acc, double2 b, double s) {
 template <class TX> __device__ __forceinline__ void st_stream(TX *p, TX v) { __stcs(p, v); }
 
 // Which kernel a tile shape is for: the single-instance apply and RK4 stages,
-// the RKF45 stages, the batched stages.
-enum TileKind : int { kTileRk4 = 0, kTileRkf45 = 1, kTileBatch = 2 };
+// the RKF45 stages, the batched stages, the resident RK4 run with one element
+// per thread or several.
+enum TileKind : int { kTileRk4 = 0, kTileRkf45 = 1, kTileBatch = 2, kTileResident = 3, kTileResidentWide = 4 };
+constexpr bool tile_resident(int kind) { return kind == kTileResident || kind == kTileResidentWide; }
 
 template <int N, bool MIXED, int KT, int BT = kTileThreads, int ST = kTileRk4>
 struct TileShape {
@@ -190,10 +192,12 @@ struct TileShape {
   // apply over 125,970 nodes 29.9 -> 26.9 us); a batch has tiles enough and
   // takes the large ones (48 instances: 30.1 -> 28.1 ms).
   static constexpr int R1 = MIXED ? 4 : 2;
-  static constexpr int kRounds = ST == kTileBatch  ? (!MIXED && R1 * CS / N > 40 ? 1 : R1)
-                                 : R1 * CS / N <= 40 ? R1
-                                 : 2 * CS / N <= 40  ? 2
-                                                     : 1;
+  static constexpr int kRounds = ST == kTileResident       ? 1
+                                 : ST == kTileResidentWide ? R1
+                                 : ST == kTileBatch        ? (!MIXED && R1 * CS / N > 40 ? 1 : R1)
+                                 : R1 * CS / N <= 40       ? R1
+                                 : 2 * CS / N <= 40        ? 2
+                                                           : 1;
   static constexpr int NT0 = kPairs ? BT / P : kRounds * CS / N;
   static constexpr int NT = NT0 < 1 ? 1 : (NT0 > 64 ? 64 : NT0);
   static constexpr int RR = (NT * N + CS - 1) / CS;  // elements per thread
@@ -383,6 +387,13 @@ __device__ __forceinline__ void tile_products(const HeomConsts &c, const TileMap
       }
     }
   }
+}
+
+// An element of a linked ADO; a resident run reads what other CTAs of its
+// launch wrote, past L1.
+template <int ST, class TX>
+__device__ __forceinline__ TX ld_neighbour(const TX *p) {
+  return tile_resident(ST) ? __ldcg(p) : *p;
 }
 
 // What a tile's derivative is computed from (shared memory, except xin).
@@ -579,7 +590,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
   } else {
     const int i = m.i;
     // FP64 issues the gathers after the products (registers).
-    constexpr bool kHoist = MIXED || KT == 1 || (KT == 2 && ST == kTileRkf45);
+    constexpr bool kHoist = MIXED || KT == 1 || tile_resident(ST) || (KT == 2 && ST == kTileRkf45);
     TX gn[RR][KT], gp[RR][KT];
     auto gather = [&](int r) {
       const bool on = nb && m.on(r, in.nt_here);
@@ -588,8 +599,8 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
 #pragma unroll
       for (int q = 0; q < KT; ++q) {
         const int2 id = in.ids[m.rec[r] + q];
-        gn[r][q] = (on && id.x >= 0 && !diag) ? *(in.xin + id.x + off) : zero;
-        gp[r][q] = (on && id.y >= 0) ? *(in.xin + id.y + off) : zero;
+        gn[r][q] = (on && id.x >= 0 && !diag) ? ld_neighbour<ST>(in.xin + id.x + off) : zero;
+        gp[r][q] = (on && id.y >= 0) ? ld_neighbour<ST>(in.xin + id.y + off) : zero;
       }
     };
     if constexpr (kHoist) {

@@ -277,12 +277,32 @@ extern "C" int phi_gpu_rk4(phi_ctx *ctx, double dt, double t_end, double output_
   hc.nout = 0;
   PHI_CK(cudaMemcpyAsync(ctx->ctl.ptr, &hc, sizeof(hc), cudaMemcpyHostToDevice, ctx->stream));
 
-  // A small hierarchy runs whole in one CTA (launches of at most
-  // kSmallChunk steps each).
-  if (!ctx->annealing && !ctx->mixed() && phi::small_rk4_eligible(ctx->c)) {
-    for (long long done = 0; done < steps; done += kSmallChunk)
-      PHI_CK(phi::launch_small_rk4(ctx->c, ctx->y.as<double2>(), dt, std::min<long long>(kSmallChunk, steps - done),
-                                   ctx->ctl.as<phi::Rk4Ctl>(), dtraj, ctx->stream));
+  // A small hierarchy runs whole in one CTA or one cluster (launches of at
+  // most kSmallChunk steps each).
+  const bool small = !ctx->annealing && !ctx->mixed() && phi::small_rk4_eligible(ctx->c);
+  bool resident = false;
+  for (long long done = 0; done < steps; done += kSmallChunk) {
+    const long long chunk = std::min<long long>(kSmallChunk, steps - done);
+    if (small) {
+      PHI_CK(phi::launch_small_rk4(ctx->c, ctx->y.as<double2>(), dt, chunk, ctx->ctl.as<phi::Rk4Ctl>(), dtraj,
+                                   ctx->stream));
+    } else {
+      phi::StageLaunch L;
+      L.c = ctx->c;
+      L.mixed = ctx->mixed();
+      L.y = ctx->y.as<double2>();
+      L.y32 = ctx->y32.ptr;
+      L.xv = ctx->xa.ptr;
+      L.outv = ctx->xb.ptr;
+      L.rk4 = ctx->ctl.as<phi::Rk4Ctl>();
+      L.traj = dtraj;
+      const cudaError_t e = phi::launch_tile_resident_rk4(L, dt, chunk, ctx->stream);
+      if (done == 0 && e == cudaErrorNotSupported) break;
+      PHI_CK(e);
+      resident = true;
+    }
+  }
+  if (small || resident) {
     if (rows > 0)
       PHI_CK(cudaMemcpyAsync(traj, dtraj, (size_t)rows * ctx->desc.num_states * ctx->desc.num_states * sizeof(double2),
                              cudaMemcpyDeviceToHost, ctx->stream));
