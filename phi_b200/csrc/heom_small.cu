@@ -133,12 +133,42 @@ __host__ __device__ inline int small_row_max(const HeomConsts &c) {
   return 2 * c.N + 1 + (c.kind == kIndependent ? 4 * c.T : 2 * c.T);
 }
 
-// RM > 0: every thread owns at most one item and keeps its row (at most RM
-// entries, padded with zero coefficients) in registers for the whole run;
-// RM = 0: rows stay in shared memory and threads loop over items.
-template <int KIND, int RM>
+// Number of an item's entries with a purely imaginary coefficient (2 of the 4
+// products): the commutator of a real H and the next terms.
+__host__ __device__ inline int small_imag_max(const HeomConsts &c) {
+  return (c.h_real ? 2 * c.N : 0) + (c.kind == kIndependent ? 2 * c.T : c.T);
+}
+
+// Moves up to `most` entries with a zero real coefficient to the front of an
+// item's row (other entries can have one too); returns their number.
+__device__ int partition_row(int n, int most, int *idx, double2 *coef) {
+  int front = 0;
+  for (int r = 0; r < n && front < most; ++r) {
+    if (coef[r].x != 0.0) continue;
+    const double2 cf = coef[front];
+    const int e = idx[front];
+    coef[front] = coef[r];
+    idx[front] = idx[r];
+    coef[r] = cf;
+    idx[r] = e;
+    ++front;
+  }
+  return front;
+}
+
+// RI + RC > 0: every thread owns at most one item and keeps its row in
+// registers for the whole run -- up to RI imaginary and RC complex entries,
+// padded with zero coefficients -- with the state and the accumulator of its
+// element and of the mirrored one.  A stage is then the gather of the row from
+// one of two shared stage inputs, its products, the combine, and one barrier:
+// stage 0 reads buffer 0 (y) and writes 1, stage 1 the reverse, and so on.
+// Bound by that chain of latencies (11-node spin-boson, 2 warps): with the
+// state in shared memory and every entry complex a stage took 0.267 us.
+// RI = RC = 0: rows stay in shared memory and threads loop over items.
+template <int KIND, int RI, int RC>
 __global__ void __launch_bounds__(kSmallThreads, 1) heom_small_rk4_kernel(SmallRk4Params p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool REG = RI + RC > 0;
   const HeomConsts &c = p.c;
   const int N = c.N, E = N * N, P = N * (N + 1) / 2;
   const long long M = c.M, ME = M * E, items = M * P;
@@ -161,123 +191,146 @@ __global__ void __launch_bounds__(kSmallThreads, 1) heom_small_rk4_kernel(SmallR
     cnt[u] = build_row<KIND>(c, Hs, n, __ldg(c.pair_i + q), __ldg(c.pair_j + q), idx + u * R, coef + u * R);
   }
   __syncthreads();
-  // Register-resident row of this thread's item (RM > 0).
-  int r_idx[RM > 0 ? RM : 1];
-  double2 r_cf[RM > 0 ? RM : 1];
-  int my_out0 = -1, my_out1 = -1;  // K offsets of the item and its mirror (-1: none)
-  if (RM > 0) {
-    const long long u = tid;
-    const int nr = u < items ? cnt[u] : 0;
-#pragma unroll
-    for (int r = 0; r < RM; ++r) {
-      r_idx[r] = r < nr ? idx[u * R + r] : 0;
-      r_cf[r] = r < nr ? coef[u * R + r] : make_double2(0.0, 0.0);
-    }
-    if (u < items) {
-      const long long n = u / P;
-      const int q = (int)(u - n * P);
-      const int i = __ldg(c.pair_i + q), j = __ldg(c.pair_j + q);
-      my_out0 = (int)(n * E + i + j * N);
-      my_out1 = i == j ? -1 : (int)(n * E + j + i * N);
-    }
-  }
   const double dt = p.dt;
   Rk4Ctl *rc = p.rk4;
   long long step = rc->step, nout = rc->nout;
   const long long out_factor = rc->out_factor, capacity = rc->capacity;
-  for (long long it = 0; it < p.steps; ++it) {
+  if constexpr (REG) {
+    int i_idx[RI], c_idx[RC];
+    double i_cf[RI];
+    double2 c_cf[RC];
+    const long long u = tid;
+    const bool own = u < items;
+    int nr = 0, ni = 0, e0 = -1, e1 = -1;  // the item's element and its mirror (-1: none)
+    if (own) {
+      nr = cnt[u];
+      ni = partition_row(nr, RI, idx + u * R, coef + u * R);
+      const long long n = u / P;
+      const int q = (int)(u - n * P);
+      const int i = __ldg(c.pair_i + q), j = __ldg(c.pair_j + q);
+      e0 = (int)(n * E + i + j * N);
+      e1 = i == j ? -1 : (int)(n * E + j + i * N);
+    }
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const double a = s == 2 ? dt : dt / 2;
-      const double w = (s == 0 || s == 3) ? dt / 6 : dt / 3;
-      if (RM > 0) {
-        // One item per thread: the thread combines its own two elements
-        // right away, and the stage inputs alternate between X and K (K
-        // holds X_2), so a stage needs one barrier:
-        //   stage 0: Y -> X,  1: X -> K,  2: K -> X,  3: X -> Y.
-        const double2 *in = s == 0 ? Y : (s == 2 ? K : X);
-        double2 *outb = s == 1 ? K : X;
-        if (my_out0 >= 0) {
-          double2 xv[RM > 0 ? RM : 1];
+    for (int r = 0; r < RI; ++r) {
+      i_idx[r] = r < ni ? idx[u * R + r] : 0;
+      i_cf[r] = r < ni ? coef[u * R + r].y : 0.0;
+    }
 #pragma unroll
-          for (int r = 0; r < RM; ++r) xv[r] = in[r_idx[r]];
+    for (int r = 0; r < RC; ++r) {
+      c_idx[r] = ni + r < nr ? idx[u * R + ni + r] : 0;
+      c_cf[r] = ni + r < nr ? coef[u * R + ni + r] : make_double2(0.0, 0.0);
+    }
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 y0 = own ? Y[e0] : zero, y1 = e1 >= 0 ? Y[e1] : zero, a0 = zero, a1 = zero;
+    for (long long it = 0; it < p.steps; ++it) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double a = s == 2 ? dt : dt / 2;
+        const double w = (s == 0 || s == 3) ? dt / 6 : dt / 3;
+        const double2 *in = s & 1 ? X : Y;
+        double2 *out = s & 1 ? Y : X;
+        double2 xi[RI], xc[RC];
+#pragma unroll
+        for (int r = 0; r < RI; ++r) xi[r] = in[i_idx[r]];
+#pragma unroll
+        for (int r = 0; r < RC; ++r) xc[r] = in[c_idx[r]];
+        // Two chains per component: the imaginary entries and the complex ones.
+        double2 v = zero, z = zero;
+#pragma unroll
+        for (int r = 0; r < RI; ++r) {
+          v.x = fma(-i_cf[r], xi[r].y, v.x);
+          v.y = fma(i_cf[r], xi[r].x, v.y);
+        }
+#pragma unroll
+        for (int r = 0; r < RC; ++r) {
+          z.x = fma(c_cf[r].x, xc[r].x, z.x);
+          z.x = fma(-c_cf[r].y, xc[r].y, z.x);
+          z.y = fma(c_cf[r].x, xc[r].y, z.y);
+          z.y = fma(c_cf[r].y, xc[r].x, z.y);
+        }
+        v.x += z.x;
+        v.y = e1 < 0 ? 0.0 : v.y + z.y;
+        double2 x0, x1;
+        if (s < 3) {
+          x0 = s_axpy(y0, v, a);
+          x1 = s_axpy(y1, s_conj(v), a);
+          a0 = s_axpy(s == 0 ? y0 : a0, v, w);
+          a1 = s_axpy(s == 0 ? y1 : a1, s_conj(v), w);
+        } else {
+          x0 = y0 = s_axpy(a0, v, w);
+          x1 = y1 = s_axpy(a1, s_conj(v), w);
+        }
+        if (own) out[e0] = x0;
+        if (e1 >= 0) out[e1] = x1;
+        __syncthreads();
+      }
+      // rho_0 row after step `step` when step % out_factor == 0 (:2858).
+      if (out_factor > 0 && step % out_factor == 0) {
+        if (p.traj && nout < capacity) {
+          if (own && e0 < E) p.traj[nout * E + e0] = y0;
+          if (e1 >= 0 && e1 < E) p.traj[nout * E + e1] = y1;
+        }
+        ++nout;
+      }
+      ++step;
+    }
+    if (own) p.y[e0] = y0;
+    if (e1 >= 0) p.y[e1] = y1;
+  } else {
+    for (long long it = 0; it < p.steps; ++it) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double a = s == 2 ? dt : dt / 2;
+        const double w = (s == 0 || s == 3) ? dt / 6 : dt / 3;
+        const double2 *in = s == 0 ? Y : X;
+        for (long long u = tid; u < items; u += nth) {
+          const int *ri = idx + u * R;
+          const double2 *rcf = coef + u * R;
           double2 v = make_double2(0.0, 0.0);
-#pragma unroll
-          for (int r = 0; r < RM; ++r) {
-            v.x = fma(r_cf[r].x, xv[r].x, v.x);
-            v.x = fma(-r_cf[r].y, xv[r].y, v.x);
-            v.y = fma(r_cf[r].x, xv[r].y, v.y);
-            v.y = fma(r_cf[r].y, xv[r].x, v.y);
+          for (int r = 0; r < cnt[u]; ++r) {
+            const double2 cf = rcf[r], x = in[ri[r]];
+            v.x = fma(cf.x, x.x, v.x);
+            v.x = fma(-cf.y, x.y, v.x);
+            v.y = fma(cf.x, x.y, v.y);
+            v.y = fma(cf.y, x.x, v.y);
           }
-          if (my_out1 < 0) v.y = 0.0;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int e = h == 0 ? my_out0 : my_out1;
-            if (e < 0) continue;
-            const double2 kv = h == 0 ? v : s_conj(v);
-            if (s == 0) {
-              const double2 ys = Y[e];
-              outb[e] = s_axpy(ys, kv, a);
-              ACC[e] = s_axpy(ys, kv, w);
-            } else if (s < 3) {
-              outb[e] = s_axpy(Y[e], kv, a);
-              ACC[e] = s_axpy(ACC[e], kv, w);
-            } else {
-              Y[e] = s_axpy(ACC[e], kv, w);
-            }
+          const long long n = u / P;
+          const int q = (int)(u - n * P);
+          const int i = __ldg(c.pair_i + q), j = __ldg(c.pair_j + q);
+          if (i == j) {
+            v.y = 0.0;
+            K[n * E + i + j * N] = v;
+          } else {
+            K[n * E + i + j * N] = v;
+            K[n * E + j + i * N] = s_conj(v);
           }
         }
         __syncthreads();
-        continue;
-      }
-      const double2 *in = s == 0 ? Y : X;
-      for (long long u = tid; u < items; u += nth) {
-        const int *ri = idx + u * R;
-        const double2 *rcf = coef + u * R;
-        double2 v = make_double2(0.0, 0.0);
-        for (int r = 0; r < cnt[u]; ++r) {
-          const double2 cf = rcf[r], x = in[ri[r]];
-          v.x = fma(cf.x, x.x, v.x);
-          v.x = fma(-cf.y, x.y, v.x);
-          v.y = fma(cf.x, x.y, v.y);
-          v.y = fma(cf.y, x.x, v.y);
+        for (long long e = tid; e < ME; e += nth) {
+          const double2 kv = K[e];
+          if (s == 0) {
+            const double2 ys = Y[e];
+            X[e] = s_axpy(ys, kv, a);
+            ACC[e] = s_axpy(ys, kv, w);
+          } else if (s < 3) {
+            X[e] = s_axpy(Y[e], kv, a);
+            ACC[e] = s_axpy(ACC[e], kv, w);
+          } else {
+            Y[e] = s_axpy(ACC[e], kv, w);
+          }
         }
-        const long long n = u / P;
-        const int q = (int)(u - n * P);
-        const int i = __ldg(c.pair_i + q), j = __ldg(c.pair_j + q);
-        if (i == j) {
-          v.y = 0.0;
-          K[n * E + i + j * N] = v;
-        } else {
-          K[n * E + i + j * N] = v;
-          K[n * E + j + i * N] = s_conj(v);
-        }
+        __syncthreads();
       }
-      __syncthreads();
-      for (long long e = tid; e < ME; e += nth) {
-        const double2 kv = K[e];
-        if (s == 0) {
-          const double2 ys = Y[e];
-          X[e] = s_axpy(ys, kv, a);
-          ACC[e] = s_axpy(ys, kv, w);
-        } else if (s < 3) {
-          X[e] = s_axpy(Y[e], kv, a);
-          ACC[e] = s_axpy(ACC[e], kv, w);
-        } else {
-          Y[e] = s_axpy(ACC[e], kv, w);
-        }
+      if (out_factor > 0 && step % out_factor == 0) {
+        if (p.traj && nout < capacity)
+          for (int e = tid; e < E; e += nth) p.traj[nout * E + e] = Y[e];
+        ++nout;
       }
-      __syncthreads();
+      ++step;
     }
-    // rho_0 row after step `step` when step % out_factor == 0 (:2858).
-    if (out_factor > 0 && step % out_factor == 0) {
-      if (p.traj && nout < capacity)
-        for (int e = tid; e < E; e += nth) p.traj[nout * E + e] = Y[e];
-      ++nout;
-    }
-    ++step;
+    for (long long e = tid; e < ME; e += nth) p.y[e] = Y[e];
   }
-  for (long long e = tid; e < ME; e += nth) p.y[e] = Y[e];
   if (tid == 0) {
     rc->step = step;
     rc->nout = nout;
@@ -300,34 +353,31 @@ int small_threads(const HeomConsts &c) {
   return (int)std::min<long long>(kSmallThreads, std::max<long long>(32, w));
 }
 
-// Register rows: the bound on a row's length, in buckets of 8 / 16
-// entries, when every item has its own thread (0 otherwise).
-int small_register_row(const HeomConsts &c) {
-  const long long items = c.M * (c.N * (c.N + 1) / 2);
-  const int r = small_row_max(c);
-  if (items > kSmallThreads) return 0;
-  return r <= 8 ? 8 : (r <= 16 ? 16 : 0);
-}
-
-template <int KIND, int RM>
+template <int KIND, int RI, int RC>
 cudaError_t launch_small_variant(const SmallRk4Params &p, size_t smem, int threads, cudaStream_t stream) {
   static int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(heom_small_rk4_kernel<KIND, RM>, smem, configured);
+  cudaError_t e = raise_smem_limit(heom_small_rk4_kernel<KIND, RI, RC>, smem, configured);
   if (e != cudaSuccess) return e;
-  heom_small_rk4_kernel<KIND, RM><<<1, threads, smem, stream>>>(p);
+  heom_small_rk4_kernel<KIND, RI, RC><<<1, threads, smem, stream>>>(p);
   return cudaGetLastError();
 }
 
+// Register rows when every item has its own thread and the bounds on its
+// imaginary and complex entries fit one of the compiled sizes.
 template <int KIND>
 cudaError_t launch_small_kind(const SmallRk4Params &p, size_t smem, cudaStream_t stream) {
   const HeomConsts &c = p.c;
-  const int rm = small_register_row(c);
-  if (rm > 0) {
-    const int threads = small_threads(c);  // >= items: one item per thread
-    if (rm == 8) return launch_small_variant<KIND, 8>(p, smem, threads, stream);
-    return launch_small_variant<KIND, 16>(p, smem, threads, stream);
+  const int threads = small_threads(c);
+  if (c.M * (c.N * (c.N + 1) / 2) <= kSmallThreads) {
+    const int ri = small_imag_max(c), total = small_row_max(c);
+    const int rc = total - ri;
+    if (ri <= 6 && rc <= 2) return launch_small_variant<KIND, 6, 2>(p, smem, threads, stream);
+    if (ri <= 8 && rc <= 4) return launch_small_variant<KIND, 8, 4>(p, smem, threads, stream);
+    if (ri <= 12 && rc <= 4) return launch_small_variant<KIND, 12, 4>(p, smem, threads, stream);
+    if (ri <= 8 && rc <= 8) return launch_small_variant<KIND, 8, 8>(p, smem, threads, stream);
+    if (ri <= 16 && rc <= 8) return launch_small_variant<KIND, 16, 8>(p, smem, threads, stream);
   }
-  return launch_small_variant<KIND, 0>(p, smem, small_threads(c), stream);
+  return launch_small_variant<KIND, 0, 0>(p, smem, threads, stream);
 }
 
 }  // namespace
