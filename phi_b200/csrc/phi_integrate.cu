@@ -429,40 +429,52 @@ int run_rkf45(phi_ctx *ctx, double dt0, double t_end, double tol, double min_dt,
   if (!ctx->host_ctl) PHI_CK(phi::cached_host_alloc(&ctx->host_ctl, sizeof(phi::Rkf45Ctl)));
   phi::Rkf45Ctl *hpin = static_cast<phi::Rkf45Ctl *>(ctx->host_ctl);
   int result = PHI_OK;
-  // Exactly max_steps attempted steps are enqueued: whole graphs of
-  // kGraphSteps, then the remainder as direct launches.  Two chunks are in
-  // flight: the done flag after chunk j is read while chunk j+1 runs; steps
-  // after completion are no-ops on the device.
+  // At most max_steps attempted steps are enqueued, in chunks: whole graphs of
+  // kGraphSteps, the remainder as one-step graphs.  A chunk is a lower bound
+  // of the steps still needed (each accepted, dt growing by dtup every time)
+  // and a quarter of those needed at the current dt on top, never more than
+  // those: steps after completion are no-ops on the device, but a no-op step
+  // of seven launches still takes about 10 us, as long as reading the control
+  // block (chunks of 16 with one always ahead ran up to 31 of them).
   long long launched = 0, graphs = 0;
-  auto enqueue_chunk = [&]() -> cudaError_t {
-    const long long left = hc.max_steps - launched;
-    if (left >= kGraphSteps) {
+  auto chunk_steps = [](const phi::Rkf45Ctl &c) -> long long {
+    const double left = (c.end_time - c.time) / c.dt;
+    if (!(left > 1.0)) return 1;
+    if (!(left < 1e6)) return 4 * kGraphSteps;
+    const double least = std::log1p(0.1 * left) / std::log(1.1);
+    return std::min<long long>(4 * kGraphSteps, (long long)std::ceil(std::min(left, least + 0.25 * left)));
+  };
+  auto enqueue_chunk = [&](long long n) -> cudaError_t {
+    n = std::min<long long>(n, hc.max_steps - launched);
+    cudaError_t e = cudaSuccess;
+    for (; n >= kGraphSteps && e == cudaSuccess; n -= kGraphSteps) {
       launched += kGraphSteps;
       ++graphs;
-      return cudaGraphLaunch(ctx->rkf45_graph, ctx->stream);
+      e = cudaGraphLaunch(ctx->rkf45_graph, ctx->stream);
     }
-    for (; launched < hc.max_steps; ++launched) {
-      cudaError_t e = cudaGraphLaunch(ctx->rkf45_graph1, ctx->stream);
-      if (e != cudaSuccess) return e;
+    for (; n > 0 && e == cudaSuccess; --n) {
+      ++launched;
+      e = cudaGraphLaunch(ctx->rkf45_graph1, ctx->stream);
     }
-    return cudaSuccess;
+    return e;
   };
-  PHI_CK(enqueue_chunk());
+  PHI_CK(enqueue_chunk(chunk_steps(hc)));
   for (;;) {
-    cudaError_t e = cudaSuccess;
-    if (launched < hc.max_steps) e = enqueue_chunk();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hpin, ctx->ctl.ptr, sizeof(phi::Rkf45Ctl), cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(hpin, ctx->ctl.ptr, sizeof(phi::Rkf45Ctl), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess && !hpin->done && launched < hc.max_steps) {
+      e = enqueue_chunk(chunk_steps(*hpin));
+      if (e == cudaSuccess) continue;
+    }
     if (e != cudaSuccess) {
       result = cuda_err(ctx, e, "rkf45 graph");
       break;
     }
     if (hpin->done) break;
-    if (launched >= hc.max_steps) {  // every step ran and the device did not stop
-      ctx->error = "rkf45: the device control block did not finish after max_steps steps";
-      result = PHI_E_CUDA;
-      break;
-    }
+    // every step ran and the device did not stop
+    ctx->error = "rkf45: the device control block did not finish after max_steps steps";
+    result = PHI_E_CUDA;
+    break;
   }
   ctx->graph_launches += graphs;
   if (result == PHI_OK) {
