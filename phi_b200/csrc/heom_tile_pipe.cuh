@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<
     return true;
   };
   if (p.dependent) {
-    pdl_launch_dependents();
+    if (RKF) pdl_launch_dependents();
     if (c.h_dynamic) pdl_wait();  // H is read below
   } else if (!begin()) {
     return;
@@ -256,6 +256,12 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<
     const long long n0 = tile * NT;
     const int nt_here = (int)((c.M - n0) < NT ? (c.M - n0) : NT);
     next_issued = tile + gridDim.x < ntiles;
+    // The next kernel may start from each CTA's last tile on: released at
+    // the start, its CTAs took the places that freed up first and a chain of
+    // waiting kernels built up (16-site FP64 RK4 3.02 ms for 32 steps, 2.53
+    // so; 3-site 1.01 and 0.83 ms).  RKF45 stages, which are dependents only
+    // with one tile per CTA, are 1-2 % faster released at the start.
+    if (!RKF && p.dependent && !next_issued) pdl_launch_dependents();
     if (tid == 0) {
       if (next_issued) issue_slot(tile + gridDim.x, s ^ 1);
       if (p.npre > 0) issue_pre(tile);
@@ -352,13 +358,14 @@ cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm
   if (p.c.tile_cps > 0 && p.c.tile_cps * sms < cap) cap = p.c.tile_cps * sms;
   if (p.dot_w && p.dot_slots < cap) cap = p.dot_slots;
   const long long grid = tiles < cap ? tiles : cap;
-  // Dependent launch (the preamble overlaps the previous kernel) for the
-  // apply and where every CTA has one tile: 8-site mixed RK4 stage 6.5 -> 5.5
-  // us, 84-node trimer 4.0 -> 3.0 us, 4-site apply 37.2 -> 34.5 us.  Stages
-  // of several tiles per CTA gained up to 10 % (24 sites) but lost up to 22 %
-  // (7-site mixed RKF45), so they keep the plain launch.
+  // Dependent launch (the preamble overlaps the previous kernel) for the RK4
+  // stages, the apply, and RKF45 stages of one tile per CTA: 8-site mixed RK4
+  // stage 6.5 -> 5.5 us, 84-node trimer 4.0 -> 3.0 us, 4-site apply 37.2 -> 34.5
+  // us, 7-site FP64 RK4 3.44 -> 3.22 ms (64 steps), 24-site 1.42 -> 1.31.  RKF45
+  // stages of several tiles per CTA gain nothing (7-site mixed 9.61 -> 9.57
+  // ms, FP64 8.67 -> 8.91) and keep the plain launch.
   TileParams d = p;
-  d.dependent = p.mode == kModeApply || tiles <= cap;
+  d.dependent = ST == kTileRk4 || tiles <= cap;
   return launch_dependent(d.dependent, kern, dim3((unsigned)grid), dim3(BT), smem, stream, d);
 }
 
