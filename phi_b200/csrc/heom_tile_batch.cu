@@ -60,14 +60,17 @@ __device__ __forceinline__ int run_tile_any(const TileParams &p, long long tile,
   }
 }
 
-// Resident CTAs per SM the register budget is fitted to: 2, because the
-// out-of-line tile functions take up to 128 registers (timed on a
-// 48-instance workload, ms for 16 RK4 steps: mixed 28.4 at 2, 32.4 at 3,
-// 43.7 at 4; FP64 45.1 at 2, 45.9 at 3).
-constexpr int kBatchMinBlocks = 2;
+// Resident CTAs per SM the register budget is fitted to.  A tile is one
+// serial chain, so more of them in flight outweigh the spills of the large
+// instantiations up to 80 registers (mixed) and 64 (FP64).  Timed with as many
+// CTAs per SM as fit, 48 instances x 16 RK4 steps / 512 instances x 1 step, ms:
+//   mixed  18.4 / 116.7 at 2, 17.1 / 115.7 at 3, 16.6 / 119.4 at 4, 18.1 / 196 at 5
+//   FP64   27.0 / 221 at 2, 22.2 / 176 at 3, 20.9 / 171 at 4, 23.1 / 248 at 5.
+template <bool MIXED>
+constexpr int kBatchMinBlocks = MIXED ? 3 : 4;
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kTileThreads, kBatchMinBlocks)
+__global__ void __launch_bounds__(kTileThreads, kBatchMinBlocks<MIXED>)
     heom_tile_batch_kernel(const TileParams *__restrict__ params, const long long *__restrict__ tile_start,
                            int count, long long total_tiles, int *err_flag) {
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -37,13 +37,16 @@ struct phi_batch {
   bool mixed = false;
   cudaStream_t stream = nullptr;
   phi::DeviceBuffer err;  // batch-level flag of the persistent kernel
-  phi_batch_schedule sched{1, 1, 0.0};
+  // ctas_per_sm 0 (not tuned): as many CTAs per SM as a stage's kernel fits.
+  // A tile is one serial chain, so the second CTA of an SM is nearly free: 48
+  // uneven instances 1.76 -> 1.15 ms per RK4 step with a second CTA, 1.07 with a third.
+  phi_batch_schedule sched{0, 1, 0.0};
   // RK4 stage plans for (dt, schedule) and the captured graph of them.
   double plan_dt = 0.0;
   int plan_order = -1;
   StagePlan rk4[4];
   cudaGraphExec_t graph = nullptr;
-  int graph_grid = 0;
+  int graph_cps = 0;
   std::string error;
 
   ~phi_batch() {
@@ -74,7 +77,9 @@ struct phi_batch {
     }
     return idx;
   }
-  int grid() const { return std::max(1, sched.ctas_per_sm) * num_sms; }
+  int grid(const phi::TileBatchPlan &plan) const {
+    return (sched.ctas_per_sm > 0 ? sched.ctas_per_sm : std::max(1, phi::tile_batch_occupancy(plan))) * num_sms;
+  }
 };
 
 namespace {
@@ -321,14 +326,13 @@ extern "C" int phi_gpu_batch_rk4(phi_batch *batch, double dt, int64_t steps, phi
     if (batch->graph) cudaGraphExecDestroy(batch->graph);
     batch->graph = nullptr;
   }
-  const int grid = batch->grid();
-  if (batch->graph && batch->graph_grid != grid) {
+  if (batch->graph && batch->graph_cps != batch->sched.ctas_per_sm) {
     cudaGraphExecDestroy(batch->graph);
     batch->graph = nullptr;
   }
   auto enqueue_step = [&]() -> cudaError_t {
     for (int st = 0; st < 4; ++st) {
-      cudaError_t e = phi::launch_tile_batch(batch->rk4[st].plan, grid, s);
+      cudaError_t e = phi::launch_tile_batch(batch->rk4[st].plan, batch->grid(batch->rk4[st].plan), s);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -355,7 +359,7 @@ extern "C" int phi_gpu_batch_rk4(phi_batch *batch, double dt, int64_t steps, phi
     cudaGraphDestroy(g);
     if (e == cudaSuccess) e = cudaGraphUpload(batch->graph, s);  // not on the first launch
     if (e != cudaSuccess) return batch->cuda_fail(e, "batch graph instantiate");
-    batch->graph_grid = grid;
+    batch->graph_cps = batch->sched.ctas_per_sm;
   }
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
