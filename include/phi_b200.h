@@ -297,8 +297,10 @@ PHI_API int phi_gpu_set_steady_deflation(phi_ctx *ctx, int32_t tiers);
  * Liouvillian apply for each block size (the shape's default and one
  * alternative) and each cap on persistent CTAs per SM, for problems of at
  * least 2^20 complex elements, and keeps the fastest (once per device,
- * shape and size class in the process).  Results do not depend on the
- * schedule, only the time.  threads = 0: the problem runs on the generic
+ * shape and size class in the process).  The RKF45 stages have a schedule of
+ * their own, timed the same way by a context's first RKF45 run; setting a
+ * schedule sets both.  Results do not depend on the
+ * schedule, only the time.  threads = 0: the problem runs on the node
  * kernel.  ctas_per_sm = 0: as many as fit. */
 typedef struct {
   int32_t threads;

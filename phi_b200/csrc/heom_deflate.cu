@@ -20,8 +20,8 @@
 // once per solve, a projection is that gather and one rows x k product,
 // L2-resident (the solve with E's factors in one CTA took 15 us of every
 // operator product on the 4-site chain; the gather takes 5).  A Z is
-// built once per solve by one batched launch of the generic Liouvillian
-// kernel over those nodes (k unit inputs).  First-tier nodes are not
+// built once per solve by one batched launch of the node kernel
+// (heom_kernels.cu) over those nodes (k unit inputs).  First-tier nodes are not
 // neighbours of one another, so E = [[A00, A01], [A10, D]] with D block
 // diagonal; E is kept factored through the Schur complement
 // S = A00 - A01 D^-1 A10 of rho_0's coordinates.

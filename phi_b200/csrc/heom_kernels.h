@@ -37,10 +37,10 @@ struct StageLaunch {
   const double2 *dot_w = nullptr;
   double *dot_part = nullptr;
   int dot_slots = 0;
-  // The generic kernel even where the tiled one applies (with c.M lowered,
+  // The node kernel even where the tiled one applies (with c.M lowered,
   // the rows of the first c.M nodes only; neighbour ids index the whole x).
   bool generic = false;
-  // Generic kernel, apply mode: `batch` inputs at x + i * x_bstride, outputs
+  // Node kernel, apply mode: `batch` inputs at x + i * x_bstride, outputs
   // at out + i * out_bstride (complex elements).
   int batch = 1;
   long long x_bstride = 0, out_bstride = 0;

@@ -7,7 +7,7 @@
 // stage input and the stage derivative in shared memory and loops over every
 // step of the run on the device: a stage is one pass over the hierarchy's
 // upper-triangle (node, pair) items and one element-wise combine, separated
-// by block barriers.  The arithmetic is that of the generic group kernel
+// by block barriers.  The arithmetic is that of the node kernel
 // (heom_kernels.cu) for IndependentBath and DiagonalBath couplings:
 // HierarchyUpdater::Get (hierarchy_updater.h:36-75, hierarchy_updater.cc
 // :84-127, :216-254) and the RK4 combines of Rk4Integrate

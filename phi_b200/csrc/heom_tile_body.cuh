@@ -43,7 +43,7 @@
 // Stores of the next stage input use the default cache policy (its neighbour
 // gathers in the next stage should hit L2); k and accumulator stores stream.
 // This kernel serves PHI's identity site map (bath m on |m><m|, terms of site
-// m are m*(K+1) .. m*(K+1)+K) with K+1 <= 3; other maps use the generic
+// m are m*(K+1) .. m*(K+1)+K) with K+1 <= 3; other maps use the node
 // kernel of heom_kernels.cu (FP64 only).
 //
 // Every mbarrier wait is bounded: after kMaxPolls polls the kernel records the

@@ -1,5 +1,5 @@
 // heom_tl_term.cuh -- the time-local truncation term of one ADO element
-// (internal; shared by the tiled and the generic stage kernels).
+// (internal; shared by the tiled and the node stage kernels).
 //
 // For an independent bath m on site m, IndependentBath::DoTimelocal
 // (hierarchy_updater.cc:171-190) forms X_m = Q_m X - X Q_m^+ and adds its

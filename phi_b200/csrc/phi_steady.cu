@@ -151,7 +151,7 @@ int plan_deflation(phi_ctx *ctx, int want, int ell, DeflPlan *plan) {
   return PHI_OK;
 }
 
-// A Z by one batched apply of the generic kernel over the nodes of tiers
+// A Z by one batched apply of the node kernel over the nodes of tiers
 // 0..tiers (input j: the unit vector Z_j on the nodes of tiers
 // 0..tiers+1, which hold every neighbour those rows read), then the
 // factors of Z^T A Z.

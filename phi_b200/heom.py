@@ -372,7 +372,7 @@ class Hierarchy:
 
     def tile_schedule(self) -> dict:
         """The tiled kernel's schedule (block size, CTAs per SM cap; threads 0
-        when the problem runs on the generic kernel) and the apply times the
+        when the problem runs on the node kernel) and the apply times the
         autotuner measured for it and for the default."""
         s = capi.PhiTileSchedule()
         self._check(self.lib.phi_gpu_get_tile_schedule(self.ctx, ctypes.byref(s)))
