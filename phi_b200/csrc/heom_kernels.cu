@@ -69,6 +69,7 @@ struct NodePlan {
   int nt;        // nodes per tile
   int cs;        // columns per round: threads / N
   int bc;        // full couplings: baths whose M_b are in shared memory at once
+  int vb;        // and whose V_b are: all of them, or those bc
   int stage_ops; // combine operands staged in shared memory (0: read directly)
   uint32_t x, u, m, v, ops, cf, ids, bytes;
 };
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
     for (int e = tid; e < E; e += nth) Hs[e] = __ldcg(c.H + e);
   }
   if (KIND == kFull && nb)
-    for (int e = tid; e < c.nb * E; e += nth) Vs[e] = __ldcg(c.bath_V + e);
+    for (int e = tid; e < pl.vb * E; e += nth) Vs[e] = __ldcg(c.bath_V + e);
   __syncthreads();  // records
 
   // The tile's X (and H) before the first read of them.
@@ -339,9 +340,13 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
     // M_b of up to bc baths at a time, then B += V_b M_b.
     for (int b0 = 0; b0 < c.nb; b0 += pl.bc) {
       const int bn = c.nb - b0 < pl.bc ? c.nb - b0 : pl.bc;
+      const int v0 = pl.vb < c.nb ? b0 : 0;  // the first bath in Vs
       if (b0 > 0) {
-        __syncthreads();  // the previous baths' M_b are read
+        __syncthreads();  // the previous baths' M_b (and V_b) are read
+        if (v0 > 0)
+          for (int e = tid; e < bn * E; e += nth) Vs[e] = __ldcg(c.bath_V + (size_t)b0 * E + e);
         full_terms(b0, bn);
+        if (v0 > 0) __syncthreads();
       }
       for (int r = 0; r < rounds; ++r) {
         const int col = c0 + r * pl.cs;
@@ -351,7 +356,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         const bool tl = c.time_local && tl_deepest(nd);
         for (int b = 0; b < bn; ++b) {
           // + Delta_b [X, V_b]
-          const double *V = Vs + (size_t)(b0 + b) * E;
+          const double *V = Vs + (size_t)(b0 - v0 + b) * E;
           double2 w = make_double2(0.0, 0.0), z = w;
 #pragma unroll 4
           for (int k = 0; k < N; ++k) {
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         if (!live || col >= ncols) continue;
         double2 u = Us[col * NP + i], w = make_double2(0.0, 0.0);
         for (int b = 0; b < bn; ++b) {
-          const double *V = Vs + (size_t)(b0 + b) * E + i;
+          const double *V = Vs + (size_t)(b0 - v0 + b) * E + i;
           const double2 *M = Ms + b * pl.nt * E + col * N;
           int k = 0;
 #pragma unroll 2
@@ -572,6 +577,8 @@ __global__ void rkf45_control_kernel(Rkf45Ctl *ctl) {
 }
 
 constexpr uint32_t kNodeMaxSmem = 224 * 1024;
+// What one CTA can be given: 227 KiB less the kernel's static shared memory.
+constexpr uint32_t kNodeSmemLimit = 227 * 1024 - 128;
 
 uint32_t align16(uint32_t b) { return (b + 15u) & ~15u; }
 
@@ -587,7 +594,7 @@ void node_layout(const HeomConsts &c, int nops, bool flags, NodePlan *pl) {
   pl->m = b;
   if (c.kind == kFull && !c.vacuum) b += (uint32_t)pl->bc * tile;
   pl->v = b;
-  if (c.kind == kFull && !c.vacuum) b += align16((uint32_t)c.nb * E * 8);
+  if (c.kind == kFull && !c.vacuum) b += align16((uint32_t)pl->vb * E * 8);
   pl->ops = b;
   b += std::max<uint32_t>(pl->stage_ops ? nops : 0, flags ? 1 : 0) * tile;
   pl->cf = b;
@@ -604,45 +611,53 @@ void node_layout(const HeomConsts &c, int nops, bool flags, NodePlan *pl) {
 // part), the SM's element slots, and a CTA's fixed work.  Fitted to a sweep of
 // 17 problems on B200 (N = 3 .. 20, 84 to 20,000 nodes): within 10 % of the
 // best shape of the sweep, where a fixed 256-thread tile was up to 1.6 times
-// slower.
+// slower.  The V_b of all baths are loaded once where that fits; where it does
+// not with any shape (N = 48 with 5 baths, 30 with 32), those of each pass over bc
+// baths are.  threads = 0: nothing fits.
 NodePlan node_plan(const HeomConsts &c, int nops, bool flags, int num_sms) {
   const int N = c.N;
   NodePlan best{};
   double best_cost = 1e300;
-  for (int threads = 64; threads <= kNodeThreads; threads += 32) {
-    const int cs = threads / N;
-    if (cs < 1) continue;
-    for (int want = 1; want <= 4; ++want) {
-      NodePlan pl{};
-      pl.nt = std::max(1, std::min<int>(want * cs / N, 64));
-      const int rounds = (pl.nt * N + cs - 1) / cs;
-      if (rounds < want && want > 1) continue;
-      pl.threads = threads;
-      pl.cs = cs;
-      pl.bc = std::min(c.nb, 8);
-      pl.stage_ops = nops > 0;
-      node_layout(c, nops, flags, &pl);
-      // Larger nodes: first read the operands directly, then take fewer
-      // baths at once.
-      if (pl.bytes > kNodeMaxSmem / 2 && pl.stage_ops) {
-        pl.stage_ops = 0;
+  const auto search = [&](bool all_v) {
+    for (int threads = 64; threads <= kNodeThreads; threads += 32) {
+      const int cs = threads / N;
+      if (cs < 1) continue;
+      for (int want = 1; want <= 4; ++want) {
+        NodePlan pl{};
+        pl.nt = std::max(1, std::min<int>(want * cs / N, 64));
+        const int rounds = (pl.nt * N + cs - 1) / cs;
+        if (rounds < want && want > 1) continue;
+        pl.threads = threads;
+        pl.cs = cs;
+        pl.bc = std::min(c.nb, 8);
+        pl.vb = all_v ? c.nb : pl.bc;
+        pl.stage_ops = nops > 0;
         node_layout(c, nops, flags, &pl);
-      }
-      while (pl.bytes > kNodeMaxSmem && pl.bc > 1 && c.kind == kFull) {
-        --pl.bc;
-        node_layout(c, nops, flags, &pl);
-      }
-      if (pl.bytes > kNodeMaxSmem && pl.nt > 1) continue;
-      const int resident = std::max(1, std::min<int>(768 / threads, (int)(kNodeMaxSmem / pl.bytes)));
-      const double tiles = (double)((c.M + pl.nt - 1) / pl.nt);
-      const double per_sm = std::ceil(tiles / num_sms);
-      const double cost = std::ceil(per_sm / resident) * (2.0 + rounds) + per_sm * (threads * rounds / 512.0 + 0.5);
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = pl;
+        // Larger nodes: first read the operands directly, then take fewer
+        // baths at once.
+        if (pl.bytes > kNodeMaxSmem / 2 && pl.stage_ops) {
+          pl.stage_ops = 0;
+          node_layout(c, nops, flags, &pl);
+        }
+        while (pl.bytes > kNodeMaxSmem && pl.bc > 1 && c.kind == kFull) {
+          --pl.bc;
+          if (!all_v) pl.vb = pl.bc;
+          node_layout(c, nops, flags, &pl);
+        }
+        if (pl.bytes > (pl.nt > 1 ? kNodeMaxSmem : kNodeSmemLimit)) continue;
+        const int resident = std::max(1, std::min<int>(768 / threads, (int)(kNodeMaxSmem / pl.bytes)));
+        const double tiles = (double)((c.M + pl.nt - 1) / pl.nt);
+        const double per_sm = std::ceil(tiles / num_sms);
+        const double cost = std::ceil(per_sm / resident) * (2.0 + rounds) + per_sm * (threads * rounds / 512.0 + 0.5);
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = pl;
+        }
       }
     }
-  }
+  };
+  search(true);
+  if (best.threads == 0 && c.kind == kFull) search(false);
   return best;
 }
 
@@ -712,6 +727,7 @@ cudaError_t launch_stage(const StageLaunch &L, cudaStream_t stream) {
     return cudaErrorInvalidDevice;
   const bool flags = L.c.filtered && L.mode != kModeApply;
   p.plan = node_plan(L.c, p.nops, flags, sms);
+  if (p.plan.threads == 0) return cudaErrorInvalidValue;
   switch (L.c.kind) {
     case kIndependent: return launch_node<kIndependent>(p, batch, stream);
     case kDiagonal: return launch_node<kDiagonal>(p, batch, stream);
