@@ -534,7 +534,8 @@ cudaError_t defl_launch_factor(const DeflView &D, cudaStream_t st) {
   if (D.E <= 32 && (long long)regions * D.E * D.E <= kSmemDoubles && (long long)regions * D.E * D.E > need)
     need = (long long)regions * D.E * D.E;  // one region per warp for the first-tier blocks
   const size_t smem = (size_t)(need < kSmemDoubles ? need : kSmemDoubles) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static thread_local int raised[kSmemLimitDevices] = {};
+  cudaError_t e = raise_smem_limit(factor_kernel, smem, raised);
   if (e != cudaSuccess) return e;
   factor_kernel<<<1, kSolveBlock, smem, st>>>(D);
   w_kernel<<<(unsigned)D.rows, kBlock, 0, st>>>(D);

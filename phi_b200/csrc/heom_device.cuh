@@ -20,23 +20,29 @@ constexpr int kMaxTier = 250;    // L limit (multi-index stored as uint8)
 
 enum BathKind : int { kIndependent = 0, kDiagonal = 1, kFull = 2 };
 
-// Raises a kernel's dynamic shared-memory limit to `bytes` when that is above
-// the default 48 KiB.  The limit belongs to the function on each device, so
-// the largest size set so far is remembered per device ordinal in `seen`
-// (one array per kernel, owned by its launcher; ordinals past the array set
-// the attribute on every launch).
+// Raises a kernel's dynamic shared-memory limit to all that a CTA of it can have
+// on the current device, once per thread (`raised`, by device ordinal, owned by
+// the kernel's launcher; ordinals past the array do it on every launch).  The
+// limit belongs to the function, not to the thread: one fixed value keeps the
+// launch of one thread from lowering it under the larger launch of another.
+// cudaErrorInvalidValue where `bytes` is more than that.
 constexpr int kSmemLimitDevices = 64;
 template <class Kernel>
-inline cudaError_t raise_smem_limit(Kernel kern, size_t bytes, int (&seen)[kSmemLimitDevices]) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+inline cudaError_t raise_smem_limit(Kernel kern, size_t bytes, int (&raised)[kSmemLimitDevices]) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const bool tracked = dev >= 0 && dev < kSmemLimitDevices;
-  if (tracked && seen[dev] >= (int)bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && tracked) seen[dev] = (int)bytes;
-  return e;
+  if (tracked && raised[dev] > 0) return bytes <= (size_t)raised[dev] ? cudaSuccess : cudaErrorInvalidValue;
+  int most = 0;
+  cudaFuncAttributes fa;
+  e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
+  if (e == cudaSuccess) most -= (int)fa.sharedSizeBytes;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e != cudaSuccess) return e;
+  if (tracked) raised[dev] = most;
+  return bytes <= (size_t)most ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // Programmatic dependent launch: the next kernel may start its preamble; this

@@ -664,8 +664,8 @@ NodePlan node_plan(const HeomConsts &c, int nops, bool flags, int num_sms) {
 template <int KIND>
 cudaError_t launch_node(const StageParams &p, int batch, cudaStream_t stream) {
   auto kern = heom_node_kernel<KIND>;
-  static thread_local int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(kern, p.plan.bytes, configured);
+  static thread_local int raised[kSmemLimitDevices] = {};
+  cudaError_t e = raise_smem_limit(kern, p.plan.bytes, raised);
   if (e != cudaSuccess) return e;
   return launch_dependent(true, kern, dim3((unsigned)((p.c.M + p.plan.nt - 1) / p.plan.nt), batch), dim3(p.plan.threads),
                           p.plan.bytes, stream, p);

@@ -355,8 +355,8 @@ int small_threads(const HeomConsts &c) {
 
 template <int KIND, int RI, int RC>
 cudaError_t launch_small_variant(const SmallRk4Params &p, size_t smem, int threads, cudaStream_t stream) {
-  static int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(heom_small_rk4_kernel<KIND, RI, RC>, smem, configured);
+  static thread_local int raised[kSmemLimitDevices] = {};
+  cudaError_t e = raise_smem_limit(heom_small_rk4_kernel<KIND, RI, RC>, smem, raised);
   if (e != cudaSuccess) return e;
   heom_small_rk4_kernel<KIND, RI, RC><<<1, threads, smem, stream>>>(p);
   return cudaGetLastError();

@@ -104,12 +104,18 @@ __global__ void __launch_bounds__(kTileThreads, kBatchMinBlocks<MIXED>)
 
 }  // namespace
 
+namespace {
+template <bool MIXED>
+cudaError_t raise_batch_limit(size_t smem) {
+  static thread_local int raised[kSmemLimitDevices] = {};
+  return raise_smem_limit(heom_tile_batch_kernel<MIXED>, smem, raised);
+}
+}  // namespace
+
 int tile_batch_occupancy(const TileBatchPlan &plan) {
   int blocks = 0;
   const void *fn = plan.mixed ? (const void *)heom_tile_batch_kernel<true> : (const void *)heom_tile_batch_kernel<false>;
-  if (plan.smem > 48 * 1024 &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) != cudaSuccess)
-    return 0;
+  if ((plan.mixed ? raise_batch_limit<true>(plan.smem) : raise_batch_limit<false>(plan.smem)) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, kTileThreads, plan.smem) != cudaSuccess) return 0;
   return blocks;
 }
@@ -118,23 +124,14 @@ cudaError_t launch_tile_batch(const TileBatchPlan &plan, int grid, cudaStream_t 
   if (plan.count <= 0 || plan.total_tiles <= 0) return cudaSuccess;
   if (grid <= 0) return cudaErrorInvalidValue;
   const TileParams *params = static_cast<const TileParams *>(plan.params);
-  if (plan.mixed) {
-    if (plan.smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(heom_tile_batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)plan.smem);
-      if (e != cudaSuccess) return e;
-    }
+  const cudaError_t e = plan.mixed ? raise_batch_limit<true>(plan.smem) : raise_batch_limit<false>(plan.smem);
+  if (e != cudaSuccess) return e;
+  if (plan.mixed)
     heom_tile_batch_kernel<true><<<grid, kTileThreads, plan.smem, stream>>>(params, plan.tile_start, plan.count,
                                                                  plan.total_tiles, plan.err_flag);
-  } else {
-    if (plan.smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(heom_tile_batch_kernel<false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
-      if (e != cudaSuccess) return e;
-    }
+  else
     heom_tile_batch_kernel<false><<<grid, kTileThreads, plan.smem, stream>>>(params, plan.tile_start, plan.count,
                                                                   plan.total_tiles, plan.err_flag);
-  }
   return cudaGetLastError();
 }
 

@@ -342,13 +342,11 @@ template <int N, int KT, bool MIXED, int BT, int ST>
 cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   using S = TileShape<N, MIXED, KT, BT, ST>;
   const long long tiles = (p.c.M + S::NT - 1) / S::NT;
-  const int max_bytes[kMaxPre] = {16, 16, 16, 16, 16};
-  const size_t smem_max = pipe_smem<N, KT, MIXED, BT, ST>(p.c.T, p.c.L, kMaxPre, max_bytes);
   auto kern = heom_tile_pipe_kernel<N, KT, MIXED, BT, ST>;
-  static thread_local int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(kern, smem_max, configured);
-  if (e != cudaSuccess) return e;
+  static thread_local int raised[kSmemLimitDevices] = {};
   const size_t smem = pipe_smem<N, KT, MIXED, BT, ST>(p.c.T, p.c.L, p.npre, p.pre_bytes);
+  cudaError_t e = raise_smem_limit(kern, smem, raised);
+  if (e != cudaSuccess) return e;
   int cap = persistent_grid((const void *)kern, BT, smem);
   if (cap <= 0) return cudaErrorInvalidConfiguration;
   int sms = 0, dev = 0;

@@ -168,8 +168,8 @@ cudaError_t launch_shape(const ResidentParams &p0, cudaStream_t stream) {
   if ((p0.c.M + size - 1) / size > ResidentLayout<N, KT, MIXED, ST>::S::NT) return cudaErrorNotSupported;
   auto kern = heom_tile_resident_kernel<N, KT, MIXED, ST>;
   constexpr size_t smem = ResidentLayout<N, KT, MIXED, ST>::kBytes;
-  static thread_local int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(kern, smem, configured);
+  static thread_local int raised[kSmemLimitDevices] = {};
+  cudaError_t e = raise_smem_limit(kern, smem, raised);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   ResidentParams p = p0;

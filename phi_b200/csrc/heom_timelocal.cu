@@ -148,8 +148,8 @@ size_t tl_smem_bytes(int N) { return (size_t)3 * N * N * sizeof(double2); }
 
 cudaError_t launch_tl(const TlLaunch &p, cudaStream_t stream) {
   const size_t smem = tl_smem_bytes(p.c.N);
-  static thread_local int configured[kSmemLimitDevices] = {};
-  cudaError_t e = raise_smem_limit(tl_kernel, smem, configured);
+  static thread_local int raised[kSmemLimitDevices] = {};
+  cudaError_t e = raise_smem_limit(tl_kernel, smem, raised);
   if (e != cudaSuccess) return e;
   tl_kernel<<<p.c.nb, kTlThreads, smem, stream>>>(p);
   return cudaGetLastError();
