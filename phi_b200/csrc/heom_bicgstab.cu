@@ -172,16 +172,7 @@ __global__ void rho_kernel(BicgVectors V, long long n, BicgScalars *sc, int j) {
     }
     acc[0] += cdot_re(V.rhat[i], rj[i]);
   }
-  if (grid_sum<1>(acc, tot, sc->partials, &sc->counter) && threadIdx.x == 0) {
-    if (!finite(tot[0])) {
-      fail(sc, kBicgNonFinite);
-    } else if (sc->rho0 == 0.0 || tot[0] == 0.0) {
-      fail(sc, kBicgRhoZero);
-    } else {
-      sc->beta = sc->alpha * tot[0] / sc->rho0;
-      sc->rho0 = tot[0];
-    }
-  }
+  if (grid_sum<1>(acc, tot, sc->partials, &sc->counter) && threadIdx.x == 0) bicg_dot_step(sc, tot[0], 0);
 }
 
 // u_i = r_i - beta u_i for i = 0..j; for j >= 1 also the x += alpha u_0 of BiCG
@@ -246,11 +237,7 @@ __global__ void gamma_kernel(BicgVectors V, long long n, BicgScalars *sc, int j)
     }
     acc[0] += cdot_re(V.rhat[i], uj[i]);
   }
-  if (grid_sum<1>(acc, tot, sc->partials, &sc->counter) && threadIdx.x == 0) {
-    if (!finite(tot[0])) fail(sc, kBicgNonFinite);
-    else if (tot[0] == 0.0) fail(sc, kBicgGammaZero);
-    else sc->alpha = sc->rho0 / tot[0];
-  }
+  if (grid_sum<1>(acc, tot, sc->partials, &sc->counter) && threadIdx.x == 0) bicg_dot_step(sc, tot[0], 1);
 }
 
 // rho_kernel / gamma_kernel's scalar steps from per-CTA partial sums of
@@ -360,6 +347,7 @@ __global__ void gram_kernel(BicgVectors V, long long n, BicgScalars *sc) {
     for (int k = 0; k < ND; ++k) ok = ok && finite(tot[k]);
     if (!ok) {
       fail(sc, kBicgNonFinite);
+      sc->x_behind = 1;
       return;
     }
     // Cholesky G = L L^T; a pivot that is not clearly positive means
@@ -405,6 +393,7 @@ __global__ void gram_kernel(BicgVectors V, long long n, BicgScalars *sc) {
       sc->restart = 1;
     } else {
       fail(sc, kBicgGramSingular);
+      sc->x_behind = 1;
       return;
     }
     for (int a = 0; a < ELL; ++a) sc->gamma[a + 1] = g[a];
@@ -475,6 +464,14 @@ __global__ void mr_update_kernel(BicgVectors V, long long n, BicgScalars *sc) {
         sc->rho0 = tot[1];
       }
     }
+  }
+}
+
+__global__ void catch_up_kernel(BicgVectors V, long long n, const BicgScalars *sc) {
+  const double alpha = sc->alpha;
+  GRID_LOOP(e, n) {
+    const double2 x = V.x[e], u0 = V.u[0][e];
+    V.x[e] = make_double2(x.x + alpha * u0.x, x.y + alpha * u0.y);
   }
 }
 
@@ -556,6 +553,10 @@ cudaError_t bicg_launch_gamma(const BicgVectors &V, long long n, BicgScalars *sc
 cudaError_t bicg_launch_r_update(const BicgVectors &V, long long n, const BicgScalars *sc, int j, int grid,
                                  cudaStream_t s) {
   return launch_dependent(bicg_dependent(n), r_update_kernel, dim3(grid), dim3(kBlock), 0, s, V, n, sc, j);
+}
+cudaError_t bicg_launch_catch_up(const BicgVectors &V, long long n, const BicgScalars *sc, int grid, cudaStream_t s) {
+  catch_up_kernel<<<grid, kBlock, 0, s>>>(V, n, sc);
+  return cudaGetLastError();
 }
 cudaError_t bicg_launch_gram(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid, cudaStream_t s) {
   switch (ell) {

@@ -34,6 +34,7 @@ struct BicgScalars {
   double inv_trace;
   int ell, steps, max_steps, done, converged, breakdown, tol_mode;
   int restart;  // the minimal-residual step fell back to one term: restart the BiCG recurrence
+  int x_behind;  // the solve stopped before x += alpha u_0 of the last BiCG step
   unsigned int counter;
   double partials[kMaxGramDots * kMaxBicgBlocks];
 };
@@ -62,6 +63,7 @@ __device__ inline void bicg_dot_step(BicgScalars *sc, double tot, int which) {
   if (code != kBicgOk) {
     sc->breakdown = code;
     sc->done = 1;
+    sc->x_behind = which == 0;  // the next u-update would have added it
   }
 }
 #endif
@@ -91,6 +93,8 @@ cudaError_t bicg_launch_r_update(const BicgVectors &V, long long n, const BicgSc
 // step of rho (which = 0) or gamma (which = 1).
 cudaError_t bicg_launch_dot_finish(const double *parts, long long nparts, BicgScalars *sc, int which,
                                    bool dependent, cudaStream_t s);
+// x += alpha u_0: the last BiCG step of a solve that stopped with x_behind.
+cudaError_t bicg_launch_catch_up(const BicgVectors &V, long long n, const BicgScalars *sc, int grid, cudaStream_t s);
 // Minimal-residual step over r_1..r_ell and the end-of-iteration control.
 cudaError_t bicg_launch_gram(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid, cudaStream_t s);
 cudaError_t bicg_launch_mr_update(const BicgVectors &V, long long n, BicgScalars *sc, int ell, int grid,

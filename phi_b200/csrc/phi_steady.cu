@@ -404,6 +404,10 @@ int steady_impl(phi_ctx *ctx, int32_t ell, double tol, int32_t tol_mode, int32_t
       break;
     }
   }
+  if (result == PHI_OK && host->x_behind) {
+    cudaError_t e = phi::bicg_launch_catch_up(V, n, sc, grid, s);
+    if (e != cudaSuccess) result = steady_err(ctx, e, "last BiCG step");
+  }
   if (result == PHI_OK && Dp) {
     // The coarse part: x = y + Z E^-1 Z^T (b - A y).
     cudaError_t e = apply_fp64(ctx, V.x, V.r[1], s);
