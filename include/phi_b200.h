@@ -441,7 +441,8 @@ PHI_API int phi_gpu_load_state(phi_ctx *ctx, const char *path, double *timestep)
 typedef struct phi_batch phi_batch;
 
 typedef struct {
-  int32_t ctas_per_sm; /* persistent CTAs per SM (grid = ctas_per_sm * SMs) */
+  int32_t ctas_per_sm; /* persistent CTAs per SM (grid = ctas_per_sm * SMs), 1..32;
+                          0: as many as each stage's kernel fits */
   int32_t order;       /* 0: instances in the given order; 1: largest tiles first */
   double ms_per_stage; /* measured by phi_gpu_batch_autotune (0 if not tuned) */
 } phi_batch_schedule;
@@ -463,6 +464,8 @@ PHI_API int phi_gpu_batch_instance(phi_batch *batch, int32_t index, phi_ctx **ct
  * Liouvillian apply of every instance (state unchanged) and keeps the
  * fastest for later RK4 calls; `chosen` may be NULL. */
 PHI_API int phi_gpu_batch_autotune(phi_batch *batch, phi_batch_schedule *chosen);
+/* Sets the schedule; a new batch has ctas_per_sm 0 and order 1.  PHI_E_INVALID
+ * outside those ranges.  Results do not depend on it. */
 PHI_API int phi_gpu_batch_set_schedule(phi_batch *batch, const phi_batch_schedule *schedule);
 /* `steps` RK4 steps of size dt on every instance (Rk4Integrate's stages,
  * hierarchy_integrator.cc:2705-2826); each instance's time advances by

@@ -249,8 +249,8 @@ extern "C" int phi_gpu_batch_instance(phi_batch *batch, int32_t index, phi_ctx *
 
 extern "C" int phi_gpu_batch_set_schedule(phi_batch *batch, const phi_batch_schedule *s) {
   if (!batch || !s) return PHI_E_INVALID;
-  if (s->ctas_per_sm < 1 || s->ctas_per_sm > 32 || (s->order != 0 && s->order != 1))
-    return batch->fail(PHI_E_INVALID, "schedule: ctas_per_sm in 1..32 and order 0 or 1");
+  if (s->ctas_per_sm < 0 || s->ctas_per_sm > 32 || (s->order != 0 && s->order != 1))
+    return batch->fail(PHI_E_INVALID, "schedule: ctas_per_sm in 0..32 and order 0 or 1");
   if (s->ctas_per_sm != batch->sched.ctas_per_sm || s->order != batch->sched.order) {
     if (batch->graph) cudaGraphExecDestroy(batch->graph);
     batch->graph = nullptr;
