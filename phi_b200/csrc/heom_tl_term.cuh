@@ -16,20 +16,20 @@
 
 namespace phi {
 
-// Q: nb*N*N sums Q_m, column-major per bath (read through the read-only
-// cache; a few KB for the sizes the tile kernel serves).  X: the ADO,
-// column-major.  The loop stays rolled so that, inlined into a stage kernel,
+// Q: nb*N*N sums Q_m, column-major per bath (a few KB for the sizes the tile
+// kernel serves), rewritten between stages: plain loads after the stage's
+// pdl_wait, not the read-only path.  X: the ADO, column-major.  The loop stays rolled so that, inlined into a stage kernel,
 // it holds few registers.
 template <class TX>
-static __device__ __forceinline__ TX tl_pair_term(const TX *X, const double2 *__restrict__ Q, int N, int i, int j) {
+static __device__ __forceinline__ TX tl_pair_term(const TX *X, const double2 *Q, int N, int i, int j) {
   using R = decltype(X->x);
   const size_t E = (size_t)N * N;
   const double2 *Qi = Q + (size_t)i * E, *Qj = Q + (size_t)j * E;
   R ar = 0, ai = 0, br = 0, bi = 0;
 #pragma unroll 1
   for (int k = 0; k < N; ++k) {
-    const double2 qji = __ldg(Qj + i + k * N), qii = __ldg(Qi + i + k * N);
-    const double2 qjj = __ldg(Qj + j + k * N), qij = __ldg(Qi + j + k * N);
+    const double2 qji = Qj[i + k * N], qii = Qi[i + k * N];
+    const double2 qjj = Qj[j + k * N], qij = Qi[j + k * N];
     const R dir = (R)(qji.x - qii.x), dii = (R)(qji.y - qii.y);  // D[i][k]
     const R djr = (R)(qjj.x - qij.x), dji = (R)(qjj.y - qij.y);  // D[j][k]
     const TX xkj = X[k + j * N], xki = X[k + i * N];
