@@ -382,6 +382,20 @@ PHI_API int phi_gpu_debug_set_rkf45_replay(phi_ctx *ctx, const int8_t *decisions
                                            int64_t trace_capacity);
 PHI_API int phi_gpu_debug_get_rkf45_errors(phi_ctx *ctx, double *out, int64_t capacity, int64_t *count);
 
+/* Test hooks: which way the last phi_gpu_rk4 of the context took its steps
+ * (PHI_RK4_NONE before the first), and the schedule of the RKF45 stages
+ * (threads 0 before a context's first RKF45 run has chosen one or one was set,
+ * and where the problem is too small to be tuned or off the tiled kernel).  No
+ * counterpart in the reference. */
+enum {
+  PHI_RK4_NONE = 0,
+  PHI_RK4_STAGES = 1,  /* a launch per stage */
+  PHI_RK4_CTA = 2,     /* whole runs in one CTA */
+  PHI_RK4_CLUSTER = 3  /* whole runs in one thread-block cluster */
+};
+PHI_API int phi_gpu_debug_get_rk4_route(const phi_ctx *ctx, int32_t *route);
+PHI_API int phi_gpu_debug_get_rkf45_schedule(const phi_ctx *ctx, int32_t *threads, int32_t *ctas_per_sm);
+
 /* Device memory of destroyed contexts is kept (up to 8 GiB) for the next
  * allocation of the same size in this process; this returns it to the
  * driver and gives the bytes released. */

@@ -365,14 +365,11 @@ int phi_ctx::tune_rkf45(const phi::StageLaunch &stage) {
     std::lock_guard<std::mutex> lock(g_sched_mu);
     g_sched[key] = sched;
   }
+  rkf45_threads = sched.threads;
   c.tile_variant_rkf = sched.variant;
   c.tile_cps_rkf = sched.cps;
   return PHI_OK;
 }
-
-namespace {
-
-}  // namespace
 
 extern "C" int phi_gpu_create(const phi_problem_desc *desc, phi_ctx **out) {
   if (!out) return fail(nullptr, PHI_E_INVALID, "out is NULL");
@@ -857,6 +854,7 @@ extern "C" int phi_gpu_set_tile_schedule(phi_ctx *ctx, int32_t threads, int32_t 
   ctx->c.tile_variant = ctx->c.tile_variant_rkf = variant;
   ctx->c.tile_cps = ctx->c.tile_cps_rkf = ctas_per_sm;
   ctx->rkf45_tuned = true;
+  ctx->rkf45_threads = threads;
   ctx->release_graphs();  // captured launches carry the old schedule
   return PHI_OK;
 }
@@ -976,6 +974,19 @@ extern "C" int phi_gpu_reset(phi_ctx *ctx, double time) {
   PHI_CUDA(ctx, ctx->reset_annealing());
   ctx->time = time;
   ctx->rkf45_started = false;
+  return PHI_OK;
+}
+
+extern "C" int phi_gpu_debug_get_rk4_route(const phi_ctx *ctx, int32_t *route) {
+  if (!ctx || !route) return PHI_E_INVALID;
+  *route = ctx->rk4_route;
+  return PHI_OK;
+}
+
+extern "C" int phi_gpu_debug_get_rkf45_schedule(const phi_ctx *ctx, int32_t *threads, int32_t *ctas_per_sm) {
+  if (!ctx || !threads || !ctas_per_sm) return PHI_E_INVALID;
+  *threads = ctx->rkf45_threads;
+  *ctas_per_sm = ctx->c.tile_cps_rkf;
   return PHI_OK;
 }
 

@@ -116,6 +116,8 @@ struct phi_ctx {
   // c.tile_variant / c.tile_cps).
   phi::TileSchedule tile_sched{};
   bool rkf45_tuned = false;  // the RKF45 stages' schedule is chosen (or set)
+  int rkf45_threads = 0;     // its block size (0: none was chosen)
+  int rk4_route = PHI_RK4_NONE;  // of the last phi_gpu_rk4
   int tune_rkf45(const phi::StageLaunch &stage);
 
   double time = 0.0;

@@ -302,6 +302,7 @@ extern "C" int phi_gpu_rk4(phi_ctx *ctx, double dt, double t_end, double output_
       resident = true;
     }
   }
+  ctx->rk4_route = small && steps > 0 ? PHI_RK4_CTA : (resident ? PHI_RK4_CLUSTER : PHI_RK4_STAGES);
   if (small || resident) {
     if (rows > 0)
       PHI_CK(cudaMemcpyAsync(traj, dtraj, (size_t)rows * ctx->desc.num_states * ctx->desc.num_states * sizeof(double2),
