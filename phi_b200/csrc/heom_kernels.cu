@@ -69,9 +69,9 @@ struct NodePlan {
   int nt;        // nodes per tile
   int cs;        // columns per round: threads / N
   int bc;        // full couplings: baths whose M_b are in shared memory at once
-  int vb;        // and whose V_b are: all of them, or those bc
   int stage_ops; // combine operands staged in shared memory (0: read directly)
   uint32_t x, u, m, v, ops, cf, ids, bytes;
+  int vb;        // full couplings: baths whose V_b are in shared memory at once (all, or bc)
 };
 
 struct StageParams {
@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
     for (int b0 = 0; b0 < c.nb; b0 += pl.bc) {
       const int bn = c.nb - b0 < pl.bc ? c.nb - b0 : pl.bc;
       const int v0 = pl.vb < c.nb ? b0 : 0;  // the first bath in Vs
+      const double *Vb = Vs + (size_t)(b0 - v0) * E;
       if (b0 > 0) {
         __syncthreads();  // the previous baths' M_b (and V_b) are read
         if (v0 > 0)
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         const bool tl = c.time_local && tl_deepest(nd);
         for (int b = 0; b < bn; ++b) {
           // + Delta_b [X, V_b]
-          const double *V = Vs + (size_t)(b0 - v0 + b) * E;
+          const double *V = Vb + (size_t)b * E;
           double2 w = make_double2(0.0, 0.0), z = w;
 #pragma unroll 4
           for (int k = 0; k < N; ++k) {
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         if (!live || col >= ncols) continue;
         double2 u = Us[col * NP + i], w = make_double2(0.0, 0.0);
         for (int b = 0; b < bn; ++b) {
-          const double *V = Vs + (size_t)(b0 - v0 + b) * E + i;
+          const double *V = Vb + (size_t)b * E + i;
           const double2 *M = Ms + b * pl.nt * E + col * N;
           int k = 0;
 #pragma unroll 2

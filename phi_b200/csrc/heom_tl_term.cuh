@@ -16,10 +16,17 @@
 
 namespace phi {
 
+// An element of Q.  Q is rewritten between stages, so it is not read through the
+// read-only path, and a volatile load stays behind the stage's pdl_wait.
+__device__ __forceinline__ double2 ld_q(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+
 // Q: nb*N*N sums Q_m, column-major per bath (a few KB for the sizes the tile
-// kernel serves), rewritten between stages: plain loads after the stage's
-// pdl_wait, not the read-only path.  X: the ADO, column-major.  The loop stays rolled so that, inlined into a stage kernel,
-// it holds few registers.
+// kernel serves).  X: the ADO, column-major.  The loop stays rolled so that,
+// inlined into a stage kernel, it holds few registers.
 template <class TX>
 static __device__ __forceinline__ TX tl_pair_term(const TX *X, const double2 *Q, int N, int i, int j) {
   using R = decltype(X->x);
@@ -28,8 +35,8 @@ static __device__ __forceinline__ TX tl_pair_term(const TX *X, const double2 *Q,
   R ar = 0, ai = 0, br = 0, bi = 0;
 #pragma unroll 1
   for (int k = 0; k < N; ++k) {
-    const double2 qji = Qj[i + k * N], qii = Qi[i + k * N];
-    const double2 qjj = Qj[j + k * N], qij = Qi[j + k * N];
+    const double2 qji = ld_q(Qj + i + k * N), qii = ld_q(Qi + i + k * N);
+    const double2 qjj = ld_q(Qj + j + k * N), qij = ld_q(Qi + j + k * N);
     const R dir = (R)(qji.x - qii.x), dii = (R)(qji.y - qii.y);  // D[i][k]
     const R djr = (R)(qjj.x - qij.x), dji = (R)(qjj.y - qij.y);  // D[j][k]
     const TX xkj = X[k + j * N], xki = X[k + i * N];
