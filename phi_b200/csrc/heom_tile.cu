@@ -15,6 +15,11 @@ using namespace tile_detail;
 
 namespace {
 cudaError_t launch_tile(const TileParams &p, bool mixed, cudaStream_t stream, int *per_sm = nullptr) {
+  if (p.c.time_local && tile_tl_kernels(p.c.N, p.mode == kModeRkf45)) {
+    if (p.mode == kModeRkf45)
+      return mixed ? launch_tile_mixed_rkf45_tl(p, stream, per_sm) : launch_tile_fp64_rkf45_tl(p, stream, per_sm);
+    return mixed ? launch_tile_mixed_rk4_tl(p, stream, per_sm) : launch_tile_fp64_rk4_tl(p, stream, per_sm);
+  }
   if (p.mode == kModeRkf45)
     return mixed ? launch_tile_mixed_rkf45(p, stream, per_sm) : launch_tile_fp64_rkf45(p, stream, per_sm);
   return mixed ? launch_tile_mixed_rk4(p, stream, per_sm) : launch_tile_fp64_rk4(p, stream, per_sm);

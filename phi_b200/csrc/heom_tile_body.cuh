@@ -413,6 +413,7 @@ struct TileIn {
   const uint8_t *mi;    // occupations (time-local truncation)
   const TX *xin;        // the stage input of every node (HBM)
   int nt_here;
+  const int *next;      // next ids of the tile's nodes (the time-local kernels)
 };
 
 // The deepest tier's time-local term of element (i, j), i < j, of node nd.
@@ -426,6 +427,28 @@ __device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileI
   tv = tl_pair_term<typename TileArith<MIXED>::TX>(in.Xs + nd * S::ES, c.tl_q, N, i, j);
   return true;
 }
+
+// The time-local share of B, ((Q_j - Q_i) X)_ij (zero above the deepest tier,
+// whose nodes alone have no next ones), of this thread's elements (TileMap's)
+// into their places of the exchange tile, one product per element.
+template <class TX>
+__device__ __forceinline__ void tile_time_local_half(TX *Us, const TX *Xs, const int *next, const double2 *Q, int N, int T,
+                                                     int ES, int EU, int NP, int CS, int ncols) {
+  const int i = threadIdx.x % N, c0 = threadIdx.x / N;
+  if (c0 >= CS) return;
+  for (int col = c0; col < ncols; col += CS) {
+    const int nd = col / N, j = col - nd * N;
+    TX g;
+    g.x = g.y = 0;
+    if (i != j && next[nd * T] < 0) g = tl_half_term<TX>(Xs + nd * ES, Q, N, i, j);
+    Us[nd * EU + i + j * NP] = g;
+  }
+}
+
+// Whether the time-local truncation of a shape's stages has kernels of its own
+// (TL below): elements, from 4 sites on.  With two or three sites, and by
+// pairs, the general kernels add the pair's term, which costs little there.
+constexpr bool tile_tl_kernels(int N, bool rkf45) { return N >= (rkf45 ? 10 : 4); }
 
 // Phase 2: the derivative dx of this thread's elements of a tile.
 //
@@ -448,7 +471,12 @@ __device__ __forceinline__ bool tile_time_local(const HeomConsts &c, const TileI
 //
 // Barriers: every thread of the CTA calls; Us must be free on entry, and is
 // free again after the CTA's next barrier.
-template <int N, int KT, bool MIXED, int BT, int ST>
+//
+// TL: a time-local run of a shape with tile_tl_kernels.  The pair's term at both
+// of its elements is twice the work (16-site mixed RK4 at 153 nodes 3.76 ms for
+// 32 steps, 1.56 so), and the products in the general kernel cost the runs
+// without them registers (10-site mixed RK4 at K = 2 up to 15 %).
+template <int N, int KT, bool MIXED, int BT, int ST, bool TL = false>
 __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileMap<N, KT, MIXED, BT, ST> &m,
                                                 const TileIn<N, KT, MIXED, BT, ST> &in,
                                                 typename TileArith<MIXED>::TX (&dx)[TileShape<N, MIXED, KT, BT, ST>::RR]) {
@@ -589,6 +617,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
     for (int r = 0; r < RR; ++r) dx[r] = Us[m.uo(r)];
   } else {
     const int i = m.i;
+    if constexpr (TL) tile_time_local_half(Us, in.Xs, in.next, c.tl_q, N, T, ES, EU, NP, S::CS, in.nt_here * N);
     // FP64 issues the gathers after the products (registers).
     constexpr bool kHoist = MIXED || KT == 1 || tile_resident(ST) || (KT == 2 && ST == kTileRkf45);
     TX gn[RR][KT], gp[RR][KT];
@@ -624,6 +653,11 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
           by = fma(f.ay, gp[r][q].y, by);
         }
       }
+      if (TL && m.on(r, in.nt_here)) {
+        const TX g = Us[m.uo(r)];
+        bx += g.x;
+        by += g.y;
+      }
       dx[r] = mk<TX>(bx, by);
       if ((m.live >> r) & 1u) Us[m.uo(r)] = dx[r];
     }
@@ -643,7 +677,7 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
       }
       dx[r] = mk<TX>(vx, vy);
     }
-    if (c.time_local) {
+    if (!TL && c.time_local) {
 #pragma unroll 1
       for (int r = 0; r < RR; ++r) {
         int j = 0, nd = 0;
@@ -1017,7 +1051,7 @@ __device__ __forceinline__ int tile_body(const TileParams &p, long long tile, un
   }
 
   const TileMap<N, KT, MIXED, BT, ST> m(c);
-  const In in{Xs, Us, Hs, mats, ids, cfs, nullptr, deph, c.mi + n0 * T, xin, nt_here};
+  const In in{Xs, Us, Hs, mats, ids, cfs, nullptr, deph, c.mi + n0 * T, xin, nt_here, nullptr};
   TX dx[S::RR];
   tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
   ok = p.npre == 0 || mbar_wait_bounded(&bars[1], par1);
@@ -1068,6 +1102,11 @@ cudaError_t launch_tile_fp64_rk4(const TileParams &p, cudaStream_t stream, int *
 cudaError_t launch_tile_fp64_rkf45(const TileParams &p, cudaStream_t stream, int *per_sm);
 cudaError_t launch_tile_mixed_rk4(const TileParams &p, cudaStream_t stream, int *per_sm);
 cudaError_t launch_tile_mixed_rkf45(const TileParams &p, cudaStream_t stream, int *per_sm);
+// The same for time-local runs of the shapes with kernels of their own.
+cudaError_t launch_tile_fp64_rk4_tl(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_fp64_rkf45_tl(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_mixed_rk4_tl(const TileParams &p, cudaStream_t stream, int *per_sm);
+cudaError_t launch_tile_mixed_rkf45_tl(const TileParams &p, cudaStream_t stream, int *per_sm);
 
 }  // namespace tile_detail
 }  // namespace phi

@@ -4,7 +4,7 @@
 namespace phi {
 namespace tile_detail {
 cudaError_t launch_tile_fp64_rk4(const TileParams &p, cudaStream_t stream, int *per_sm) {
-  return launch_tile_dispatch<false, kTileRk4>(p, stream, per_sm);
+  return launch_tile_dispatch<false, kTileRk4, false>(p, stream, per_sm);
 }
 }  // namespace tile_detail
 }  // namespace phi

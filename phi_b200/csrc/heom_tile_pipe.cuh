@@ -1,7 +1,8 @@
 // heom_tile_pipe.cuh -- the persistent tile kernel of one IndependentBath
 // hierarchy and its launch.  Each including file instantiates it for one
-// arithmetic and one kind of stage (RKF: RKF45; otherwise apply and RK4), so
-// the four sets compile side by side.  Internal header.
+// arithmetic and one kind of stage (RKF: RKF45; otherwise apply and RK4), for
+// time-local runs or in general, so the sets compile side by side.  Internal
+// header.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -78,7 +79,7 @@ size_t pipe_smem(int T, int L, int npre, const int *pre_bytes) {
   return b;
 }
 
-template <int N, int KT, bool MIXED, int BT, int ST>
+template <int N, int KT, bool MIXED, int BT, int ST, bool TL>
 __global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<N, MIXED, KT, BT, ST>::kPairs>::value) heom_tile_pipe_kernel(TileParams p) {
   using S = TileShape<N, MIXED, KT, BT, ST>;
   using Lay = PipeLayout<N, KT, MIXED, BT, ST>;
@@ -216,13 +217,16 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<
   auto slot_mi = [&](int s, long long n0) {
     return reinterpret_cast<const uint8_t *>(slot(s) + Lay::kSlotX + 2 * Lay::kSlotIds) + ((n0 * T) & 15);
   };
+  auto slot_next = [&](int s, long long n0) {
+    return reinterpret_cast<const int *>(slot(s) + Lay::kSlotX) + ((n0 * T) & 3);
+  };
   // Per (node, term) of the tile in slot s: neighbour element offsets (-1 when
   // absent or inactive) and coefficients.
   auto records = [&](long long tile, int s) {
     const long long n0 = tile * NT;
     const int nt = (int)((c.M - n0) < NT ? (c.M - n0) : NT);
     const unsigned char *sb = slot(s);
-    const int *nx_s = reinterpret_cast<const int *>(sb + Lay::kSlotX) + ((n0 * T) & 3);
+    const int *nx_s = slot_next(s, n0);
     const int *pv_s = reinterpret_cast<const int *>(sb + Lay::kSlotX + Lay::kSlotIds) + ((n0 * T) & 3);
     const uint8_t *mi_s = slot_mi(s, n0);
     for (int q = tid; q < nt * T; q += BT) {
@@ -271,9 +275,9 @@ __global__ void __launch_bounds__(BT, TileMinBlocks<N, KT, MIXED, BT, TileShape<
     const double *deph =
         reinterpret_cast<const double *>(sb + Lay::kSlotX + 2 * Lay::kSlotIds + Lay::kSlotMi) + (n0 & 1);
     const TileIn<N, KT, MIXED, BT, ST> in{Xs,   Us,   Hs, mats, ids + s * NT * T, cfs + s * NT * T,
-                                      ccs, deph, slot_mi(s, n0), xin, nt_here};
+                                      ccs, deph, slot_mi(s, n0), xin, nt_here, slot_next(s, n0)};
     TX dx[S::RR];
-    tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
+    tile_derivative<N, KT, MIXED, BT, ST, TL>(c, m, in, dx);
     // The operands have had the derivative's time to land.  A wait that gave
     // up skips the stores; the tile's last barrier then ends the CTA.
     ok = p.npre == 0 || mbar_wait_bounded(&bars[2], (uint32_t)i & 1u);
@@ -338,11 +342,11 @@ int persistent_grid(const void *fn, int threads, size_t smem) {
 // this launch's shared-memory size (capped at tile_cps CTAs per SM when the
 // schedule sets it) and never more than the tiles.  *per_sm (optional)
 // receives the resident CTAs per SM before the cap.
-template <int N, int KT, bool MIXED, int BT, int ST>
+template <int N, int KT, bool MIXED, int BT, int ST, bool TL>
 cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   using S = TileShape<N, MIXED, KT, BT, ST>;
   const long long tiles = (p.c.M + S::NT - 1) / S::NT;
-  auto kern = heom_tile_pipe_kernel<N, KT, MIXED, BT, ST>;
+  auto kern = heom_tile_pipe_kernel<N, KT, MIXED, BT, ST, TL>;
   static thread_local int raised[kSmemLimitDevices] = {};
   const size_t smem = pipe_smem<N, KT, MIXED, BT, ST>(p.c.T, p.c.L, p.npre, p.pre_bytes);
   cudaError_t e = raise_smem_limit(kern, smem, raised);
@@ -367,37 +371,38 @@ cudaError_t launch_tile_bt(const TileParams &p, cudaStream_t stream, int *per_sm
   return launch_dependent(d.dependent, kern, dim3((unsigned)grid), dim3(BT), smem, stream, d);
 }
 
-template <int N, int KT, bool MIXED, int ST>
+template <int N, int KT, bool MIXED, int ST, bool TL>
 cudaError_t launch_tile_nk(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   if (p.c.tile_variant == 1)
-    return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::alt, ST>(p, stream, per_sm);
-  return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::threads, ST>(p, stream, per_sm);
+    return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::alt, ST, TL>(p, stream, per_sm);
+  return launch_tile_bt<N, KT, MIXED, TileBlock<N, MIXED>::threads, ST, TL>(p, stream, per_sm);
 }
 
-template <int N, bool MIXED, int ST>
+template <int N, bool MIXED, int ST, bool TL>
 cudaError_t launch_tile_n(const TileParams &p, cudaStream_t stream, int *per_sm) {
-  switch (p.c.K1) {
-    case 1: return launch_tile_nk<N, 1, MIXED, ST>(p, stream, per_sm);
-    case 2: return launch_tile_nk<N, 2, MIXED, ST>(p, stream, per_sm);
-    case 3: return launch_tile_nk<N, 3, MIXED, ST>(p, stream, per_sm);
+  if constexpr (TL && !tile_tl_kernels(N, ST == kTileRkf45)) return cudaErrorInvalidValue;
+  else switch (p.c.K1) {
+    case 1: return launch_tile_nk<N, 1, MIXED, ST, TL>(p, stream, per_sm);
+    case 2: return launch_tile_nk<N, 2, MIXED, ST, TL>(p, stream, per_sm);
+    case 3: return launch_tile_nk<N, 3, MIXED, ST, TL>(p, stream, per_sm);
     default: return cudaErrorInvalidValue;
   }
 }
 
-template <bool MIXED, int ST>
+template <bool MIXED, int ST, bool TL>
 cudaError_t launch_tile_dispatch(const TileParams &p, cudaStream_t stream, int *per_sm = nullptr) {
   switch (p.c.N) {
-    case 2: return launch_tile_n<2, MIXED, ST>(p, stream, per_sm);
-    case 3: return launch_tile_n<3, MIXED, ST>(p, stream, per_sm);
-    case 4: return launch_tile_n<4, MIXED, ST>(p, stream, per_sm);
-    case 5: return launch_tile_n<5, MIXED, ST>(p, stream, per_sm);
-    case 6: return launch_tile_n<6, MIXED, ST>(p, stream, per_sm);
-    case 7: return launch_tile_n<7, MIXED, ST>(p, stream, per_sm);
-    case 8: return launch_tile_n<8, MIXED, ST>(p, stream, per_sm);
-    case 10: return launch_tile_n<10, MIXED, ST>(p, stream, per_sm);
-    case 12: return launch_tile_n<12, MIXED, ST>(p, stream, per_sm);
-    case 16: return launch_tile_n<16, MIXED, ST>(p, stream, per_sm);
-    case 24: return launch_tile_n<24, MIXED, ST>(p, stream, per_sm);
+    case 2: return launch_tile_n<2, MIXED, ST, TL>(p, stream, per_sm);
+    case 3: return launch_tile_n<3, MIXED, ST, TL>(p, stream, per_sm);
+    case 4: return launch_tile_n<4, MIXED, ST, TL>(p, stream, per_sm);
+    case 5: return launch_tile_n<5, MIXED, ST, TL>(p, stream, per_sm);
+    case 6: return launch_tile_n<6, MIXED, ST, TL>(p, stream, per_sm);
+    case 7: return launch_tile_n<7, MIXED, ST, TL>(p, stream, per_sm);
+    case 8: return launch_tile_n<8, MIXED, ST, TL>(p, stream, per_sm);
+    case 10: return launch_tile_n<10, MIXED, ST, TL>(p, stream, per_sm);
+    case 12: return launch_tile_n<12, MIXED, ST, TL>(p, stream, per_sm);
+    case 16: return launch_tile_n<16, MIXED, ST, TL>(p, stream, per_sm);
+    case 24: return launch_tile_n<24, MIXED, ST, TL>(p, stream, per_sm);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) heom_tile_resident_kernel(con
       // Stage inputs: y, X_a, X_b, X_a; the tile's own in Xs[s & 1].
       const TX *xin = s == 0 ? ybuf : static_cast<const TX *>(p.xbuf[s == 2]);
       TX *out = (s == 3 ? ybuf : static_cast<TX *>(p.xbuf[s == 1])) + n0 * ES;
-      const In in{Xs[s & 1], Us, Hs, mats, ids, cfs, nullptr, deph, nullptr, xin, nt};
+      const In in{Xs[s & 1], Us, Hs, mats, ids, cfs, nullptr, deph, nullptr, xin, nt, nullptr};
       TX dx[RR];
       tile_derivative<N, KT, MIXED, BT, ST>(c, m, in, dx);
 #pragma unroll

@@ -7,7 +7,9 @@
 // deepest-tier ADO X gains X_j[i][j] - X_i[i][j].  With D = Q_j - Q_i and X
 // Hermitian that is
 //     (D X)_ij - conj((D X)_ji),
-// the same shape as the commutator with H; for i == j it vanishes.
+// the same shape as the commutator with H; for i == j it vanishes.  Either a
+// thread evaluates a pair (tl_pair_term), or each element adds its own product
+// (tl_half_term) before the transposed elements are exchanged.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -53,6 +55,29 @@ static __device__ __forceinline__ TX tl_pair_term(const TX *X, const double2 *Q,
   out.x = ar - br;  // a - conj(b)
   out.y = ai + bi;
   return out;
+}
+
+// ((Q_j - Q_i) X)_ij: added to its conjugate transpose over the pair, the term
+// above (element (j, i) has -D).
+template <class TX>
+static __device__ __forceinline__ TX tl_half_term(const TX *X, const double2 *Q, int N, int i, int j) {
+  using R = decltype(X->x);
+  const size_t E = (size_t)N * N;
+  const double2 *Qi = Q + (size_t)i * E + i, *Qj = Q + (size_t)j * E + i;
+  const TX *Xj = X + j * N;
+  TX g;
+  g.x = g.y = 0;
+#pragma unroll 4
+  for (int k = 0; k < N; ++k) {
+    const double2 qj = ld_q(Qj + k * N), qi = ld_q(Qi + k * N);
+    const R dr = (R)(qj.x - qi.x), di = (R)(qj.y - qi.y);
+    const TX x = Xj[k];
+    g.x = fma(dr, x.x, g.x);
+    g.x = fma(-di, x.y, g.x);
+    g.y = fma(dr, x.y, g.y);
+    g.y = fma(di, x.x, g.y);
+  }
+  return g;
 }
 
 }  // namespace phi
