@@ -772,7 +772,7 @@ def main():
             "propagations_completed_in_timed_region": propagations,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "heom_tile_kernel x6 + rkf45_control_kernel (one RKF45 step)",
+                         "kernel": "heom_tile_pipe_kernel x6 + rkf45_control_kernel (one RKF45 step)",
                          "algorithmic_bytes_per_step": step_bytes, "peak_kind": peak_kind},
             "apply_kernel": {"ms": apply_ms, "algorithmic_bytes": apply_bytes, "achieved_gbs": apply_gbs,
                              "frac": apply_gbs / peak, "node_applies_per_s": M / (apply_ms / 1e3)},

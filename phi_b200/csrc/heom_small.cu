@@ -3,11 +3,12 @@
 // A hierarchy of a few hundred elements (PHI's spin-boson configuration has
 // 11 nodes of 2 x 2) gives each stage kernel a handful of warps of work, so
 // a run of four launches per step is bound by launch and memory latency,
-// not by the SMs.  Here one CTA keeps the state y, the RK4 accumulator, the
-// stage input and the stage derivative in shared memory and loops over every
-// step of the run on the device: a stage is one pass over the hierarchy's
-// upper-triangle (node, pair) items and one element-wise combine, separated
-// by block barriers.  The arithmetic is that of the node kernel
+// not by the SMs.  Here one CTA loops over every step of the run on the
+// device.  With a thread per upper-triangle (node, pair) item the state, the RK4
+// accumulator and the item's coefficients are in registers, only the stage
+// inputs in shared memory, and a stage has one barrier; larger hierarchies keep
+// all of it in shared memory, a stage being one pass over the items and one
+// element-wise combine, separated by block barriers.  The arithmetic is that of the node kernel
 // (heom_kernels.cu) for IndependentBath and DiagonalBath couplings:
 // HierarchyUpdater::Get (hierarchy_updater.h:36-75, hierarchy_updater.cc
 // :84-127, :216-254) and the RK4 combines of Rk4Integrate

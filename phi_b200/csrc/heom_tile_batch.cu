@@ -4,9 +4,9 @@
 // The instances' tile lists are concatenated (tile_start[i] = first tile of
 // instance i); CTAs stride over the concatenated list, find the instance of a
 // tile by binary search over tile_start, and run the tile with the
-// instantiation of that instance's (N, K+1) -- the same tile_body as the
-// single-instance kernel, so every instance gets the same arithmetic it gets
-// alone.  Small hierarchies that would fill only a few CTAs of their own
+// instantiation of that instance's (N, K+1): tile_body, one tile in flight
+// around the tile_derivative and tile_epilogue of the single-instance kernel, so
+// every instance gets the same arithmetic it gets alone.  Small hierarchies that would fill only a few CTAs of their own
 // launch share the GPU with the large ones; one launch per stage serves them
 // all, and the step loop replays from a CUDA graph.
 //

@@ -8,12 +8,14 @@
 //
 //   FP64   every buffer complex128 (the path PHI computes).
 //   MIXED  stage inputs X_s and stage derivatives k_s stored as complex64 and
-//          the Liouvillian evaluated in FP32; the state y, the RK4
-//          accumulator, every stage combine (X_{s+1} = y + sum b k), the
-//          fourth/fifth-order solutions, the RKF45 error norm and the step
-//          control stay FP64.  A complex64 copy of y (y32) is the stage-0
-//          input.  complex64 buffers pad every node to an even number of
-//          elements so each node range is 16-byte aligned.
+//          the Liouvillian evaluated in FP32, and with it the next stage
+//          input (X_{s+1} = y + sum b k) of RK4 stages 0-2 and RKF45
+//          stages 0-4, which is stored as complex64; the state y, the RK4
+//          accumulator, the fourth/fifth-order solutions, the RKF45 error
+//          norm and the step control stay FP64.  A complex64 copy of y
+//          (y32) is the stage-0 input.  complex64 buffers pad every node
+//          to an even number of elements so each node range is 16-byte
+//          aligned.
 //
 // A CTA of BT threads (kTileThreads = 256, or what the single-instance
 // launch picks) owns a tile of NT consecutive nodes.  Everything the tile
@@ -222,7 +224,14 @@ struct TileLayout {
   static constexpr size_t kPre = kU + kUBytes;
 };
 
-// Resident warps per SM the register budget is fitted to.
+// Resident warps per SM the register budget is fitted to: 24 (80 registers)
+// unless 32 (64 registers) hold the shape without many spills and pay.  Timed
+// 32 against 24: FP64 elements with one term per site 2.53 and 2.68 ms (16-site
+// RK4, 32 steps), 9.65 and 9.82 (24-site, 64 steps), but 1.14 and 1.09 (7-site
+// with 3,432 nodes); mixed pairs with two terms per site from 6 sites on 8.1 and
+// 8.8 ms (7-site RKF45, 38,760 nodes; 3 to 5 % the other way below 1,000
+// nodes).  Elsewhere 32 is slower, by up to 1.6 (mixed RK4 with two or three
+// terms per site, which spill).
 template <int N, int KT, bool MIXED, int BT, bool PAIRS>
 struct TileMinBlocks {
   static constexpr int warps = MIXED ? (PAIRS && KT == 2 && N >= 6 ? 32 : 24) : (KT == 1 && !PAIRS ? 32 : 24);
@@ -467,7 +476,11 @@ constexpr bool tile_tl_kernels(int N, bool rkf45) { return N >= (rkf45 ? 10 : 4)
 // of a stiff hierarchy (7 sites, K = 1, depth 6) is rounding amplified in the
 // deep tiers, so another order of this sum accepts and rejects other steps,
 // and a run can then end past t_end instead of at it (PHI's clamp does not
-// see a grown step).
+// see a grown step): 2 of 16 seeds in mixed precision.  From 10 sites on, where
+// the element mapping is up to 1.4 times faster, the order does not matter so:
+// over 10 to 24 sites, K = 0 and 1, depths 2 to 6, both arithmetics and three
+// seeds, 107 of 108 runs take the steps of the pair order (one 24-site mixed
+// run 87 instead of 86) and all end at t_end.
 //
 // Barriers: every thread of the CTA calls; Us must be free on entry, and is
 // free again after the CTA's next barrier.
@@ -618,7 +631,13 @@ __device__ __forceinline__ void tile_derivative(const HeomConsts &c, const TileM
   } else {
     const int i = m.i;
     if constexpr (TL) tile_time_local_half(Us, in.Xs, in.next, c.tl_q, N, T, ES, EU, NP, S::CS, in.nt_here * N);
-    // FP64 issues the gathers after the products (registers).
+    // The gathers before the products, whose work hides their latency, where the
+    // registers allow.  After them instead: mixed RK4 3 to 29 % slower at one or
+    // two terms per site (3 to 10 % faster at three from 16 sites on), FP64 of one
+    // term 1 to 16 % slower.  FP64 RK4 of two or three terms would spill: 24 sites
+    // 5.00 -> 6.44 ms, 5 to 8 sites at three 10 to 19 % (4 sites at two gain 10 %).
+    // FP64 RKF45 of two is within 1 % either way at 10 to 16 sites; 24 sites take
+    // 2.01 ms so and 1.74 after.
     constexpr bool kHoist = MIXED || KT == 1 || tile_resident(ST) || (KT == 2 && ST == kTileRkf45);
     TX gn[RR][KT], gp[RR][KT];
     auto gather = [&](int r) {
@@ -899,21 +918,21 @@ template <bool MIXED, int BT>
 __device__ __forceinline__ void tile_error_max(const TileParams &p, double emax, unsigned long long *wmax) {
   const int tid = threadIdx.x;
   if (MIXED) emax = sqrt(emax);
-    unsigned long long bits = (unsigned long long)__double_as_longlong(emax);
-    for (int off = 16; off > 0; off >>= 1) {
-      const unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
-      bits = o > bits ? o : bits;
-    }
-    // One atomic per CTA: a single error word takes every CTA's maximum,
-    // so per-warp atomics would serialise tens of thousands of updates.
-    if ((tid & 31) == 0) wmax[tid >> 5] = bits;
-    __syncthreads();
-    if (tid == 0) {
-      unsigned long long m = wmax[0];
+  unsigned long long bits = (unsigned long long)__double_as_longlong(emax);
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
+    bits = o > bits ? o : bits;
+  }
+  // One atomic per CTA: a single error word takes every CTA's maximum,
+  // so per-warp atomics would serialise tens of thousands of updates.
+  if ((tid & 31) == 0) wmax[tid >> 5] = bits;
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long m = wmax[0];
 #pragma unroll
-      for (int w = 1; w < (BT / 32); ++w) m = wmax[w] > m ? wmax[w] : m;
-      if (m) atomicMax(&p.ctl->err_bits, m);
-    }
+    for (int w = 1; w < (BT / 32); ++w) m = wmax[w] > m ? wmax[w] : m;
+    if (m) atomicMax(&p.ctl->err_bits, m);
+  }
 }
 
 // An apply's inner product: the sum over the CTA's threads into its slot, in
@@ -1082,10 +1101,10 @@ inline size_t tile_smem(int T, int npre, const int *pre_bytes) {
 }
 
 // Threads per CTA of the single-instance kernel: 320 for the 24-site mixed
-// kernel (a node's 300 pairs in one pass, two nodes per tile: timed on B200,
-// its RKF45 step 1.65 -> 1.56 ms), 256 otherwise (320 everywhere was slower
-// on the 7-site and the batched workloads).  The batched kernel always runs
-// 256, so its tile counts (tile_count) use that.
+// kernel (20,475 nodes: RKF45 step 0.88 ms against 1.00 with 256, RK4 step 0.58
+// against 0.65), 256 otherwise (320 everywhere was slower on the 7-site and the
+// batched workloads).  The batched kernel always runs 256, so its tile counts
+// (tile_count) use that.
 template <int N, bool MIXED>
 struct TileBlock {
   static constexpr int threads = (MIXED && N == 24) ? 320 : kTileThreads;
