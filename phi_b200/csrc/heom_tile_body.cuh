@@ -476,11 +476,13 @@ constexpr bool tile_tl_kernels(int N, bool rkf45) { return N >= (rkf45 ? 10 : 4)
 // of a stiff hierarchy (7 sites, K = 1, depth 6) is rounding amplified in the
 // deep tiers, so another order of this sum accepts and rejects other steps,
 // and a run can then end past t_end instead of at it (PHI's clamp does not
-// see a grown step): 2 of 16 seeds in mixed precision.  From 10 sites on, where
-// the element mapping is up to 1.4 times faster, the order does not matter so:
-// over 10 to 24 sites, K = 0 and 1, depths 2 to 6, both arithmetics and three
-// seeds, 107 of 108 runs take the steps of the pair order (one 24-site mixed
-// run 87 instead of 86) and all end at t_end.
+// see a grown step): 2 of 16 seeds in mixed precision.  From 10 sites on the
+// order does not matter so: over 10 to 24 sites, K = 0 and 1, depths 2 to 6, both
+// arithmetics and three seeds, 107 of 108 runs take the steps of the pair order
+// (one 24-site mixed run 87 instead of 86) and all end at t_end.  There the pair
+// mapping would take, over K = 0 to 2 and both arithmetics, 0.80 to 1.06 times the
+// element mapping's time at 10 sites, 0.84 to 1.21 at 12, 1.01 to 1.38 at 16 and
+// 0.90 to 1.23 at 24.
 //
 // Barriers: every thread of the CTA calls; Us must be free on entry, and is
 // free again after the CTA's next barrier.
