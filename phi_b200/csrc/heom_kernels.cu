@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
       Us[col * NP + i] = make_double2(fma(a[r].y, ih, acc[r].x), fma(-a[r].x, ih, acc[r].y));
     }
   }
-  if (TL && nb) {
+  if (TL) {
     for (int r = 0; r < rounds; ++r) {
       const int col = c0 + r * pl.cs, nd = col / N, j = col - nd * N;
       if (!live || col >= ncols || i == j || !tl_deepest(nd)) continue;

@@ -41,3 +41,16 @@ def test_time_local_runs(n, k1, filtered):
         with Hierarchy(p, precision=capi.PHI_PREC_MIXED) as h:
             h.rk4(dt, t_end)
             assert np.abs(h.rho0() - rho).max() <= 1e-6
+
+
+@pytest.mark.parametrize("n", [3, 4, 9, 16])
+def test_single_tier(n):
+    """One tier: every node is deepest and there are no neighbour terms."""
+    p = cases.random_problem("independent", n=n, matsubara=1, truncation=1, seed=n, scale=20.0)
+    p.use_time_local_truncation = True
+    p.fix_incompatible_combinations("rkf45")
+    with Hierarchy(p) as h:
+        o = O.Oracle(p)
+        ref, *_ = o.rk4(o.initial_state(), 1e-4, 9.5e-4)
+        h.rk4(1e-4, 9.5e-4)
+        assert np.abs(h.get_state() - ref).max() <= 1e-10 * np.abs(ref).max()
