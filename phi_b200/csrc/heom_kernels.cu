@@ -109,16 +109,23 @@ struct alignas(16) NodeCoef {
   double s, pad, ax, ay;
 };
 
-// TL: time-local runs of independent baths from 9 sites on, where each element
-// adds its own product of the term before the exchange; the pair's term at both
-// of its elements is twice the work (48 sites 27.3 ms for 32 RK4 steps, 13.1
-// so; 20 sites 3.79 and 2.18), which a few sites do not notice.
-template <int KIND, bool TL>
+// What a kernel of its own keeps out of the others (registers and 0.6 % of a
+// 6-state full coupling):
+//   kTimeLocal  time-local runs of independent baths from 9 sites on, where each
+//               element adds its own product of the term before the exchange;
+//               the pair's term at both of its elements is twice the work (48
+//               sites 27.3 ms for 32 RK4 steps, 13.1 so; 20 sites 3.79 and
+//               2.18), which a few sites do not notice.
+//   kVPerPass   full couplings whose V_b do not all fit (NodePlan::vb = bc).
+enum NodeVariant : int { kPlain = 0, kTimeLocal = 1, kVPerPass = 2 };
+
+template <int KIND, int VARIANT>
 __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_constant__ StageParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const HeomConsts &c = p.c;
   const NodePlan &pl = p.plan;
   const int N = c.N, E = N * N, T = c.T, tid = threadIdx.x, nth = blockDim.x;
+  constexpr bool TL = VARIANT == kTimeLocal, VP = VARIANT == kVPerPass;
   const int NP = N | 1;  // odd column stride of the exchange tile: transposed reads in distinct banks
   double2 *Hs = reinterpret_cast<double2 *>(smem_raw);
   double2 *Xs = reinterpret_cast<double2 *>(smem_raw + pl.x);
@@ -185,7 +192,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
     for (int e = tid; e < E; e += nth) Hs[e] = __ldcg(c.H + e);
   }
   if (KIND == kFull && nb)
-    for (int e = tid; e < pl.vb * E; e += nth) Vs[e] = __ldcg(c.bath_V + e);
+    for (int e = tid; e < (VP ? pl.vb : c.nb) * E; e += nth) Vs[e] = __ldcg(c.bath_V + e);
   __syncthreads();  // records
 
   // The tile's X (and H) before the first read of them.
@@ -353,14 +360,12 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
     // M_b of up to bc baths at a time, then B += V_b M_b.
     for (int b0 = 0; b0 < c.nb; b0 += pl.bc) {
       const int bn = c.nb - b0 < pl.bc ? c.nb - b0 : pl.bc;
-      const int v0 = pl.vb < c.nb ? b0 : 0;  // the first bath in Vs
-      const double *Vb = Vs + (size_t)(b0 - v0) * E;
       if (b0 > 0) {
         __syncthreads();  // the previous baths' M_b (and V_b) are read
-        if (v0 > 0)
+        if (VP)
           for (int e = tid; e < bn * E; e += nth) Vs[e] = __ldcg(c.bath_V + (size_t)b0 * E + e);
         full_terms(b0, bn);
-        if (v0 > 0) __syncthreads();
+        if (VP) __syncthreads();
       }
       for (int r = 0; r < rounds; ++r) {
         const int col = c0 + r * pl.cs;
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         const bool tl = c.time_local && tl_deepest(nd);
         for (int b = 0; b < bn; ++b) {
           // + Delta_b [X, V_b]
-          const double *V = Vb + (size_t)b * E;
+          const double *V = Vs + (size_t)(VP ? b : b0 + b) * E;
           double2 w = make_double2(0.0, 0.0), z = w;
 #pragma unroll 4
           for (int k = 0; k < N; ++k) {
@@ -389,7 +394,7 @@ __global__ void __launch_bounds__(kNodeThreads) heom_node_kernel(const __grid_co
         if (!live || col >= ncols) continue;
         double2 u = Us[col * NP + i], w = make_double2(0.0, 0.0);
         for (int b = 0; b < bn; ++b) {
-          const double *V = Vb + (size_t)b * E + i;
+          const double *V = Vs + (size_t)(VP ? b : b0 + b) * E + i;
           const double2 *M = Ms + b * pl.nt * E + col * N;
           int k = 0;
 #pragma unroll 2
@@ -675,9 +680,9 @@ NodePlan node_plan(const HeomConsts &c, int nops, bool flags, int num_sms) {
   return best;
 }
 
-template <int KIND, bool TL = false>
+template <int KIND, int VARIANT = kPlain>
 cudaError_t launch_node(const StageParams &p, int batch, cudaStream_t stream) {
-  auto kern = heom_node_kernel<KIND, TL>;
+  auto kern = heom_node_kernel<KIND, VARIANT>;
   static thread_local int raised[kSmemLimitDevices] = {};
   cudaError_t e = raise_smem_limit(kern, p.plan.bytes, raised);
   if (e != cudaSuccess) return e;
@@ -744,10 +749,11 @@ cudaError_t launch_stage(const StageLaunch &L, cudaStream_t stream) {
   if (p.plan.threads == 0) return cudaErrorInvalidValue;
   switch (L.c.kind) {
     case kIndependent:
-      return p.c.time_local && p.c.N > 8 ? launch_node<kIndependent, true>(p, batch, stream)
+      return p.c.time_local && p.c.N > 8 ? launch_node<kIndependent, kTimeLocal>(p, batch, stream)
                                          : launch_node<kIndependent>(p, batch, stream);
     case kDiagonal: return launch_node<kDiagonal>(p, batch, stream);
-    default: return launch_node<kFull>(p, batch, stream);
+    default:
+      return p.plan.vb < p.c.nb ? launch_node<kFull, kVPerPass>(p, batch, stream) : launch_node<kFull>(p, batch, stream);
   }
 }
 
